@@ -1,5 +1,6 @@
 // C ABI: device and scene lifetime plus the ray-query entry points declared in include/selas.h.
 // Status codes instead of exceptions; the message of the last failure is kept per host thread.
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -60,11 +61,14 @@ int read_error_word(SelDeviceTy* dev, cudaStream_t s) {
                            : (word & 4u)  ? "Ptex filter frame stack overflow"
                            : (word & 8u)  ? "render queue overflow"
                            : (word & 16u) ? "instances nested deeper than two levels"
+                           : (word & 32u) ? "work request timed out"
                                           : "kernel iteration cap reached";
         return fail(SEL_ERR_DEVICE_LIMIT, what);
     }
     return SEL_OK;
 }
+
+uint32_t scene_stack_depth(const SelSceneTy* sc) { return std::max(1u, sc->stack_need); }
 
 DeviceBvh device_bvh(const SelSceneTy* sc) {
     DeviceBvh b;
@@ -72,6 +76,8 @@ DeviceBvh device_bvh(const SelSceneTy* sc) {
     b.nodes = sc->d_nodes;
     b.tris = static_cast<const float4*>(sc->d_tris);
     b.tri_count = uint32_t(sc->info.triangle_count);
+    b.stack_depth = int(scene_stack_depth(sc));
+    b.sm_count = sc->dev->sm_count;
     b.insts = static_cast<const InstanceRecord*>(sc->d_insts);
     for (int a = 0; a < 3; ++a) {
         b.lo[a] = sc->info.bounds_lo[a];
@@ -115,6 +121,7 @@ int sel_device_new(int cuda_device, SelDevice* out_device) {
     if (int rc = set_device(dev)) { delete dev; return rc; }
     e = cudaStreamCreateWithFlags(&dev->stream, cudaStreamNonBlocking);
     for (int k = 0; k < 4 && e == cudaSuccess; ++k) e = cudaStreamCreateWithFlags(&dev->qstream[k], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&dev->sm_count, cudaDevAttrMultiProcessorCount, cuda_device);
     if (e == cudaSuccess) e = cudaMalloc(&dev->d_err, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(dev->d_err, 0, sizeof(uint32_t));
     // The allocation-free query's staging array: resolving its address here loads its module (and so

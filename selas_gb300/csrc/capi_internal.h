@@ -15,6 +15,7 @@ struct SelDeviceTy {
     int cuda_device = 0;
     cudaStream_t stream = nullptr;  // internal stream for the host-memory entry points
     cudaStream_t qstream[4] = {nullptr, nullptr, nullptr, nullptr};  // pipelined host-memory queries (chunk k on k % 4)
+    int sm_count = 1;
     uint32_t* d_err = nullptr;      // kernel error word (iteration cap / stack overflow bits)
     cudaMemPool_t order_pool = nullptr;  // stream-ordered scratch of ordered queries (keeps freed memory)
     bool graph_replay = true;       // SEL_OPTION_GRAPH_REPLAY
@@ -152,6 +153,7 @@ int cuda_fail(cudaError_t e, const char* what);
 int set_device(SelDeviceTy* dev);
 int read_error_word(SelDeviceTy* dev, cudaStream_t s);
 DeviceBvh device_bvh(const SelSceneTy* sc);
+uint32_t scene_stack_depth(const SelSceneTy* sc);  // traversal stack entries a ray of the committed scene may need
 // noalloc.cu: looks up the device address of the fixed staging array on dev's GPU (dev's device current)
 int resolve_noalloc_staging(SelDeviceTy* dev);
 }  // namespace sel

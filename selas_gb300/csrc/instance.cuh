@@ -20,6 +20,7 @@
 namespace sel {
 
 constexpr uint32_t kErrInstanceDepth = 16u;  // an instance below the second level (commit prevents it)
+constexpr uint32_t kPendingLeaf = 0x80000000u;  // stack entries: leaf records (base | this, mask); bases lie below 2^31
 
 // Affine transforms with every rounding fixed (fmaf chains), so that the CPU oracle's std::fma restatement
 // transforms rays bit for bit alike.  Rows r0..r2 of a 3 x 4 matrix.
@@ -57,7 +58,6 @@ struct InstState {
     const InstanceRecord* chain0;      // entered instances (kept in named fields so that the state
     const InstanceRecord* chain1;      // stays in registers)
     int level;
-    uint2 pend;                        // leaf records still to test at this level (y = bit mask; 0: none)
     uint64_t cur_inst, best_inst;      // (instID[0] << 32 | instID[1]) of the current level / the best hit
     InstHit hit;
 };
@@ -112,7 +112,6 @@ __device__ __forceinline__ void inst_init(InstState& s, const QueryRay& r, const
     s.chain0 = s.chain1 = nullptr;
     s.level = 0;
     inst_level_pointers(s);
-    s.pend = make_uint2(0u, 0u);
     s.best_inst = ~0ull;
     s.hit.tri = 0xffffffffu;
     s.hit.tris = nullptr;
@@ -129,51 +128,64 @@ __device__ __forceinline__ void inst_record_hit(InstState& s, float t, float u, 
     s.hit.inst[1] = uint32_t(s.cur_inst);
 }
 
-// One step: a node visit (or a pending leaf) and the leaf records it exposes.  Returns true when the ray is
-// finished (any-hit: on the first hit).
-template <bool kAnyHit>
-__device__ __forceinline__ bool inst_step(InstState& s, uint2* stack, int stride, uint32_t& status) {
-    uint32_t tmask = 0, tbase = 0;
-    if (s.pend.y) {
-        tbase = s.pend.x;
-        tmask = s.pend.y;
-        s.pend = make_uint2(0u, 0u);
-    } else if (s.w.group.y & 0xff000000u) {
-        if (!wide_visit<kInstStack>(s.w, s.nodes, stack, stride, status, tmask, tbase)) return true;
+// The instanced traversal of one lane, as trace_stream steps it.
+struct InstWalk {
+    InstState s;
+    uint32_t tmask, tbase;  // leaf records of the current level still to test: bit k is record tbase + k
+
+    template <typename Rays>
+    __device__ __forceinline__ bool start(const QueryRay& r, const Rays& rays) {
+        inst_init(s, r, rays.nodes(), rays.tris(), rays.insts());
+        tmask = 0;
+        return !ray_untraceable(r);
     }
-    while (tmask) {
-        const int b = __ffs(tmask) - 1;
+
+    // Enters the instance of leaf record words p0: pushes what is left of the current node and leaf and a level
+    // marker, and goes on at the instanced BVH's root.  Returns false when a limit is reached.
+    __device__ __forceinline__ bool enter(const float4& p0, const WideStack& stack, uint32_t& status) {
+        if (s.level >= 2) {
+            status |= kErrInstanceDepth;
+            return true;  // the record is skipped
+        }
+        const bool more = (s.w.group.y & 0xff000000u) != 0u;
+        const int need = (more ? 1 : 0) + (tmask ? 1 : 0) + 1;
+        if (s.w.sp + need > stack.depth) {
+            status |= kErrStackOverflow;
+            return false;
+        }
+        if (more) stack.mem[(s.w.sp++) * stack.stride] = s.w.group;
+        if (tmask) stack.mem[(s.w.sp++) * stack.stride] = make_uint2(tbase | kPendingLeaf, tmask);
+        stack.mem[(s.w.sp++) * stack.stride] = make_uint2(0u, 0u);  // level marker
+        if (s.level == 0) s.chain0 = s.insts + __float_as_uint(p0.w);
+        else s.chain1 = s.insts + __float_as_uint(p0.w);
+        ++s.level;
+        inst_level_pointers(s);
+        inst_level_ray(s);
+        QueryRay lr;
+        lr.ox = s.w.ox; lr.oy = s.w.oy; lr.oz = s.w.oz;
+        lr.dx = s.w.dx; lr.dy = s.w.dy; lr.dz = s.w.dz;
+        // the instanced BVH's root; nothing to do in an instance the transformed ray cannot hit
+        s.w.group = ray_untraceable(lr) ? make_uint2(0u, 0u) : make_uint2(0u, (1u << (24 + s.w.oct)) | 1u);
+        tmask = 0;
+        return true;
+    }
+
+    __device__ __forceinline__ bool pending() const { return tmask != 0u; }
+
+    template <typename Rays>
+    __device__ __forceinline__ bool visit(const Rays&, const WideStack& stack, uint32_t& status) {
+        return !(s.w.group.y & 0xff000000u) || wide_visit(s.w, s.nodes, stack, status, tmask, tbase);
+    }
+
+    // Takes one pending leaf record: an instance is entered, a triangle or curve segment tested.  False: the ray is
+    // finished (any-hit: on the first hit).
+    template <bool kAnyHit, typename Rays>
+    __device__ __forceinline__ bool test(const Rays&, const WideStack& stack, uint32_t& status) {
+        const uint32_t ti = tbase + uint32_t(__ffs(tmask) - 1);
         tmask &= tmask - 1u;
-        const uint32_t ti = tbase + uint32_t(b);
         const float4* tp = s.tris + size_t(ti) * 3;
         const float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
-        if (__float_as_uint(p1.w) == kInstanceGeom) {
-            if (s.level >= 2) {
-                status |= kErrInstanceDepth;
-                continue;
-            }
-            const bool more = (s.w.group.y & 0xff000000u) != 0u;
-            const int need = (more ? 1 : 0) + (tmask ? 1 : 0) + 1;
-            if (s.w.sp + need > kInstStack) {
-                status |= kErrStackOverflow;
-                return true;
-            }
-            if (more) stack[(s.w.sp++) * stride] = s.w.group;
-            if (tmask) stack[(s.w.sp++) * stride] = make_uint2(tbase, tmask);
-            stack[(s.w.sp++) * stride] = make_uint2(0u, 0u);  // level marker
-            if (s.level == 0) s.chain0 = s.insts + __float_as_uint(p0.w);
-            else s.chain1 = s.insts + __float_as_uint(p0.w);
-            ++s.level;
-            inst_level_pointers(s);
-            inst_level_ray(s);
-            QueryRay lr;
-            lr.ox = s.w.ox; lr.oy = s.w.oy; lr.oz = s.w.oz;
-            lr.dx = s.w.dx; lr.dy = s.w.dy; lr.dz = s.w.dz;
-            // the instanced BVH's root; nothing to do in an instance the transformed ray cannot hit
-            s.w.group = ray_untraceable(lr) ? make_uint2(0u, 0u) : make_uint2(0u, (1u << (24 + s.w.oct)) | 1u);
-            tmask = 0;
-            break;
-        }
+        if (__float_as_uint(p1.w) == kInstanceGeom) return enter(p0, stack, status);
         float t, u, v;
         bool hit;
         if (__float_as_uint(p2.w) == kTriCurve) {  // a round B-spline curve segment (curve.cuh)
@@ -183,61 +195,43 @@ __device__ __forceinline__ bool inst_step(InstState& s, uint2* stack, int stride
         } else {
             hit = watertight_intersect(s.w.wt, s.w.ox, s.w.oy, s.w.oz, p0, p1, p2, s.w.tnear, s.w.tfar, t, u, v);
         }
-        if (hit) {
-            if (kAnyHit) {
-                inst_record_hit(s, t, u, v, ti);
-                return true;
-            }
-            const uint64_t key = tri_key(p0, p1);
-            if (t < s.w.tfar || s.cur_inst < s.best_inst || (s.cur_inst == s.best_inst && key < s.w.best_key)) {
-                s.w.tfar = t;
-                s.w.best_key = key;
-                s.best_inst = s.cur_inst;
-                inst_record_hit(s, t, u, v, ti);
+        if (!hit) return true;
+        bool take = t < s.w.tfar || s.hit.tri == 0xffffffffu || s.cur_inst < s.best_inst;
+        if (!take && s.cur_inst == s.best_inst) {  // a tie within one instance: the smaller (geomID, primID)
+            const float4* bp = s.hit.tris + size_t(s.hit.tri) * 3;
+            take = tri_key(p0, p1) < tri_key(__ldg(bp), __ldg(bp + 1));
+        }
+        if (take) {
+            s.w.tfar = t;
+            s.best_inst = s.cur_inst;
+            inst_record_hit(s, t, u, v, ti);
+        }
+        return !kAnyHit;
+    }
+
+    // Ends a step: with nothing pending, pops node groups, leaf records and level markers until there is work.
+    // False: the ray is finished.
+    __device__ __forceinline__ bool advance(const WideStack& stack, uint32_t& status) {
+        if (++s.w.iters > kIterationCap) {
+            status |= kErrIterationCap;
+            return false;
+        }
+        while (!tmask && !(s.w.group.y & 0xff000000u)) {
+            if (s.w.sp == 0) return false;
+            const uint2 e = stack.mem[(--s.w.sp) * stack.stride];
+            if (e.y == 0u) {  // level marker: back to the parent level
+                --s.level;
+                inst_level_pointers(s);
+                inst_level_ray(s);
+            } else if (e.x & kPendingLeaf) {
+                tbase = e.x & ~kPendingLeaf;
+                tmask = e.y;
+            } else {
+                s.w.group = e;
             }
         }
-    }
-    if (++s.w.iters > kIterationCap) {
-        status |= kErrIterationCap;
         return true;
     }
-    while (!(s.w.group.y & 0xff000000u) && !s.pend.y) {
-        if (s.w.sp == 0) return true;
-        const uint2 e = stack[(--s.w.sp) * stride];
-        if (e.y == 0u) {  // level marker: back to the parent level
-            --s.level;
-            inst_level_pointers(s);
-            inst_level_ray(s);
-        } else if ((e.y >> 24) == 0u) {
-            s.pend = e;
-        } else {
-            s.w.group = e;
-        }
-    }
-    return false;
-}
-
-// Render-kernel policy of the instanced traversal (the flat layouts are Tracer<0> and Tracer<1>).
-template <>
-struct Tracer<2> {
-    using Entry = uint2;
-    static constexpr int kDepth = kInstStack;
 };
-
-// Whole-ray form (one thread, one ray) over a scene with instances.
-template <bool kAnyHit>
-__device__ __forceinline__ bool trace_instanced(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
-                                                const InstanceRecord* insts, const QueryRay& r, InstHit& hit,
-                                                uint2* stack, int stride, uint32_t& status) {
-    if (ray_untraceable(r)) {
-        hit.tri = 0xffffffffu;
-        return false;
-    }
-    InstState s;
-    inst_init(s, r, nodes, tris, insts);
-    while (!inst_step<kAnyHit>(s, stack, stride, status)) {}
-    hit = s.hit;
-    return s.hit.tri != 0xffffffffu;
-}
 
 }  // namespace sel

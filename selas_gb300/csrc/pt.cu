@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "capi_internal.h"
 #include "cmj.cuh"
@@ -51,6 +52,11 @@ constexpr float kFloatMax = 3.402823466e+38f;  // FloatMax_ (SystemLib/BasicType
 struct PtParams {
     PtState st;
     uint32_t* err;
+    int stack_depth;      // traversal stack entries per thread (8-wide layout): the jobs' deepest scene
+    // the scene of every job when they share one (null: each ray reads its job's)
+    const uint4* nodes;
+    const float4* tris;
+    const InstanceRecord* insts;
 };
 
 __device__ __forceinline__ CameraDev camera_of(const PtCamera& c) {
@@ -183,81 +189,122 @@ __device__ __forceinline__ HitRef hit_ref(const PtState& st, const PtScene& S, u
     return hit_ref_of<kInst>(S, kInst ? st.hinst[s] : make_uint2(0u, 0u), tri);
 }
 
-// Per-thread traversal stacks of a B-thread block in shared memory (entry k of thread t at k * B + t).  The
-// instanced traversal's 40-entry stacks of a 256-thread block take 80 KB: they live in dynamic shared memory
-// (launched with trace_stack_bytes<K, B>() bytes and the matching MaxDynamicSharedMemorySize attribute); every
-// other stack is a static array.
-template <int K, int B>
-constexpr size_t trace_stack_bytes() {
-    return size_t(Tracer<K>::kDepth) * B * sizeof(typename Tracer<K>::Entry);
-}
-template <int K, int B>
-constexpr bool kDynamicStack = trace_stack_bytes<K, B>() > 48u * 1024u;
+// Closest hit for the queued paths.  Persistent blocks of B threads; the 8-wide layouts trace the queue as a stream
+// (trace_stream: finished lanes are refilled while the others go on).  K = 0: 8-wide, 2: 8-wide with instances,
+// 1: the binary comparison layout, one ray a lane in packets of 32 entries.
 
-template <int K, int B>
-__device__ __forceinline__ typename Tracer<K>::Entry* trace_stack() {
-    if constexpr (kDynamicStack<K, B>) {
-        extern __shared__ __align__(16) unsigned char pt_dynamic_stack[];
-        return reinterpret_cast<typename Tracer<K>::Entry*>(pt_dynamic_stack);
-    } else {
-        __shared__ typename Tracer<K>::Entry stack_mem[Tracer<K>::kDepth * B];
-        return stack_mem;
+// Isotropic::SampleDistance (Shading/IsotropicScattering.cpp:18-47): the ray's length limit.
+__device__ __forceinline__ float medium_distance(const PtState& st, uint32_t s, const float4& med) {
+    if (med.x == 0.0f) return kFloatMax;
+    Pcg32 rng = load_rng(st, s);
+    const float ps = med.y + med.z + med.w;
+    const float pr = med.y / ps, pg = med.z / ps;
+    const float r0 = pcg_float(rng);
+    const float c = r0 < pr ? med.y : (r0 < pr + pg ? med.z : med.w);
+    const float tfar = -logf(pcg_float(rng)) / c;
+    st.rng[s] = rng.state;
+    return tfar;
+}
+
+__device__ __forceinline__ QueryRay path_ray(const PtState& st, uint32_t s) {
+    const float4 o = st.ray_o[s], d = st.ray_d[s];
+    const float4 med = st.medium[s];
+    QueryRay q;
+    q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = 0.0f;
+    q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = medium_distance(st, s, med);
+    return q;
+}
+
+// The scene a lane's ray belongs to: the one scene of the batch (kOne; kernel arguments), or its job's.
+template <bool kOne>
+struct LaneScene;
+template <>
+struct LaneScene<true> {
+    const PtParams& P;
+    __device__ __forceinline__ explicit LaneScene(const PtParams& p) : P(p) {}
+    __device__ __forceinline__ void take(uint32_t) {}
+    __device__ __forceinline__ const uint4* nodes() const { return P.nodes; }
+    __device__ __forceinline__ const float4* tris() const { return P.tris; }
+    __device__ __forceinline__ const InstanceRecord* insts() const { return P.insts; }
+};
+template <>
+struct LaneScene<false> {
+    const PtParams& P;
+    const uint4* n;
+    const float4* t;
+    const InstanceRecord* i;
+    __device__ __forceinline__ explicit LaneScene(const PtParams& p) : P(p), n(nullptr), t(nullptr), i(nullptr) {}
+    __device__ __forceinline__ void take(uint32_t job) {
+        const PtScene& sc = P.st.jobs[job].scene;
+        n = static_cast<const uint4*>(sc.nodes);
+        t = sc.tris;
+        i = sc.insts;
     }
-}
+    __device__ __forceinline__ const uint4* nodes() const { return n; }
+    __device__ __forceinline__ const float4* tris() const { return t; }
+    __device__ __forceinline__ const InstanceRecord* insts() const { return i; }
+};
 
-// Closest hit for the queued paths.  Warps take 32-entry packets from the queue through an atomic cursor,
-// so expensive and cheap rays balance across the GPU.  K = 2: the instanced traversal of the 8-wide layout.
+template <bool kOne>
+struct PathRays : QueueRanges, LaneScene<kOne> {
+    const PtState& st;
+    const uint32_t* queue;
+    __device__ __forceinline__ PathRays(const PtParams& P, const uint32_t* q, uint32_t n)
+        : QueueRanges(n, &P.st.counters[3]), LaneScene<kOne>(P), st(P.st), queue(q) {}
+    __device__ __forceinline__ bool begin(uint32_t e, QueryRay& r) {
+        const uint32_t s = queue[e];
+        if constexpr (!kOne) this->take(st.job[s]);
+        r = path_ray(st, s);
+        return true;
+    }
+    __device__ __forceinline__ void end(uint32_t e, const WideState& h) const {
+        const bool found = h.hit.tri != 0xffffffffu;
+        st.hit[queue[e]] = make_float4(h.tfar, found ? h.hit.u : 0.0f, found ? h.hit.v : 0.0f,
+                                       __uint_as_float(h.hit.tri));
+    }
+    __device__ __forceinline__ void end(uint32_t e, const InstState& h) const {
+        const uint32_t s = queue[e];
+        const bool found = h.hit.tri != 0xffffffffu;
+        st.hit[s] = make_float4(h.w.tfar, found ? h.hit.u : 0.0f, found ? h.hit.v : 0.0f,
+                                __uint_as_float(h.hit.tri));
+        st.hinst[s] = found ? inst_indices(h.top_insts, h.hit) : make_uint2(0u, 0u);
+    }
+};
+
+extern __shared__ uint2 pt_stack[];
+
 template <int K, int B>
-__global__ void __launch_bounds__(B, K == 2 ? 512 / B : 1024 / B) k_extend(PtParams P, int cur) {
-    typename Tracer<K>::Entry* stack_mem = trace_stack<K, B>();
+constexpr int kTraceBlocksPerSm = (K == 2 ? 512 : 1024) / B;
+
+template <int K, int B, bool kOne>
+__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_extend(const __grid_constant__ PtParams P, int cur) {
     const uint32_t n = P.st.counters[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays, (unsigned long long)n);
     const uint32_t* queue = P.st.queue[cur];
     uint32_t status = 0;
-    for (;;) {
-        uint32_t base = 0;
-        if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[3], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const uint32_t e = base + (threadIdx.x & 31u);
-        if (e < n) {
-            const uint32_t s = queue[e];
-            const float4 o = P.st.ray_o[s], d = P.st.ray_d[s];
-            const float4 med = P.st.medium[s];
-            float tfar = kFloatMax;
-            if (med.x != 0.0f) {
-                // Isotropic::SampleDistance (Shading/IsotropicScattering.cpp:18-47)
-                Pcg32 rng = load_rng(P.st, s);
-                const float ps = med.y + med.z + med.w;
-                const float pr = med.y / ps, pg = med.z / ps, pb = med.w / ps;
-                float c, p;
-                const float r0 = pcg_float(rng);
-                if (r0 < pr) { c = med.y; p = pr; }
-                else if (r0 < pr + pg) { c = med.z; p = pg; }
-                else { c = med.w; p = pb; }
-                (void)p;
-                tfar = -logf(pcg_float(rng)) / c;
-                P.st.rng[s] = rng.state;
-            }
-            QueryRay q;
-            q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = 0.0f;
-            q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = tfar;
-            const PtScene& sc = P.st.jobs[P.st.job[s]].scene;
-            if constexpr (K == 2) {
-                InstHit h;
-                const bool found = trace_instanced<false>(static_cast<const uint4*>(sc.nodes), sc.tris, sc.insts, q,
-                                                          h, stack_mem + threadIdx.x, B, status);
-                P.st.hit[s] = found ? make_float4(h.t, h.u, h.v, __uint_as_float(h.tri))
-                                    : make_float4(tfar, 0.0f, 0.0f, __uint_as_float(0xffffffffu));
-                P.st.hinst[s] = found ? inst_indices(sc.insts, h) : make_uint2(0u, 0u);
-            } else {
+    if constexpr (K == 1) {
+        __shared__ int stack_mem[kBinaryStack * B];
+        for (;;) {
+            uint32_t base = 0;
+            if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[3], 32u);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= n) break;
+            const uint32_t e = base + (threadIdx.x & 31u);
+            if (e < n) {
+                const uint32_t s = queue[e];
+                const QueryRay q = path_ray(P.st, s);
+                const PtScene& sc = P.st.jobs[P.st.job[s]].scene;
                 QueryHit h;
-                const bool found = Tracer<K>::template trace<false>(sc.nodes, sc.tris, q, h, stack_mem + threadIdx.x,
-                                                                    B, status);
+                const bool found = trace_binary<false>(static_cast<const float4*>(sc.nodes), sc.tris, q, h,
+                                                       stack_mem + threadIdx.x, B, status);
                 P.st.hit[s] = found ? make_float4(h.t, h.u, h.v, __uint_as_float(h.tri))
-                                    : make_float4(tfar, 0.0f, 0.0f, __uint_as_float(0xffffffffu));
+                                    : make_float4(q.tfar, 0.0f, 0.0f, __uint_as_float(0xffffffffu));
             }
         }
+    } else {
+        PathRays<kOne> rays(P, queue, n);
+        using Walk = std::conditional_t<K == 2, InstWalk, WideWalk>;
+        trace_stream<false, Walk>(rays, WideStack{pt_stack + threadIdx.x, B, P.stack_depth}, status);
     }
     if (status) atomicOr(P.err, status);
 }
@@ -645,40 +692,61 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
     }
 }
 
-template <int K, int B>
-__global__ void __launch_bounds__(B, K == 2 ? 512 / B : 1024 / B) k_shadow(PtParams P) {
-    typename Tracer<K>::Entry* stack_mem = trace_stack<K, B>();
+// The queued shadow rays of the batch.
+template <bool kOne>
+struct ShadowRays : QueueRanges, LaneScene<kOne> {
+    const PtState& st;
+    __device__ __forceinline__ ShadowRays(const PtParams& P, uint32_t n)
+        : QueueRanges(n, &P.st.counters[4]), LaneScene<kOne>(P), st(P.st) {}
+    __device__ __forceinline__ bool begin(uint32_t e, QueryRay& q) {
+        if constexpr (!kOne) this->take(__float_as_uint(st.sh_c[e].w) >> 28);
+        const float4 o = st.sh_o[e], d = st.sh_d[e];
+        q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = o.w;
+        q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = d.w;
+        return true;
+    }
+    __device__ __forceinline__ void add(uint32_t e) const {
+        const float4 c = st.sh_c[e];
+        const uint32_t tag = __float_as_uint(c.w);
+        const PtJob& J = st.jobs[tag >> 28];
+        accumulate(J.accum, J.cam.width * J.cam.height, J.mode == kPtModeDeferred ? 0 : 1, tag & 0x0fffffffu,
+                   f3(c.x, c.y, c.z));
+    }
+    __device__ __forceinline__ void end(uint32_t e, const WideState& h) const {
+        if (h.hit.tri == 0xffffffffu) add(e);
+    }
+    __device__ __forceinline__ void end(uint32_t e, const InstState& h) const {
+        if (h.hit.tri == 0xffffffffu) add(e);
+    }
+};
+
+template <int K, int B, bool kOne>
+__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_shadow(const __grid_constant__ PtParams P) {
     const uint32_t n = P.st.counters[2];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays + 1, (unsigned long long)n);
     uint32_t status = 0;
-    for (;;) {
-        uint32_t base = 0;
-        if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[4], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const uint32_t e = base + (threadIdx.x & 31u);
-        if (e < n) {
-            const float4 o = P.st.sh_o[e], d = P.st.sh_d[e];
-            const float4 c = P.st.sh_c[e];
-            const uint32_t tag = __float_as_uint(c.w);
-            const PtJob& J = P.st.jobs[tag >> 28];
-            QueryRay q;
-            q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = o.w;
-            q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = d.w;
-            bool blocked;
-            if constexpr (K == 2) {
-                InstHit h;
-                blocked = trace_instanced<true>(static_cast<const uint4*>(J.scene.nodes), J.scene.tris, J.scene.insts,
-                                                q, h, stack_mem + threadIdx.x, B, status);
-            } else {
+    if constexpr (K == 1) {
+        __shared__ int stack_mem[kBinaryStack * B];
+        for (;;) {
+            uint32_t base = 0;
+            if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[4], 32u);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= n) break;
+            const uint32_t e = base + (threadIdx.x & 31u);
+            if (e < n) {
+                ShadowRays<false> rays(P, n);
+                QueryRay q;
+                rays.begin(e, q);
                 QueryHit h;
-                blocked = Tracer<K>::template trace<true>(J.scene.nodes, J.scene.tris, q, h, stack_mem + threadIdx.x, B,
-                                                          status);
+                if (!trace_binary<true>(reinterpret_cast<const float4*>(rays.nodes()), rays.tris(), q, h,
+                                        stack_mem + threadIdx.x, B, status))
+                    rays.add(e);
             }
-            if (!blocked)
-                accumulate(J.accum, J.cam.width * J.cam.height, J.mode == kPtModeDeferred ? 0 : 1, tag & 0x0fffffffu,
-                           f3(c.x, c.y, c.z));
         }
+    } else {
+        ShadowRays<kOne> rays(P, n);
+        using Walk = std::conditional_t<K == 2, InstWalk, WideWalk>;
+        trace_stream<true, Walk>(rays, WideStack{pt_stack + threadIdx.x, B, P.stack_depth}, status);
     }
     if (status) atomicOr(P.err, status);
 }
@@ -814,23 +882,40 @@ void launch_shade(uint32_t modes, bool inst, int shader, int grid, cudaStream_t 
     }
 }
 
+// Calls f(K, block threads, one scene) with the traversal kernels' template arguments as constants.
+template <typename F>
+void launch_trace(int bvh_kind, bool instanced, int tb, bool one_scene, F f) {
+    using std::integral_constant;
+    auto with_block = [&](auto k) {
+        auto with_scene = [&](auto b) {
+            if (one_scene) f(k, b, std::true_type{});
+            else f(k, b, std::false_type{});
+        };
+        if (tb == 256) with_scene(integral_constant<int, 256>{});
+        else with_scene(integral_constant<int, 128>{});
+    };
+    if (instanced) with_block(integral_constant<int, 2>{});
+    else if (bvh_kind == 0) with_block(integral_constant<int, 0>{});
+    else f(integral_constant<int, 1>{}, integral_constant<int, 128>{}, std::false_type{});
+}
+
 cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtState& st, uint32_t* d_err,
                            uint64_t batches, cudaStream_t stream, GraphCache* graphs, int trace_block, uint32_t modes,
                            bool instanced, bool texture, bool ray_sort, uint64_t batch_paths, uint32_t shader_kinds,
-                           bool quad_ptex) {
+                           bool quad_ptex, int stack_depth, const PtScene* one_scene) {
     const bool face_order = sort && texture && !instanced && batch_paths >= kFaceOrderPaths;
-    // 256-thread traversal blocks for the 8-wide layout, flat (its 24-entry stacks fill 48 KB of static shared
-    // memory) or instanced (40-entry stacks, 80 KB of dynamic shared memory); the binary layout's 64-entry
-    // stacks stay at 128 threads
+    // 256-thread traversal blocks for the 8-wide layout; the binary layout's 64-entry stacks stay at 128 threads
     const int tb = (trace_block == 256 && bvh_kind == 0) ? 256 : 128;
-    constexpr size_t kInstStackBytes = trace_stack_bytes<2, 256>();
-    if (instanced && tb == 256) {
-        cudaError_t e = cudaFuncSetAttribute(k_extend<2, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(kInstStackBytes));
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_shadow<2, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(kInstStackBytes));
-        if (e != cudaSuccess) return e;
+    const size_t stack_bytes = bvh_kind == 0 ? size_t(stack_depth) * size_t(tb) * sizeof(uint2) : 0;
+    if (stack_bytes > 48u * 1024u) {  // deep instanced scenes with 256-thread blocks
+        for (const void* f : {reinterpret_cast<const void*>(&k_extend<2, 256, true>),
+                              reinterpret_cast<const void*>(&k_extend<2, 256, false>),
+                              reinterpret_cast<const void*>(&k_shadow<2, 256, true>),
+                              reinterpret_cast<const void*>(&k_shadow<2, 256, false>)}) {
+            const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       int(kInstStack * 256 * sizeof(uint2)));
+            if (e != cudaSuccess) return e;
+        }
     }
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -839,7 +924,23 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
     std::memset(&P, 0, sizeof(P));
     P.st = st;
     P.err = d_err;
-    const int trace_grid = grid_for(sms, 1024 / tb);
+    P.stack_depth = stack_depth;
+    if (one_scene) {
+        P.nodes = static_cast<const uint4*>(one_scene->nodes);
+        P.tris = one_scene->tris;
+        P.insts = one_scene->insts;
+    }
+    const int trace_grid = grid_for(sms, (instanced ? 512 : 1024) / tb);
+    auto extend = [&](cudaStream_t s, int cur) {
+        launch_trace(bvh_kind, instanced, tb, one_scene != nullptr, [&](auto k, auto b, auto one) {
+            k_extend<k.value, b.value, one.value><<<trace_grid, tb, stack_bytes, s>>>(P, cur);
+        });
+    };
+    auto shadow = [&](cudaStream_t s) {
+        launch_trace(bvh_kind, instanced, tb, one_scene != nullptr, [&](auto k, auto b, auto one) {
+            k_shadow<k.value, b.value, one.value><<<trace_grid, tb, stack_bytes, s>>>(P);
+        });
+    };
     const int shade_grid = grid_for(sms, 8);
     const int gen_grid = int((st.capacity + kBlock - 1) / kBlock);
     // the shading kernel (4 or 5 resident blocks per SM) runs one resident wave of grid-striding blocks, sized by
@@ -865,11 +966,7 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
         for (uint32_t b = 0; b < bounces; ++b) {
             const int cur = int(b & 1u);
             k_bounce_reset<<<1, 32, 0, s>>>(st.counters, cur ^ 1);
-            if (instanced && tb == 256) k_extend<2, 256><<<trace_grid, tb, kInstStackBytes, s>>>(P, cur);
-            else if (instanced) k_extend<2, 128><<<trace_grid, tb, 0, s>>>(P, cur);
-            else if (bvh_kind == 0 && tb == 256) k_extend<0, 256><<<trace_grid, tb, 0, s>>>(P, cur);
-            else if (bvh_kind == 0) k_extend<0, 128><<<trace_grid, tb, 0, s>>>(P, cur);
-            else k_extend<1, 128><<<trace_grid, tb, 0, s>>>(P, cur);
+            extend(s, cur);
             if (face_order) {
                 // textured scenes, large batches: order by (class, Ptex face, footprint region), three 8-bit
                 // radix passes from the queue to queue_sorted (through rvals)
@@ -917,11 +1014,7 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
             } else {
                 launch_shade(modes, instanced, -1, wave_grid, s, P, cur, b, q, whole);
             }
-            if (instanced && tb == 256) k_shadow<2, 256><<<trace_grid, tb, kInstStackBytes, s>>>(P);
-            else if (instanced) k_shadow<2, 128><<<trace_grid, tb, 0, s>>>(P);
-            else if (bvh_kind == 0 && tb == 256) k_shadow<0, 256><<<trace_grid, tb, 0, s>>>(P);
-            else if (bvh_kind == 0) k_shadow<0, 128><<<trace_grid, tb, 0, s>>>(P);
-            else k_shadow<1, 128><<<trace_grid, tb, 0, s>>>(P);
+            shadow(s);
             if (ray_sort && b + 1 < bounces) {
                 // order the next bounce's queue by (direction bin, origin cell): two 8-bit radix passes, the
                 // queue ping-ponging through rvals
@@ -991,7 +1084,7 @@ cudaError_t pt_render(const PtScene& sc, const PtCamera& cam, const PtSettings& 
     return pt_run_batches(sc.bvh_kind, set.max_bounces, sc.sort_hint != 0, st, d_err, batches, stream, graphs,
                           trace_block, set.mode == kPtModeDeferred ? 2u : 1u, sc.insts != nullptr,
                           pt_scene_textured(sc), sc.ray_sort != 0, std::min<uint64_t>(job.total, st.capacity),
-                          sc.shader_kinds, sc.ptex_quads != 0);
+                          sc.shader_kinds, sc.ptex_quads != 0, int(sc.stack_depth), &sc);
 }
 
 cudaError_t pt_resolve(const double* d_accum, uint32_t values, double scale, float* d_out, cudaStream_t stream) {

@@ -1,5 +1,5 @@
 // Ray-query kernels over SelRay / SelRayHit records (Embree's RTCRay / RTCRayHit layouts) and their
-// launchers.  One thread per ray; each thread keeps its traversal stack in shared memory.
+// launchers.  One lane per ray; each thread keeps its traversal stack in shared memory.
 #include "query.h"
 
 #include "hitref.cuh"
@@ -12,7 +12,7 @@ namespace sel {
 
 namespace {
 
-constexpr int kQueryBlock = 128;
+constexpr int kQueryBlock = 128;  // the binary layout's blocks
 
 __device__ __forceinline__ QueryRay load_ray(const float4* rp) {
     const float4 a = rp[0], b = rp[1], c = rp[2];
@@ -75,74 +75,196 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
     reinterpret_cast<uint32_t*>(base)[20] = h.inst[1];
 }
 
-// Scenes with instances: one thread per ray, the instanced traversal with its deeper shared-memory stack.
-template <bool kAnyHit>
-__global__ void __launch_bounds__(kQueryBlock)
-    k_query_instanced(const uint4* __restrict__ nodes, const float4* __restrict__ tris, const InstanceRecord* insts,
-                      float4* rays, uint32_t record_float4s, uint32_t n, uint32_t* err) {
-    __shared__ uint2 stack_mem[kInstStack * kQueryBlock];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    InstHit h;
-    uint32_t status = 0;
-    const bool found = trace_instanced<kAnyHit>(nodes, tris, insts, load_ray(rays + size_t(i) * record_float4s), h,
-                                                stack_mem + threadIdx.x, kQueryBlock, status);
-    if (status) atomicOr(err, status);
-    if (found) {
-        if (kAnyHit)
-            reinterpret_cast<float*>(rays + size_t(i) * record_float4s)[8] = -__int_as_float(0x7f800000);
-        else
-            store_hit_instanced(reinterpret_cast<SelRayHit*>(rays + size_t(i) * record_float4s), h);
+// ---------------------------------------------------------------------------------------------------
+// 8-wide traversal.  Blocks are one warp and block index k stands for records [32 k, 32 k + 32).  A warp whose
+// lanes run out of rays takes over the block index of a block that has not started (cluster launch control) and
+// refills its finished lanes from it (trace_stream), so a batch of any size is balanced without a work counter in
+// memory, on any number of streams at once and under graph capture.  The next index is requested while the
+// warp still traces the last, which hides the answer's latency.  An atomic counter in place of the block indices
+// measured 3 % faster (4 M incoherent rays over 5.2 M triangles, closest hit 1.81 against 1.87 ms) but would have to
+// be allocated and zeroed by every call.
+// 64 registers, 32 warps per SM: with 36 (56 registers) closest hit takes 1.89 against 1.81 ms and any hit 1.34
+// against 1.22, with 40 (48 registers) 2.08 and 1.46.  Whole calls on that scene, start of a call to its end: closest
+// hit 2.92 ms with one thread per ray and a 24-entry stack, 1.95 now; any hit 1.95 and 1.33; camera rays 0.50 and
+// 0.45, any hit 0.28 and 0.27.
+// ---------------------------------------------------------------------------------------------------
+constexpr int kWarpsPerSm = 32;
+constexpr uint32_t kErrClaimTimeout = 32u;  // the answer to a work request never came
+
+__device__ __forceinline__ uint32_t shared_address(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
+
+// The records a warp traces.  kOrdered: record `order[i]` in place of record i when ctl[0] is non-zero.
+struct RecordRanges {
+    uint32_t n, status;
+    bool claim, started;     // claim: more blocks were launched than run at once
+    uint32_t phase;
+    uint32_t answer, barrier;  // shared memory: 16-byte answer, its mbarrier
+
+    __device__ __forceinline__ RecordRanges(uint32_t count, bool more_blocks, const uint4* ans, const uint64_t* bar)
+        : n(count), status(0), claim(more_blocks), started(false), phase(0), answer(shared_address(ans)),
+          barrier(shared_address(bar)) {
+        if (!claim) return;
+        if ((threadIdx.x & 31u) == 0) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barrier) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncwarp();
+        request();
     }
+
+    __device__ __forceinline__ void request() {
+        if ((threadIdx.x & 31u) != 0) return;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the last answer was read
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" ::"r"(barrier) : "memory");
+        asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                     ::"r"(answer), "r"(barrier) : "memory");
+    }
+
+    // The whole warp: waits for the answer; true and a block index when a block was taken over.  After a refusal
+    // no further request is made (there is nothing left to take).
+    __device__ __forceinline__ bool claimed(uint32_t& block) {
+        uint32_t done = 0;
+        for (uint32_t k = 0; k < (1u << 20) && !done; ++k)
+            asm volatile("{\n\t.reg .pred p;\n\t"
+                         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                         "selp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(done) : "r"(barrier), "r"(phase) : "memory");
+        if (!done) {
+            status |= kErrClaimTimeout;
+            return false;
+        }
+        phase ^= 1u;
+        uint32_t got = 0;
+        asm volatile("{\n\t.reg .b128 a;\n\t.reg .pred p;\n\t.reg .b64 lo, hi;\n\t"
+                     "ld.shared.v2.b64 {lo, hi}, [%2];\n\tmov.b128 a, {lo, hi};\n\t"
+                     "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+                     "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, a;\n\t}"
+                     : "=r"(got), "=r"(block) : "r"(answer) : "memory");
+        __syncwarp();
+        return got != 0;
+    }
+
+    __device__ __forceinline__ bool next(uint32_t& b, uint32_t& e) {
+        uint32_t block = blockIdx.x;
+        if (started) {
+            if (!claim) return false;
+            if (!claimed(block)) {
+                claim = false;
+                return false;
+            }
+            request();
+        }
+        started = true;
+        b = block * 32u;
+        e = n - b < 32u ? n : b + 32u;
+        return true;
+    }
+};
+
+template <bool kAnyHit, bool kInst>
+struct RecordRays : RecordRanges {
+    const uint4* node_array;
+    const float4* tri_array;
+    const InstanceRecord* inst_array;
+    float4* recs;
+    uint32_t record_float4s;
+    const uint32_t* order;  // null: records in their own order
+
+    using RecordRanges::RecordRanges;
+
+    __device__ __forceinline__ const uint4* nodes() const { return node_array; }
+    __device__ __forceinline__ const float4* tris() const { return tri_array; }
+    __device__ __forceinline__ const InstanceRecord* insts() const { return inst_array; }
+    __device__ __forceinline__ float4* record(uint32_t i) const {
+        return recs + size_t(order ? order[i] : i) * record_float4s;
+    }
+    __device__ __forceinline__ bool begin(uint32_t i, QueryRay& r) const {
+        r = load_ray(record(i));
+        return true;
+    }
+    __device__ __forceinline__ void end(uint32_t i, WideState& s) const {
+        if (s.hit.tri == 0xffffffffu) return;
+        float4* rec = record(i);
+        if constexpr (kAnyHit) {
+            reinterpret_cast<float*>(rec)[8] = -__int_as_float(0x7f800000);
+        } else {
+            s.hit.t = s.tfar;
+            store_hit(reinterpret_cast<SelRayHit*>(rec), tri_array, s.hit);
+        }
+    }
+    __device__ __forceinline__ void end(uint32_t i, InstState& s) const {
+        if (s.hit.tri == 0xffffffffu) return;
+        float4* rec = record(i);
+        if constexpr (kAnyHit) reinterpret_cast<float*>(rec)[8] = -__int_as_float(0x7f800000);
+        else store_hit_instanced(reinterpret_cast<SelRayHit*>(rec), s.hit);
+    }
+};
+
+struct QueryArgs {
+    const uint4* nodes;
+    const float4* tris;
+    const InstanceRecord* insts;
+    float4* rays;
+    uint32_t record_float4s, n;
+    const uint32_t* order;  // with ctl: the records' order, used when ctl[0] is non-zero
+    const uint32_t* ctl;
+    int stack_depth;
+    uint32_t claim;
+    uint32_t* err;
+};
+
+template <bool kAnyHit, bool kInst, typename Walk>
+__device__ __forceinline__ void query_warp(const QueryArgs& a) {
+    extern __shared__ uint2 query_stack[];
+    __shared__ __align__(16) uint4 answer;
+    __shared__ __align__(8) uint64_t barrier;
+    RecordRays<kAnyHit, kInst> rays(a.n, a.claim != 0, &answer, &barrier);
+    rays.node_array = a.nodes;
+    rays.tri_array = a.tris;
+    rays.inst_array = a.insts;
+    rays.recs = a.rays;
+    rays.record_float4s = a.record_float4s;
+    rays.order = a.ctl && a.ctl[0] ? a.order : nullptr;
+    uint32_t status = 0;
+    trace_stream<kAnyHit, Walk>(rays, WideStack{query_stack + threadIdx.x, 32, a.stack_depth}, status);
+    status |= rays.status;
+    if (status) atomicOr(a.err, status);
 }
 
-// 8-wide traversal: one thread per ray over the whole batch, 8 resident 128-thread blocks per SM for closest
-// hit (64 registers, 24 KB of shared-memory stacks per block).  A sweep of persistent variants that refill
-// finished lanes from per-warp ray blocks was slower on both coherent and incoherent rays (lanes lose
-// the lockstep that makes node fetches shared), so the hardware block scheduler does the balancing.
-// Postponing a lane's leaf triangles while few lanes of its warp test triangles (Ylitie, Karras, Laine 2017)
-// was slower too at every threshold tried (6, 10, 16 lanes: incoherent closest hit 1,382 / 1,376 / 1,356
-// against 1,418 Mrays/s without), with identical hits.  So was prefetching, before each step's leaf tests, the
-// lines of its leaf records and of the node the next step visits (prefetch.global.L1 / .L2): incoherent closest
-// hit 1,417 against 1,431 Mrays/s, and the Cornell box's path tracer 11 % slower.  Node loads marked L2
-// evict_last (createpolicy + ld.global.nc.L2::cache_hint) left every set unchanged (1,432 against 1,431).
-// Nine blocks per SM (56 registers, a few bytes spilled) help the any-hit kernel (incoherent 2,069 against
-// 2,026 Mrays/s) and slow the closest-hit one (1,363 against 1,433), so each takes its own.  The any-hit kernel
-// tests each step's leaf triangles with the whole warp (trace_wide_warp: incoherent 2,147 against 2,068, coherent
-// 14,660 against 14,200); for closest hit the shuffles, slots and key loads cost what the fuller warps save
-// (incoherent 1,416 against 1,434, coherent 7,780 against 8,240), so it keeps one lane per ray.  Choosing per
-// step (each lane its own triangles unless one lane holds 1.5x more pairs than the warp's rounds) was slower
-// still (1,402 and 7,780): the warp-synchronous loop itself costs the closest-hit kernel.
 template <bool kAnyHit>
-constexpr int kWideBlocksPerSm = kAnyHit ? 9 : 8;
+__global__ void __launch_bounds__(32, kWarpsPerSm) k_query_wide(const __grid_constant__ QueryArgs a) {
+    query_warp<kAnyHit, false, WideWalk>(a);
+}
+
+// Scenes with instances or curves: 16 warps per SM (the walk's state takes up to 128 registers).
+template <bool kAnyHit>
+__global__ void __launch_bounds__(32, 16) k_query_instanced(const __grid_constant__ QueryArgs a) {
+    query_warp<kAnyHit, true, InstWalk>(a);
+}
 
 template <bool kAnyHit>
-__global__ void __launch_bounds__(kQueryBlock, kWideBlocksPerSm<kAnyHit>)
-    k_query_wide(const uint4* __restrict__ nodes, const float4* __restrict__ tris, float4* rays,
-                 uint32_t record_float4s, uint32_t n, uint32_t* err) {
-    __shared__ uint2 stack_mem[kWideStack * kQueryBlock];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < n;
-    QueryHit h;
-    uint32_t status = 0;
-    bool found;
-    if constexpr (kAnyHit) {  // the warp tests its leaf triangles together; lanes past the batch stay to help
-        QueryRay r{};
-        if (valid) r = load_ray(rays + size_t(i) * record_float4s);
-        found = trace_wide_warp<true>(nodes, tris, valid, r, h, stack_mem + threadIdx.x, kQueryBlock, nullptr,
-                                      status);
-    } else {
-        if (!valid) return;
-        found = trace_wide<false>(nodes, tris, load_ray(rays + size_t(i) * record_float4s), h,
-                                  stack_mem + threadIdx.x, kQueryBlock, status);
-    }
-    if (status) atomicOr(err, status);
-    if (found) {
-        if (kAnyHit)
-            reinterpret_cast<float*>(rays + size_t(i) * record_float4s)[8] = -__int_as_float(0x7f800000);
-        else
-            store_hit(reinterpret_cast<SelRayHit*>(rays + size_t(i) * record_float4s), tris, h);
-    }
+cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_float4s, uint32_t n,
+                        const uint32_t* order, const uint32_t* ctl, uint32_t* d_err, cudaStream_t s) {
+    const bool inst = bvh.insts != nullptr;
+    const uint32_t blocks = (n + 31u) / 32u;
+    QueryArgs a;
+    a.nodes = static_cast<const uint4*>(bvh.nodes);
+    a.tris = bvh.tris;
+    a.insts = bvh.insts;
+    a.rays = d_rays;
+    a.record_float4s = record_float4s;
+    a.n = n;
+    a.order = order;
+    a.ctl = ctl;
+    a.stack_depth = bvh.stack_depth;
+    // a batch whose blocks all run at once leaves none to take over
+    a.claim = blocks > uint32_t(bvh.sm_count) * (inst ? 16u : uint32_t(kWarpsPerSm)) ? 1u : 0u;
+    a.err = d_err;
+    const size_t stack_bytes = size_t(bvh.stack_depth) * 32 * sizeof(uint2);
+    if (inst) k_query_instanced<kAnyHit><<<blocks, 32, stack_bytes, s>>>(a);
+    else k_query_wide<kAnyHit><<<blocks, 32, stack_bytes, s>>>(a);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -196,38 +318,6 @@ __global__ void __launch_bounds__(256) k_order_keys(const float4* rays, uint32_t
     }
 }
 
-// The 8-wide traversal over rays taken in `order` when ctl[0] (the sorted count) is non-zero.
-template <bool kAnyHit>
-__global__ void __launch_bounds__(kQueryBlock, kWideBlocksPerSm<kAnyHit>)
-    k_query_wide_ordered(const uint4* __restrict__ nodes, const float4* __restrict__ tris, float4* rays,
-                         uint32_t record_float4s, uint32_t n, const uint32_t* __restrict__ order,
-                         const uint32_t* ctl, uint32_t* err) {
-    __shared__ uint2 stack_mem[kWideStack * kQueryBlock];
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < n;
-    const uint32_t r = !valid ? 0u : (ctl[0] ? order[i] : i);
-    QueryHit h;
-    uint32_t status = 0;
-    bool found;
-    if constexpr (kAnyHit) {
-        QueryRay ray{};
-        if (valid) ray = load_ray(rays + size_t(r) * record_float4s);
-        found = trace_wide_warp<true>(nodes, tris, valid, ray, h, stack_mem + threadIdx.x, kQueryBlock, nullptr,
-                                      status);
-    } else {
-        if (!valid) return;
-        found = trace_wide<false>(nodes, tris, load_ray(rays + size_t(r) * record_float4s), h,
-                                  stack_mem + threadIdx.x, kQueryBlock, status);
-    }
-    if (status) atomicOr(err, status);
-    if (found) {
-        if (kAnyHit)
-            reinterpret_cast<float*>(rays + size_t(r) * record_float4s)[8] = -__int_as_float(0x7f800000);
-        else
-            store_hit(reinterpret_cast<SelRayHit*>(rays + size_t(r) * record_float4s), tris, h);
-    }
-}
-
 // Gate, keys, three radix passes and the ordered traversal on stream s, with stream-ordered scratch.
 template <bool kAnyHit>
 cudaError_t launch_query_ordered(const DeviceBvh& bvh, float4* d_rays, uint32_t record_float4s, uint32_t n,
@@ -264,10 +354,7 @@ cudaError_t launch_query_ordered(const DeviceBvh& bvh, float4* d_rays, uint32_t 
                                                ntiles);
         in ^= 1;
     }
-    const dim3 grid((n + kQueryBlock - 1) / kQueryBlock);
-    k_query_wide_ordered<kAnyHit><<<grid, kQueryBlock, 0, s>>>(static_cast<const uint4*>(bvh.nodes), bvh.tris,
-                                                                d_rays, record_float4s, n, vals[in], ctl, d_err);
-    e = cudaGetLastError();
+    e = launch_wide<kAnyHit>(bvh, d_rays, record_float4s, n, vals[in], ctl, d_err, s);
     const cudaError_t ef = cudaFreeAsync(mem, s);
     return e != cudaSuccess ? e : ef;
 }
@@ -297,17 +384,11 @@ template <bool kAnyHit>
 cudaError_t launch_query(const DeviceBvh& bvh, float4* d_rays, uint32_t record_float4s, uint32_t n, uint32_t* d_err,
                          cudaStream_t s) {
     if (n == 0) return cudaSuccess;
+    if (bvh.insts || bvh.kind == SEL_BVH_WIDE8_Q8)
+        return launch_wide<kAnyHit>(bvh, d_rays, record_float4s, n, nullptr, nullptr, d_err, s);
     const dim3 grid((n + kQueryBlock - 1) / kQueryBlock);
-    if (bvh.insts) {
-        k_query_instanced<kAnyHit><<<grid, kQueryBlock, 0, s>>>(static_cast<const uint4*>(bvh.nodes), bvh.tris,
-                                                                bvh.insts, d_rays, record_float4s, n, d_err);
-    } else if (bvh.kind == SEL_BVH_WIDE8_Q8) {
-        k_query_wide<kAnyHit><<<grid, kQueryBlock, 0, s>>>(static_cast<const uint4*>(bvh.nodes), bvh.tris, d_rays,
-                                                           record_float4s, n, d_err);
-    } else {
-        k_query_binary<kAnyHit><<<grid, kQueryBlock, 0, s>>>(static_cast<const float4*>(bvh.nodes), bvh.tris, d_rays,
-                                                             record_float4s, n, d_err);
-    }
+    k_query_binary<kAnyHit><<<grid, kQueryBlock, 0, s>>>(static_cast<const float4*>(bvh.nodes), bvh.tris, d_rays,
+                                                         record_float4s, n, d_err);
     return cudaGetLastError();
 }
 

@@ -13,6 +13,8 @@ struct DeviceBvh {
     const void* nodes = nullptr;   // WideNode[] or BinaryNode[]
     const float4* tris = nullptr;  // TriRecord[] as 3 x float4
     uint32_t tri_count = 0;
+    int stack_depth = kWideStack;  // traversal stack entries a ray may need (8-wide layout)
+    int sm_count = 1;
     const InstanceRecord* insts = nullptr;  // instance table of a scene with instances (8-wide layout only)
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // scene bounds (ray ordering keys)
     bool order_rays = false;  // SEL_OPTION_RAY_SORT: large incoherent batches in HBM are traced in key order

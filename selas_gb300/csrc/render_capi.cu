@@ -503,6 +503,7 @@ PtScene scene_view(const SelSceneTy* sc) {
     PtScene ps;
     ps.nodes = sc->d_nodes;
     ps.bvh_kind = sc->info.bvh_kind == SEL_BVH_WIDE8_Q8 ? 0 : 1;
+    ps.stack_depth = scene_stack_depth(sc);
     ps.tris = static_cast<const float4*>(sc->d_tris);
     ps.materials = static_cast<const MaterialDev*>(sc->d_materials);
     const uint32_t max_geom = geom_limit(sc);
@@ -651,7 +652,7 @@ int render_views_device(SelSceneTy* sc, const SelCamera* cams, uint32_t count, c
     e = pt_run_batches(ps.bvh_kind, settings.maxBounces, ps.sort_hint != 0, st, sc->dev->d_err, batches, stream,
                        sc->dev->graph_replay ? &sc->pt_graph : nullptr, block, mode == kPtModeDeferred ? 2u : 1u,
                        ps.insts != nullptr, pt_scene_textured(ps), ps.ray_sort != 0, batch_paths, ps.shader_kinds,
-                       ps.ptex_quads != 0);
+                       ps.ptex_quads != 0, int(ps.stack_depth), &ps);
     return e == cudaSuccess ? SEL_OK : cuda_fail(e, "multi-view render launch");
 }
 

@@ -287,9 +287,11 @@ bool pt_round(SelServerTy* S) {
     cudaMemcpyAsync(S->pst.jobs, table, sizeof(PtJob) * kMaxPtJobs, cudaMemcpyHostToDevice, S->pt_stream);
     cudaMemcpyAsync(S->pst.control, &c, sizeof(PtControl), cudaMemcpyHostToDevice, S->pt_stream);
     bool sort = false, instanced = false, texture = false, ray_sort = false, quad_ptex = false;
-    uint32_t modes = 0, shader_kinds = 0;
+    uint32_t modes = 0, shader_kinds = 0, stack_depth = 4;
     for (int k = 0; k < kMaxPtJobs; ++k)
         if (S->slots[k]) {
+            // in steps of four entries: fewer distinct launches to capture as jobs come and go
+            stack_depth = std::max(stack_depth, (S->slots[k]->scene.stack_depth + 3u) & ~3u);
             sort |= S->slots[k]->scene.sort_hint != 0;
             instanced |= S->slots[k]->scene.insts != nullptr;
             texture |= pt_scene_textured(S->slots[k]->scene);
@@ -302,7 +304,8 @@ bool pt_round(SelServerTy* S) {
     uint64_t batch_paths = 0;
     for (int k = 0; k < kMaxPtJobs; ++k) batch_paths += c.quota[k];
     cudaError_t e = pt_run_batches(0, bounces, sort, S->pst, S->dev->d_err, 1, S->pt_stream, &S->pt_graph, 128,
-                                   modes, instanced, texture, ray_sort, batch_paths, shader_kinds, quad_ptex);
+                                   modes, instanced, texture, ray_sort, batch_paths, shader_kinds, quad_ptex,
+                                   int(stack_depth));
     for (int k = 0; k < kMaxPtJobs; ++k) {
         Job* j = S->slots[k];
         if (!j || c.quota[k] == 0) continue;

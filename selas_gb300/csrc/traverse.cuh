@@ -106,15 +106,11 @@ __device__ __forceinline__ uint64_t tri_key(const float4& p0, const float4& p1) 
     return (uint64_t(__float_as_uint(p1.w)) << 32) | uint64_t(__float_as_uint(p0.w));
 }
 
-__device__ __forceinline__ float byte_as_float(uint32_t word, int byte) {
-    return __uint2float_rn((word >> (8 * byte)) & 0xffu);
-}
-
 // ---------------------------------------------------------------------------------------------------
 // 8-wide quantised BVH.  Node groups on the stack are (child_base, hit bits 24..31 | imask bits 0..7);
 // hit bit 24 + (slot ^ octant) so that the lowest set bit is the nearest child for this ray octant.
-// The traversal is written as a resumable per-ray state plus one step (one node visit and the triangles
-// it exposes), so that persistent kernels can refill finished lanes with new rays between steps.
+// A ray's traversal is a resumable per-lane state and one step (a node visit or one leaf record), so that
+// the lanes of a warp can be refilled with new rays between steps (trace_stream).
 // ---------------------------------------------------------------------------------------------------
 struct WideState {
     float ox, oy, oz, dx, dy, dz;
@@ -125,8 +121,17 @@ struct WideState {
     uint2 group;
     int sp;
     uint32_t iters;
-    uint64_t best_key;
-    QueryHit hit;
+    QueryHit hit;  // t is tfar
+};
+
+// A thread's traversal stack in shared memory: entry k at mem[k * stride], `depth` entries (the scene's tree
+// depth: a descent pushes at most one group a level).  Sizing it to the scene leaves the rest of the SM's 256 KB
+// to L1: with 12 entries instead of 24 a thread, 4 M incoherent rays over 5.2 M triangles take 1.81 ms, not 2.68
+// (closest hit), and 1.22, not 1.44 (any hit).
+struct WideStack {
+    uint2* mem;
+    int stride;
+    int depth;
 };
 
 // A ray that no triangle can hit under the watertight test: a non-finite origin or direction component
@@ -151,38 +156,75 @@ __device__ __forceinline__ void wide_init(WideState& s, const QueryRay& r) {
     s.group = make_uint2(0u, (1u << (24 + s.oct)) | 1u);
     s.sp = 0;
     s.iters = 0;
-    s.best_key = ~0ull;
     s.hit.tri = 0xffffffffu;
 }
 
-// q as float: 0x4B0000qq is 2^23 + q exactly, the subtraction is exact as well.
+// Three-input minimum / maximum (one instruction on sm_100 and later); NaN operands are ignored, as by fminf / fmaxf.
+__device__ __forceinline__ float max3_f32(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float min3_f32(float a, float b, float c) {
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// Packed FP32 pairs (sm_100 and later): two multiply-adds an instruction, each rounded once.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t r, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// 2^15 + q exactly: 0x4700qq00.
 __device__ __forceinline__ float qbyte(uint32_t word, uint32_t byte) {
-    return __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u | byte)) - 8388608.0f;
+    return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7404u | (byte << 4)));
 }
 
 // Visits the nearest pending node of s.group (which must have one): pushes the rest of the group, tests the
 // node's eight child boxes, makes its hit internal children the new group and returns the triangles of its
 // hit leaf children as a bit mask over records tbase..tbase+31.  Returns false on stack overflow.
-template <int kDepth>
-__device__ __forceinline__ bool wide_visit(WideState& s, const uint4* __restrict__ nodes, uint2* stack, int stride,
+//
+// A plane's distance is (2^15 + q) * (scale / d) + (origin - 2^15 * scale / d): one byte permute and one
+// multiply-add, the bias folded into the offset.  The fold costs 2^-9 of a quantum in the offset's rounding;
+// widening the offsets outward by 2^-22 of their magnitude covers that and the offset's own rounding, so no
+// distance of the ray's origin makes a box smaller.  Offsets that overflow turn into infinities and NaN that the
+// minima and maxima ignore: their axis then accepts every box.
+__device__ __forceinline__ bool wide_visit(WideState& s, const uint4* __restrict__ nodes, const WideStack& stack,
                                            uint32_t& status, uint32_t& tmask, uint32_t& tbase) {
     const int b = __ffs(s.group.y >> 24) - 1;
     s.group.y &= ~(1u << (24 + b));
     const uint32_t slot = uint32_t(b) ^ s.oct;
     const uint32_t idx = s.group.x + __popc(s.group.y & ((1u << slot) - 1u));
-    if (s.group.y & 0xff000000u) {
-        if (s.sp >= kDepth) { status |= kErrStackOverflow; return false; }
-        stack[s.sp * stride] = s.group;
-        ++s.sp;
-    }
     const uint4* np = nodes + size_t(idx) * 5;
     const uint4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3), n4 = __ldg(np + 4);
-    const float sxs = __fmul_rn(__uint_as_float((n0.w & 0xffu) << 23), s.ix);
-    const float sys = __fmul_rn(__uint_as_float(((n0.w >> 8) & 0xffu) << 23), s.iy);
-    const float szs = __fmul_rn(__uint_as_float(((n0.w >> 16) & 0xffu) << 23), s.iz);
-    const float oxa = __fmul_rn(__fsub_rn(__uint_as_float(n0.x), s.ox), s.ix);
-    const float oya = __fmul_rn(__fsub_rn(__uint_as_float(n0.y), s.oy), s.iy);
-    const float oza = __fmul_rn(__fsub_rn(__uint_as_float(n0.z), s.oz), s.iz);
+    if (s.group.y & 0xff000000u) {
+        if (s.sp >= stack.depth) { status |= kErrStackOverflow; return false; }
+        stack.mem[s.sp * stack.stride] = s.group;
+        ++s.sp;
+    }
+    const float sx = __fmul_rn(__uint_as_float((n0.w << 23) & 0x7f800000u), s.ix);
+    const float sy = __fmul_rn(__uint_as_float((n0.w << 15) & 0x7f800000u), s.iy);
+    const float sz = __fmul_rn(__uint_as_float((n0.w << 7) & 0x7f800000u), s.iz);
+    const float ax = fmaf(-32768.0f, sx, __fmul_rn(__fsub_rn(__uint_as_float(n0.x), s.ox), s.ix));
+    const float ay = fmaf(-32768.0f, sy, __fmul_rn(__fsub_rn(__uint_as_float(n0.y), s.oy), s.iy));
+    const float az = fmaf(-32768.0f, sz, __fmul_rn(__fsub_rn(__uint_as_float(n0.z), s.oz), s.iz));
+    constexpr float kOut = 1.0f / 4194304.0f;
+    // (near, far) pairs
+    const uint64_t sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
+    const uint64_t ax2 = pack2(fmaf(-kOut, fabsf(ax), ax), fmaf(kOut, fabsf(ax), ax));
+    const uint64_t ay2 = pack2(fmaf(-kOut, fabsf(ay), ay), fmaf(kOut, fabsf(ay), ay));
+    const uint64_t az2 = pack2(fmaf(-kOut, fabsf(az), az), fmaf(kOut, fabsf(az), az));
     const uint32_t imask = n0.w >> 24;
     const float tnear_box = s.tnear - fabsf(s.tnear) * kBoxMargin;
     const float tfar_box = s.tfar + fabsf(s.tfar) * kBoxMargin;
@@ -190,211 +232,188 @@ __device__ __forceinline__ bool wide_visit(WideState& s, const uint4* __restrict
     const uint32_t nx0 = px ? n2.x : n3.z, nx1 = px ? n2.y : n3.w, fx0 = px ? n3.z : n2.x, fx1 = px ? n3.w : n2.y;
     const uint32_t ny0 = py ? n2.z : n4.x, ny1 = py ? n2.w : n4.y, fy0 = py ? n4.x : n2.z, fy1 = py ? n4.y : n2.w;
     const uint32_t nz0 = pz ? n3.x : n4.z, nz1 = pz ? n3.y : n4.w, fz0 = pz ? n4.z : n3.x, fz1 = pz ? n4.w : n3.y;
-    uint32_t new_hits = 0;
+    uint32_t miss = 0;  // bit c: child c's interval is empty, the sign of its length
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
+    for (int c = 7; c >= 0; --c) {
         const uint32_t byte = uint32_t(c & 3);
-        const float tnx = fmaf(qbyte(c < 4 ? nx0 : nx1, byte), sxs, oxa);
-        const float tfx = fmaf(qbyte(c < 4 ? fx0 : fx1, byte), sxs, oxa);
-        const float tny = fmaf(qbyte(c < 4 ? ny0 : ny1, byte), sys, oya);
-        const float tfy = fmaf(qbyte(c < 4 ? fy0 : fy1, byte), sys, oya);
-        const float tnz = fmaf(qbyte(c < 4 ? nz0 : nz1, byte), szs, oza);
-        const float tfz = fmaf(qbyte(c < 4 ? fz0 : fz1, byte), szs, oza);
-        const float tmin = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, tnear_box));
-        const float tmax = fminf(fminf(tfx, tfy), fminf(tfz, tfar_box));
-        if (tmin <= tmax) {
-            if ((imask >> c) & 1u) {
-                new_hits |= 1u << (uint32_t(c) ^ s.oct);
-            } else {
-                const uint32_t meta = ((c < 4 ? n1.z : n1.w) >> (8 * byte)) & 0xffu;
-                if (meta != kLeafNone) tmask |= (0xffu >> (7u - (meta >> 5))) << (meta & 31u);
-            }
-        }
+        float tnx, tny, tnz, tfx, tfy, tfz;
+        unpack2(fma2(pack2(qbyte(c < 4 ? nx0 : nx1, byte), qbyte(c < 4 ? fx0 : fx1, byte)), sx2, ax2), tnx, tfx);
+        unpack2(fma2(pack2(qbyte(c < 4 ? ny0 : ny1, byte), qbyte(c < 4 ? fy0 : fy1, byte)), sy2, ay2), tny, tfy);
+        unpack2(fma2(pack2(qbyte(c < 4 ? nz0 : nz1, byte), qbyte(c < 4 ? fz0 : fz1, byte)), sz2, az2), tnz, tfz);
+        const float tmin = fmaxf(max3_f32(tnx, tny, tnz), tnear_box);
+        const float tmax = fminf(min3_f32(tfx, tfy, tfz), tfar_box);
+        miss = __funnelshift_l(__float_as_uint(__fsub_rn(tmax, tmin)), miss, 1);
     }
-    s.group = make_uint2(n1.x, (new_hits << 24) | imask);
+    const uint32_t hits = ~miss & 0xffu;
+    uint32_t in = hits & imask, t;  // the internal hits, bit c moved to bit c ^ octant
+    t = ((in >> 1) ^ in) & ((s.oct & 1u) ? 0x55u : 0u);
+    in ^= t ^ (t << 1);
+    t = ((in >> 2) ^ in) & ((s.oct & 2u) ? 0x33u : 0u);
+    in ^= t ^ (t << 2);
+    t = ((in >> 4) ^ in) & ((s.oct & 4u) ? 0x0fu : 0u);
+    in ^= t ^ (t << 4);
+    for (uint32_t leaf = hits & ~imask; leaf; leaf &= leaf - 1u) {
+        const uint32_t meta = __byte_perm(n1.z, n1.w, __ffs(leaf) - 1) & 0xffu;
+        if (meta != kLeafNone) tmask |= ((2u << (meta >> 5)) - 1u) << (meta & 31u);
+    }
+    s.group = make_uint2(n1.x, (in << 24) | imask);
     tbase = n1.y;
     return true;
 }
 
-// One traversal step.  Returns true when the ray is finished (any-hit: on the first hit).
-template <bool kAnyHit>
-__device__ __forceinline__ bool wide_step(WideState& s, const uint4* __restrict__ nodes, const float4* __restrict__ tris,
-                                          uint2* stack, int stride, uint32_t& status) {
-    uint32_t tmask = 0, tbase = 0;
-    if (s.group.y & 0xff000000u) {
-        if (!wide_visit<kWideStack>(s, nodes, stack, stride, status, tmask, tbase)) return true;
-    }
-    while (tmask) {
-        const int b = __ffs(tmask) - 1;
-        tmask &= tmask - 1u;
-        const uint32_t ti = tbase + uint32_t(b);
-        const float4* tp = tris + size_t(ti) * 3;
-        const float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
-        float t, u, v;
-        if (watertight_intersect(s.wt, s.ox, s.oy, s.oz, p0, p1, p2, s.tnear, s.tfar, t, u, v)) {
-            if (kAnyHit) {
-                s.hit.t = t; s.hit.u = u; s.hit.v = v; s.hit.tri = ti;
-                return true;
-            }
-            const uint64_t key = tri_key(p0, p1);
-            if (t < s.tfar || key < s.best_key) {
-                s.tfar = t;
-                s.best_key = key;
-                s.hit.t = t; s.hit.u = u; s.hit.v = v; s.hit.tri = ti;
-            }
-        }
-    }
-    if (++s.iters > kIterationCap) { status |= kErrIterationCap; return true; }
-    if (!(s.group.y & 0xff000000u)) {
-        if (s.sp == 0) return true;
-        --s.sp;
-        s.group = stack[s.sp * stride];
-    }
-    return false;
-}
-
-// Whole-ray form (one thread, one ray).
-template <bool kAnyHit>
-__device__ __forceinline__ bool trace_wide(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
-                                           const QueryRay& r, QueryHit& hit, uint2* stack, int stride,
-                                           uint32_t& status) {
-    if (ray_untraceable(r)) {
-        hit.tri = 0xffffffffu;
-        return false;
-    }
-    WideState s;
-    wide_init(s, r);
-    while (!wide_step<kAnyHit>(s, nodes, tris, stack, stride, status)) {}
-    hit = s.hit;
-    return s.hit.tri != 0xffffffffu;
-}
-
-// Warp-cooperative form (one ray per lane, all 32 lanes of the warp together, finished and idle lanes included):
-// each step every lane with a pending node visits it, then the warp tests the leaf triangles those visits exposed
-// together, 32 (ray, triangle) pairs a round, each lane testing one pair with its owner's ray taken by shuffles.
-// Incoherent rays leave most lanes of the one-lane form idle during leaf tests (9 of 32 active per instruction);
-// here the tests run on full warps.  The owner takes its candidates in the one-lane form's order (ascending
-// record index within a step) under the same rule (t < tfar, or t == tfar and a smaller (geomID, primID)), and a
-// candidate's t, u, v do not depend on the tfar it was tested against, so the hits are the same bits.
-// slots: this warp's 32 result slots in shared memory (closest hit only; any hit needs none).  The query kernels
-// use this form for any hit only: for closest hit it measured no faster than the one-lane form.
-struct CoopSlot {
+// Tests leaf record ti and keeps it when it is the ray's new closest hit: t < tfar, or t == tfar and a smaller
+// (geomID, primID) than the hit so far (whose record is read again then: ties are rare).  Returns whether the
+// record is hit.
+__device__ __forceinline__ bool wide_test(WideState& s, const float4* __restrict__ tris, uint32_t ti) {
+    const float4* tp = tris + size_t(ti) * 3;
+    const float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
     float t, u, v;
-    uint32_t ti;
+    if (!watertight_intersect(s.wt, s.ox, s.oy, s.oz, p0, p1, p2, s.tnear, s.tfar, t, u, v)) return false;
+    bool take = t < s.tfar || s.hit.tri == 0xffffffffu;
+    if (!take) {
+        const float4* bp = tris + size_t(s.hit.tri) * 3;
+        take = tri_key(p0, p1) < tri_key(__ldg(bp), __ldg(bp + 1));
+    }
+    if (take) {
+        s.tfar = t;
+        s.hit.u = u;
+        s.hit.v = v;
+        s.hit.tri = ti;
+    }
+    return true;
+}
+
+// The flat traversal of one lane, as trace_stream steps it.
+struct WideWalk {
+    WideState s;
+    uint32_t tmask, tbase;  // leaf records still to test: bit k is record tbase + k
+
+    template <typename Rays>
+    __device__ __forceinline__ bool start(const QueryRay& r, const Rays&) {
+        wide_init(s, r);
+        tmask = 0;
+        return !ray_untraceable(r);
+    }
+
+    __device__ __forceinline__ bool pending() const { return tmask != 0u; }
+
+    // Visits the nearest pending node (there is one when no leaf record is pending).  False: the ray is given up.
+    template <typename Rays>
+    __device__ __forceinline__ bool visit(const Rays& rays, const WideStack& stack, uint32_t& status) {
+        return wide_visit(s, rays.nodes(), stack, status, tmask, tbase);
+    }
+
+    // Tests one pending leaf record.  False: the ray is finished (any-hit: on the first hit).
+    template <bool kAnyHit, typename Rays>
+    __device__ __forceinline__ bool test(const Rays& rays, const WideStack&, uint32_t&) {
+        const uint32_t ti = tbase + uint32_t(__ffs(tmask) - 1);
+        tmask &= tmask - 1u;
+        return !(wide_test(s, rays.tris(), ti) && kAnyHit);
+    }
+
+    // Ends a step: with nothing pending, goes back to the nearest node group.  False: the ray is finished.
+    __device__ __forceinline__ bool advance(const WideStack& stack, uint32_t& status) {
+        if (++s.iters > kIterationCap) {
+            status |= kErrIterationCap;
+            return false;
+        }
+        if (!tmask && !(s.group.y & 0xff000000u)) {
+            if (s.sp == 0) return false;
+            --s.sp;
+            s.group = stack.mem[s.sp * stack.stride];
+        }
+        return true;
+    }
 };
 
-template <bool kAnyHit>
-__device__ __forceinline__ bool trace_wide_warp(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
-                                                bool valid, const QueryRay& r, QueryHit& hit, uint2* stack,
-                                                int stride, CoopSlot* slots, uint32_t& status) {
-    const uint32_t lane = threadIdx.x & 31u;
-    WideState s;
-    wide_init(s, r);
-    bool done = !valid || ray_untraceable(r);
-    while (__any_sync(0xffffffffu, !done)) {
-        uint32_t tmask = 0, tbase = 0;
-        if (!done && (s.group.y & 0xff000000u)) {
-            if (!wide_visit<kWideStack>(s, nodes, stack, stride, status, tmask, tbase)) {
-                done = true;
-                tmask = 0;
+// Traces a stream of rays with one warp.  The lanes step together; whenever kRefillLanes of them have finished
+// (or all have), these write their results and take the next rays, so the warp neither waits for its longest ray
+// nor pays a ray's set-up with few lanes.  A step visits a node in the lanes without pending leaf records, then tests
+// one record in the lanes with some (and further ones while at least kTestLanes lanes test): testing all that a visit
+// exposed at once would hold the other lanes up.  32 incoherent rays over 5.2 M triangles take 19 visits of 23 lanes
+// and 19 record tests of 9 lanes, against 32 visits of 14 lanes and 53 tests of 3 with a packet of 32 rays and all
+// records a visit.  The ballots between the phases matter beyond their masks: they bring the lanes back together,
+// without them the record tests run twice (2.34 against 1.95 ms, 4 M of those rays, closest hit; 2.41 for the packet
+// form).  Kernels of the wavefront (room at 1280 x 720, a bounce): closest hit 1.07 against 1.58 ms, any hit 0.52
+// against 0.61.  kRefillLanes 2, 4, 6, 8, 12: 1.90, 1.82, 1.80, 1.81, 1.88 ms; a threshold following the rays' length
+// lost everywhere.  kTestLanes 4, 8, 16: closest hit 2.39, 2.20, 2.13 ms, the Cornell box's path tracer (few
+// nodes, many records) 24.06, 24.06, 24.31 ms.
+// A Rays object gives the warp its rays:
+//   bool next(b, e)        the next range of ray indices, warp-uniform, called by the whole warp; false: no more
+//   bool begin(i, ray)     a lane's ray i; false: nothing to trace or to write for it
+//   void end(i, state)     its result: state.hit (tri 0xffffffff: no hit, else at distance s.tfar)
+//   nodes(), tris(), insts()  the lane's scene
+constexpr int kRefillLanes = 8;
+constexpr int kTestLanes = 16;
+
+template <bool kAnyHit, typename Walk, typename Rays>
+__device__ __forceinline__ void trace_stream(Rays& rays, const WideStack& stack, uint32_t& status) {
+    const uint32_t below = (1u << (threadIdx.x & 31u)) - 1u;
+    uint32_t next = 0, end = 0, id = 0;
+    bool busy = false, have = false, more = true;
+    Walk w;
+    for (;;) {
+        const uint32_t idle = __ballot_sync(0xffffffffu, !busy);
+        if (idle == 0xffffffffu || (more && __popc(idle) >= kRefillLanes)) {
+            if (!busy && have) {
+                rays.end(id, w.s);
+                have = false;
             }
-        }
-        // pairs: lane L owns pairs [excl, incl) of the warp's concatenation, its set tmask bits in ascending order
-        const uint32_t cnt = __popc(tmask);
-        uint32_t incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= uint32_t(o)) incl += y;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        const uint32_t excl = incl - cnt;
-        const uint32_t kpack = uint32_t(s.wt.kx) | (uint32_t(s.wt.ky) << 2) | (uint32_t(s.wt.kz) << 4);
-        for (uint32_t r0 = 0; r0 < total; r0 += 32) {
-            const uint32_t j = r0 + lane;
-            uint32_t owner = 0;  // the first lane whose inclusive end exceeds j
-#pragma unroll
-            for (uint32_t step = 16; step >= 1; step >>= 1) {
-                const uint32_t e = __shfl_sync(0xffffffffu, incl, owner + step - 1);
-                if (e <= j) owner += step;
-            }
-            const uint32_t o_mask = __shfl_sync(0xffffffffu, tmask, owner);
-            const uint32_t o_base = __shfl_sync(0xffffffffu, tbase, owner);
-            const uint32_t o_excl = __shfl_sync(0xffffffffu, excl, owner);
-            const uint32_t kp = __shfl_sync(0xffffffffu, kpack, owner);
-            Watertight w;
-            w.kx = int(kp & 3u);
-            w.ky = int((kp >> 2) & 3u);
-            w.kz = int((kp >> 4) & 3u);
-            w.sx = __shfl_sync(0xffffffffu, s.wt.sx, owner);
-            w.sy = __shfl_sync(0xffffffffu, s.wt.sy, owner);
-            w.sz = __shfl_sync(0xffffffffu, s.wt.sz, owner);
-            const float rox = __shfl_sync(0xffffffffu, s.ox, owner);
-            const float roy = __shfl_sync(0xffffffffu, s.oy, owner);
-            const float roz = __shfl_sync(0xffffffffu, s.oz, owner);
-            const float rtn = __shfl_sync(0xffffffffu, s.tnear, owner);
-            const float rtf = __shfl_sync(0xffffffffu, s.tfar, owner);
-            bool got = false;
-            float t = 0.0f, u = 0.0f, v = 0.0f;
-            uint32_t ti = 0xffffffffu;
-            const uint32_t bit = j < total ? __fns(o_mask, 0u, int(j - o_excl) + 1) : 0xffffffffu;
-            if (bit < 32u) {
-                ti = o_base + bit;
-                const float4* tp = tris + size_t(ti) * 3;
-                const float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
-                got = watertight_intersect(w, rox, roy, roz, p0, p1, p2, rtn, rtf, t, u, v);
-            }
-            // this lane's own pairs in the round: [a, b) of the concatenation
-            const uint32_t a = excl > r0 ? excl : r0;
-            const uint32_t b = incl < r0 + 32 ? incl : r0 + 32;
-            if constexpr (kAnyHit) {
-                const uint32_t hits = __ballot_sync(0xffffffffu, got);
-                if (!done && a < b) {
-                    const uint32_t span = b - a;
-                    const uint32_t mine = (hits >> (a - r0)) & (span >= 32 ? 0xffffffffu : ((1u << span) - 1u));
-                    if (mine) {
-                        s.hit.tri = 0u;  // occluded: only the fact of a hit is reported
-                        done = true;
-                    }
+            if (more && next >= end) more = rays.next(next, end);
+            if (more) {
+                const uint32_t mine = next + __popc(idle & below);
+                next += __popc(idle);
+                QueryRay r;
+                if (!busy && mine < end && rays.begin(mine, r)) {
+                    id = mine;
+                    have = true;
+                    busy = w.start(r, rays);
                 }
-            } else {
-                slots[lane] = CoopSlot{t, u, v, got ? ti : 0xffffffffu};
-                __syncwarp();
-                for (uint32_t q = a; q < b; ++q) {
-                    const CoopSlot c = slots[q - r0];
-                    if (c.ti == 0xffffffffu || c.t > s.tfar) continue;
-                    const float4* cp = tris + size_t(c.ti) * 3;
-                    const uint64_t key = (uint64_t(__float_as_uint(__ldg(&cp[1].w))) << 32) |
-                                         uint64_t(__float_as_uint(__ldg(&cp[0].w)));
-                    if (c.t < s.tfar || key < s.best_key) {
-                        s.tfar = c.t;
-                        s.best_key = key;
-                        s.hit.t = c.t;
-                        s.hit.u = c.u;
-                        s.hit.v = c.v;
-                        s.hit.tri = c.ti;
-                    }
-                }
-                __syncwarp();
+            } else if (idle == 0xffffffffu) {
+                break;
             }
         }
-        if (!done) {
-            if (++s.iters > kIterationCap) {
-                status |= kErrIterationCap;
-                done = true;
-            } else if (!(s.group.y & 0xff000000u)) {
-                if (s.sp == 0) {
-                    done = true;
-                } else {
-                    --s.sp;
-                    s.group = stack[s.sp * stride];
-                }
-            }
+        if (busy && !w.pending()) busy = w.visit(rays, stack, status);
+        uint32_t testing = __ballot_sync(0xffffffffu, busy && w.pending());
+        while (testing) {
+            if (busy && w.pending()) busy = w.template test<kAnyHit>(rays, stack, status);
+            if (__popc(testing) < kTestLanes) break;
+            testing = __ballot_sync(0xffffffffu, busy && w.pending());
         }
+        if (busy) busy = w.advance(stack, status);
     }
-    hit = s.hit;
-    return valid && s.hit.tri != 0xffffffffu;
 }
+
+// Ray ranges of a queue of n entries for the persistent kernels: every warp's first range is its own, then warps
+// take further ones through an atomic cursor (which starts at 0).  Short queues are spread over all warps, so
+// that few lanes of many warps trace them rather than all lanes of a few, and need no atomics.
+struct QueueRanges {
+    uint32_t n, chunk, first, rest;
+    uint32_t* cursor;
+    bool started;
+
+    __device__ __forceinline__ QueueRanges(uint32_t count, uint32_t* cur) : n(count), cursor(cur), started(false) {
+        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+        const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        chunk = (n + warps - 1) / warps;
+        chunk = chunk < 32u ? (chunk ? chunk : 1u) : 32u;
+        first = warp * chunk;
+        rest = warps * chunk;
+    }
+    __device__ __forceinline__ bool next(uint32_t& b, uint32_t& e) {
+        if (!started) {
+            started = true;
+            b = first;
+        } else {
+            if (rest >= n) return false;
+            b = 0;
+            if ((threadIdx.x & 31u) == 0) b = rest + atomicAdd(cursor, chunk);
+            b = __shfl_sync(0xffffffffu, b, 0);
+        }
+        e = b + chunk < n ? b + chunk : n;
+        return b < n;
+    }
+};
 
 // ---------------------------------------------------------------------------------------------------
 // Binary FP32 BVH (the plain GPU path): classic stack traversal, nearer child first.
@@ -487,23 +506,11 @@ __device__ __forceinline__ bool trace_binary(const float4* __restrict__ nodes, c
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Traversal policies for the render kernels, which are instantiated for both BVH layouts: the 8-wide
-// quantised one and the plain binary FP32 one (the comparison path).  Stack entries live in shared memory,
-// `stride` entries apart per thread.
+// Traversal policy of the plain binary FP32 layout (the comparison path) for the render kernels.  Stack entries
+// live in shared memory, `stride` entries apart per thread.
 // ---------------------------------------------------------------------------------------------------
 template <int kKind>
 struct Tracer;
-
-template <>
-struct Tracer<0> {  // SEL_BVH_WIDE8_Q8
-    using Entry = uint2;
-    static constexpr int kDepth = kWideStack;
-    template <bool kAnyHit>
-    static __device__ __forceinline__ bool trace(const void* nodes, const float4* tris, const QueryRay& r, QueryHit& h,
-                                                 Entry* stack, int stride, uint32_t& status) {
-        return trace_wide<kAnyHit>(static_cast<const uint4*>(nodes), tris, r, h, stack, stride, status);
-    }
-};
 
 template <>
 struct Tracer<1> {  // SEL_BVH_BINARY_FP32

@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "capi_internal.h"
 #include "graph.h"
@@ -459,96 +460,130 @@ __global__ void __launch_bounds__(kBlock) k_c_generate(VcmParams P) {
     if (blockIdx.x == 0 && threadIdx.x == 0) P.st.counters[0] = N;
 }
 
-// Closest hits of the queued paths: persistent blocks, warps take 32-entry packets through an atomic cursor.
+// Closest hits of the queued paths: persistent blocks of B threads; the 8-wide layouts trace the queue as a stream
+// (trace_stream), K = 0 flat, 2 with instances; the binary comparison layout (K = 1) takes packets of 32 entries.
+struct PathRays : QueueRanges {
+    const VcmParams& P;
+    const uint32_t* queue;
+    __device__ __forceinline__ PathRays(const VcmParams& p, const uint32_t* q, uint32_t n)
+        : QueueRanges(n, &p.st.counters[3]), P(p), queue(q) {}
+    __device__ __forceinline__ const uint4* nodes() const { return static_cast<const uint4*>(P.nodes); }
+    __device__ __forceinline__ const float4* tris() const { return P.tris; }
+    __device__ __forceinline__ const InstanceRecord* insts() const { return P.insts; }
+    __device__ __forceinline__ bool begin(uint32_t e, QueryRay& q) const {
+        const uint32_t s = queue[e];
+        const float4 o = P.st.po[s], d = P.st.pd[s];
+        q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = 0.0f;
+        q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = kFloatMax;
+        return true;
+    }
+    __device__ __forceinline__ void store(uint32_t s, float t, const float uv[2], uint32_t tri) const {
+        const bool found = tri != 0xffffffffu;
+        P.st.phit[s] = make_float4(found ? t : 0.0f, found ? uv[0] : 0.0f, found ? uv[1] : 0.0f, __uint_as_float(tri));
+    }
+    __device__ __forceinline__ void end(uint32_t e, const WideState& h) const {
+        const float uv[2] = {h.hit.u, h.hit.v};
+        store(queue[e], h.tfar, uv, h.hit.tri);
+    }
+    __device__ __forceinline__ void end(uint32_t e, const InstState& h) const {
+        const uint32_t s = queue[e];
+        const float uv[2] = {h.hit.u, h.hit.v};
+        store(s, h.w.tfar, uv, h.hit.tri);
+        P.st.phinst[s] = h.hit.tri != 0xffffffffu ? inst_indices(P.insts, h.hit) : make_uint2(0u, 0u);
+    }
+};
+
+extern __shared__ uint2 vcm_stack[];
+
 template <int K, int B>
-__global__ void __launch_bounds__(B, 1024 / B) k_extend(VcmParams P, int cur) {
-    __shared__ typename Tracer<K>::Entry stack_mem[Tracer<K>::kDepth * B];
+constexpr int kTraceBlocksPerSm = (K == 2 ? 512 : 1024) / B;
+
+template <int K, int B>
+__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_extend(const __grid_constant__ VcmParams P, int cur,
+                                                                       int stack_depth) {
     const uint32_t n = P.st.counters[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays, (unsigned long long)n);
     const uint32_t* queue = P.st.queue[cur];
     uint32_t status = 0;
-    for (;;) {
-        uint32_t base = 0;
-        if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[3], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const uint32_t e = base + (threadIdx.x & 31u);
-        if (e < n) {
-            const uint32_t s = queue[e];
-            const float4 o = P.st.po[s], d = P.st.pd[s];
-            QueryRay q;
-            q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = 0.0f;
-            q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = kFloatMax;
-            if constexpr (K == 2) {
-                InstHit h;
-                const bool found = trace_instanced<false>(static_cast<const uint4*>(P.nodes), P.tris, P.insts, q, h,
-                                                          stack_mem + threadIdx.x, B, status);
-                P.st.phit[s] = found ? make_float4(h.t, h.u, h.v, __uint_as_float(h.tri))
-                                     : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(0xffffffffu));
-                P.st.phinst[s] = found ? inst_indices(P.insts, h) : make_uint2(0u, 0u);
-            } else {
+    PathRays rays(P, queue, n);
+    if constexpr (K == 1) {
+        __shared__ int stack_mem[kBinaryStack * B];
+        for (;;) {
+            uint32_t base = 0;
+            if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[3], 32u);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= n) break;
+            const uint32_t e = base + (threadIdx.x & 31u);
+            if (e < n) {
+                QueryRay q;
+                rays.begin(e, q);
                 QueryHit h;
-                const bool found = Tracer<K>::template trace<false>(P.nodes, P.tris, q, h, stack_mem + threadIdx.x, B,
-                                                                    status);
-                P.st.phit[s] = found ? make_float4(h.t, h.u, h.v, __uint_as_float(h.tri))
-                                     : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(0xffffffffu));
+                trace_binary<false>(static_cast<const float4*>(P.nodes), P.tris, q, h, stack_mem + threadIdx.x, B,
+                                    status);
+                const float uv[2] = {h.u, h.v};
+                rays.store(queue[e], h.t, uv, h.tri);
             }
         }
+    } else {
+        using Walk = std::conditional_t<K == 2, InstWalk, WideWalk>;
+        trace_stream<false, Walk>(rays, WideStack{vcm_stack + threadIdx.x, B, stack_depth}, status);
     }
     if (status) atomicOr(P.err, status);
 }
 
 // Any-hit of the queued shadow rays; unoccluded ones add their contribution to their pixel.
+struct ShadowRays : QueueRanges {
+    const VcmParams& P;
+    __device__ __forceinline__ ShadowRays(const VcmParams& p, uint32_t n) : QueueRanges(n, &p.st.counters[4]), P(p) {}
+    __device__ __forceinline__ const uint4* nodes() const { return static_cast<const uint4*>(P.nodes); }
+    __device__ __forceinline__ const float4* tris() const { return P.tris; }
+    __device__ __forceinline__ const InstanceRecord* insts() const { return P.insts; }
+    __device__ __forceinline__ bool begin(uint32_t e, QueryRay& q) const {
+        const float4 c = P.st.sc[e];
+        if (c.x == 0.0f && c.y == 0.0f && c.z == 0.0f) return false;  // a null entry
+        const float4 o = P.st.so[e], d = P.st.sd[e];
+        q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = o.w;
+        q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = d.w;
+        return true;
+    }
+    __device__ __forceinline__ void add(uint32_t e) const {
+        const float4 c = P.st.sc[e];
+        splat(P.accum, __float_as_uint(c.w), f3(c.x, c.y, c.z));
+    }
+    __device__ __forceinline__ void end(uint32_t e, const WideState& h) const {
+        if (h.hit.tri == 0xffffffffu) add(e);
+    }
+    __device__ __forceinline__ void end(uint32_t e, const InstState& h) const {
+        if (h.hit.tri == 0xffffffffu) add(e);
+    }
+};
+
 template <int K, int B>
-__global__ void __launch_bounds__(B, 1024 / B) k_shadow(VcmParams P) {
-    __shared__ typename Tracer<K>::Entry stack_mem[Tracer<K>::kDepth * B];
+__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_shadow(const __grid_constant__ VcmParams P,
+                                                                       int stack_depth) {
     const uint32_t n = P.st.counters[2];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays + 1, (unsigned long long)n);
     uint32_t status = 0;
-    for (;;) {
-        uint32_t base = 0;
-        if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[4], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= n) break;
-        const uint32_t e = base + (threadIdx.x & 31u);
-        // 8-wide layout: the packet's lanes test their leaf triangles together (trace_wide_warp): passes 1.2 % faster
-        // on the room at 1280 x 720 (20.54 against 20.79 ms).  The path tracer's shadow kernel, whose packets can mix
-        // jobs' scenes, measured 3 % slower this way on the Cornell box and keeps one lane per ray.
-        if constexpr (K == 0) {
-            float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (e < n) c = P.st.sc[e];
-            const bool live = c.x != 0.0f || c.y != 0.0f || c.z != 0.0f;
-            QueryRay q{};
-            if (live) {
-                const float4 o = P.st.so[e], d = P.st.sd[e];
-                q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = o.w;
-                q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = d.w;
-            }
-            QueryHit h;
-            const bool hit = trace_wide_warp<true>(static_cast<const uint4*>(P.nodes), P.tris, live, q, h,
-                                                   stack_mem + threadIdx.x, B, nullptr, status);
-            if (live && !hit) splat(P.accum, __float_as_uint(c.w), f3(c.x, c.y, c.z));
-            continue;
-        }
-        if (e < n) {
-            const float4 c = P.st.sc[e];
-            if (c.x != 0.0f || c.y != 0.0f || c.z != 0.0f) {
-                const float4 o = P.st.so[e], d = P.st.sd[e];
-                QueryRay q;
-                q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = o.w;
-                q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = d.w;
-                bool hit;
-                if constexpr (K == 2) {
-                    InstHit h;
-                    hit = trace_instanced<true>(static_cast<const uint4*>(P.nodes), P.tris, P.insts, q, h,
-                                                stack_mem + threadIdx.x, B, status);
-                } else {
-                    QueryHit h;
-                    hit = Tracer<K>::template trace<true>(P.nodes, P.tris, q, h, stack_mem + threadIdx.x, B, status);
-                }
-                if (!hit) splat(P.accum, __float_as_uint(c.w), f3(c.x, c.y, c.z));
+    ShadowRays rays(P, n);
+    if constexpr (K == 1) {
+        __shared__ int stack_mem[kBinaryStack * B];
+        for (;;) {
+            uint32_t base = 0;
+            if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[4], 32u);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= n) break;
+            const uint32_t e = base + (threadIdx.x & 31u);
+            QueryRay q;
+            if (e < n && rays.begin(e, q)) {
+                QueryHit h;
+                if (!trace_binary<true>(static_cast<const float4*>(P.nodes), P.tris, q, h, stack_mem + threadIdx.x, B,
+                                        status))
+                    rays.add(e);
             }
         }
+    } else {
+        using Walk = std::conditional_t<K == 2, InstWalk, WideWalk>;
+        trace_stream<true, Walk>(rays, WideStack{vcm_stack + threadIdx.x, B, stack_depth}, status);
     }
     if (status) atomicOr(P.err, status);
 }
@@ -1352,21 +1387,23 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kBlock, 0);
         return sms * std::max(blocks, 1);
     };
-    // scenes with instances: the instanced traversal (128-thread blocks, 4 per SM: its 40-entry stacks) and the
-    // shading kernels that read a hit's scene through its instances
+    // scenes with instances: the instanced traversal (128-thread blocks, 4 per SM: its registers) and the shading
+    // kernels that read a hit's scene through its instances
     const bool inst = sc.insts != nullptr;
     const int inst_grid = sms * 4;
+    const int depth = int(sc.stack_depth);
+    const size_t stack_128 = size_t(depth) * 128 * sizeof(uint2), stack_256 = 2 * stack_128;
     auto extend = [&](cudaStream_t stream, int cur) {
-        if (inst) k_extend<2, 128><<<inst_grid, 128, 0, stream>>>(P, cur);
-        else if (sc.bvh_kind != 0) k_extend<1, 128><<<trace_grid, 128, 0, stream>>>(P, cur);
-        else if (tb == 256) k_extend<0, 256><<<trace_grid, 256, 0, stream>>>(P, cur);
-        else k_extend<0, 128><<<trace_grid, 128, 0, stream>>>(P, cur);
+        if (inst) k_extend<2, 128><<<inst_grid, 128, stack_128, stream>>>(P, cur, depth);
+        else if (sc.bvh_kind != 0) k_extend<1, 128><<<trace_grid, 128, 0, stream>>>(P, cur, depth);
+        else if (tb == 256) k_extend<0, 256><<<trace_grid, 256, stack_256, stream>>>(P, cur, depth);
+        else k_extend<0, 128><<<trace_grid, 128, stack_128, stream>>>(P, cur, depth);
     };
     auto shadow = [&](cudaStream_t stream) {
-        if (inst) k_shadow<2, 128><<<inst_grid, 128, 0, stream>>>(P);
-        else if (sc.bvh_kind != 0) k_shadow<1, 128><<<trace_grid, 128, 0, stream>>>(P);
-        else if (tb == 256) k_shadow<0, 256><<<trace_grid, 256, 0, stream>>>(P);
-        else k_shadow<0, 128><<<trace_grid, 128, 0, stream>>>(P);
+        if (inst) k_shadow<2, 128><<<inst_grid, 128, stack_128, stream>>>(P, depth);
+        else if (sc.bvh_kind != 0) k_shadow<1, 128><<<trace_grid, 128, 0, stream>>>(P, depth);
+        else if (tb == 256) k_shadow<0, 256><<<trace_grid, 256, stack_256, stream>>>(P, depth);
+        else k_shadow<0, 128><<<trace_grid, 128, stack_128, stream>>>(P, depth);
     };
     // Textures are filtered by the texture pass (k_vtexture) over the sorted queue when the hits are sorted; the
     // plain form (SEL_OPTION_MATERIAL_SORT 0) filters triangle Ptex inline in queue order, and quad-mesh Ptex, which
@@ -1452,7 +1489,7 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
     };
     struct Key {
         VcmParams P;
-        int kind, sms, radix_passes, sort, tb, quads;
+        int kind, sms, radix_passes, sort, tb, quads, depth;
     } key;
     std::memset(&key, 0, sizeof(key));
     std::memcpy(&key.P, &P, sizeof(P));
@@ -1462,6 +1499,7 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
     key.radix_passes = radix_passes;
     key.sort = sort ? 1 : 0;
     key.quads = quads ? 1 : 0;
+    key.depth = depth;
     return replay(graphs, &key, sizeof(key), stream, passes, enqueue);
 }
 
