@@ -303,8 +303,10 @@ __global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_extend(const __g
         }
     } else {
         PathRays<kOne> rays(P, queue, n);
-        using Walk = std::conditional_t<K == 2, InstWalk, WideWalk>;
-        trace_stream<false, Walk>(rays, WideStack{pt_stack + threadIdx.x, B, P.stack_depth}, status);
+        const WideStack stack{pt_stack + threadIdx.x, B, P.stack_depth};
+        if constexpr (K == 2) trace_stream<false, InstWalk>(rays, stack, status);
+        else if (short_queue(n)) trace_groups<false>(rays, n, stack, status);
+        else trace_stream<false, WideWalk>(rays, stack, status);
     }
     if (status) atomicOr(P.err, status);
 }
@@ -745,8 +747,10 @@ __global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_shadow(const __g
         }
     } else {
         ShadowRays<kOne> rays(P, n);
-        using Walk = std::conditional_t<K == 2, InstWalk, WideWalk>;
-        trace_stream<true, Walk>(rays, WideStack{pt_stack + threadIdx.x, B, P.stack_depth}, status);
+        const WideStack stack{pt_stack + threadIdx.x, B, P.stack_depth};
+        if constexpr (K == 2) trace_stream<true, InstWalk>(rays, stack, status);
+        else if (short_queue(n)) trace_groups<true>(rays, n, stack, status);
+        else trace_stream<true, WideWalk>(rays, stack, status);
     }
     if (status) atomicOr(P.err, status);
 }

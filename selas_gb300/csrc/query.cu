@@ -101,9 +101,10 @@ struct RecordRanges {
     uint32_t answer, barrier;  // shared memory: 16-byte answer, its mbarrier
 
     __device__ __forceinline__ RecordRanges(uint32_t count, bool more_blocks, const uint4* ans, const uint64_t* bar)
-        : n(count), status(0), claim(more_blocks), started(false), phase(0), answer(shared_address(ans)),
-          barrier(shared_address(bar)) {
+        : n(count), status(0), claim(more_blocks), started(false), phase(0), answer(0), barrier(0) {
         if (!claim) return;
+        answer = shared_address(ans);
+        barrier = shared_address(bar);
         if ((threadIdx.x & 31u) == 0) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barrier) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -243,6 +244,21 @@ __global__ void __launch_bounds__(32, 16) k_query_instanced(const __grid_constan
     query_warp<kAnyHit, true, InstWalk>(a);
 }
 
+// Batches of at most one ray a group of eight lanes: 4 rays a one-warp block.
+template <bool kAnyHit>
+__global__ void __launch_bounds__(32, kWarpsPerSm) k_query_groups(const __grid_constant__ QueryArgs a) {
+    extern __shared__ uint2 query_stack[];
+    RecordRays<kAnyHit, false> rays(a.n, false, nullptr, nullptr);
+    rays.node_array = a.nodes;
+    rays.tri_array = a.tris;
+    rays.recs = a.rays;
+    rays.record_float4s = a.record_float4s;
+    rays.order = nullptr;
+    uint32_t status = 0;
+    trace_groups<kAnyHit>(rays, a.n, WideStack{query_stack + threadIdx.x, 32, a.stack_depth}, status);
+    if (status) atomicOr(a.err, status);
+}
+
 template <bool kAnyHit>
 cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_float4s, uint32_t n,
                         const uint32_t* order, const uint32_t* ctl, uint32_t* d_err, cudaStream_t s) {
@@ -262,7 +278,10 @@ cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_fl
     a.claim = blocks > uint32_t(bvh.sm_count) * (inst ? 16u : uint32_t(kWarpsPerSm)) ? 1u : 0u;
     a.err = d_err;
     const size_t stack_bytes = size_t(bvh.stack_depth) * 32 * sizeof(uint2);
+    const uint32_t group_blocks = (n + 3u) / 4u;
     if (inst) k_query_instanced<kAnyHit><<<blocks, 32, stack_bytes, s>>>(a);
+    else if (group_blocks <= kGroupWaves * uint32_t(bvh.sm_count) * kWarpsPerSm)
+        k_query_groups<kAnyHit><<<group_blocks, 32, stack_bytes, s>>>(a);
     else k_query_wide<kAnyHit><<<blocks, 32, stack_bytes, s>>>(a);
     return cudaGetLastError();
 }

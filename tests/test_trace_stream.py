@@ -6,14 +6,17 @@ import pytest
 import oracle
 import selas_gb300 as sel
 from conftest import assert_hits_equal
+from edge_scenes import grid_rays, grid_scene, segment_rayhits, segment_rays
 from selas_gb300 import scenes
 
 pytestmark = pytest.mark.gpu
 
 RESIDENT = 152 * 32 * 32  # rays of a grid whose one-warp blocks all run at once on 152 SMs
+GROUPS = 152 * 32 * 4 * 3  # rays of the largest batch traced by eight lanes a ray
 
 
-@pytest.mark.parametrize("n", [1, 31, 32, 33, 1000, RESIDENT, RESIDENT + 1, 2 * RESIDENT + 37])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 31, 32, 33, 1000, GROUPS, GROUPS + 1, RESIDENT, RESIDENT + 1,
+                               2 * RESIDENT + 37])
 def test_batch_sizes(device, n):
     data = scenes.displaced_icospheres(count=2, level=2, seed=21)
     sc = sel.Scene(device)
@@ -56,4 +59,24 @@ def test_box_tests_stay_outside_the_boxes(device, scale, distance):
     if distance <= 1e4:
         assert (want["geomID"] != sel.INVALID_ID).mean() > 0.9
     assert_hits_equal(got, want, fields=("tfar", "u", "v", "primID", "geomID"))
+    sc.release()
+
+
+def test_ties_and_edges_in_long_batches(device):
+    """The edge-case rays (shared edges and vertices, ties, segment ends) among enough copies to be streamed."""
+    data = grid_scene()
+    sc = sel.Scene(device)
+    data.attach_to(sc)
+    sc.commit()
+    org, d, _ = grid_rays()
+    for make, query, ref in ((lambda: sel.make_rayhits(org, d), sc.intersect1M, oracle.intersect_bruteforce),
+                             (segment_rayhits, sc.intersect1M, oracle.intersect_bruteforce),
+                             (segment_rays, sc.occluded1M, oracle.occluded_bruteforce)):
+        want = make()
+        ref(data.soup(), want)
+        copies = GROUPS // want.size + 2
+        got = np.tile(make(), copies)
+        query(got)
+        assert_hits_equal(got, np.tile(want, copies), fields=("tfar",) if want.dtype == sel.RAY_DTYPE else
+                          ("tfar", "u", "v", "Ng_x", "primID", "geomID"))
     sc.release()
