@@ -1,39 +1,50 @@
-// Device SAH-binned BVH builder: the 8-wide quantised layout of bvh_build.cpp built on the GPU.
+// Device SAH BVH builder: the 8-wide quantised layout of bvh_build.cpp built on the GPU.
 //
-// Same method as the host builder (binned SAH after Wald 2007, 32 bins per axis, leaves of at most 3
-// triangles by default (1..8 selectable), object-median splits beyond depth 40, greedy collapse to 8 children by largest surface area,
-// octant slot assignment and outward 8-bit child-box quantisation after Ylitie, Karras and Laine 2017),
-// organised for the GPU:
-//   1. one thread per triangle: bounds, centroid (box centre, as the host builder);
-//   2. binary tree, top levels breadth first: every task of more than kSmall triangles is binned by many
-//      blocks (block-local bins flushed with atomics), one warp per task picks the split, and the
-//      triangles are partitioned with warp-aggregated cursors;
-//   3. subtrees of at most kSmall triangles: one warp each, depth first with a shared-memory task stack;
-//   4. collapse and quantisation breadth first: one thread per 8-wide node, scans place the next level's
-//      nodes and the leaf triangles.
+// Same method as the host builder (binned SAH after Wald 2007, 32 bins per axis, leaves of at most 3 triangles by
+// default (1..8 selectable), median splits beyond depth 40, greedy collapse to 8 children by largest surface area,
+// octant slot assignment and outward 8-bit child-box quantisation after Ylitie, Karras and Laine 2017), in four
+// launches:
+//   1. k_records: one thread per triangle: leaf record, bounds, scene box and centroid box;
+//   2. k_top (cooperative): subtrees of more than kSmall triangles, one level at a time: chunks of triangles are
+//      binned into block-local bins, one warp per subtree picks the split, chunks are partitioned;
+//   3. k_small: subtrees of at most kSmall triangles, one block each with the triangles' boxes in shared memory, one
+//      level at a time: a warp bins a part of more than 16 triangles, 16 or 8 lanes sweep smaller ones exactly
+//      (every centroid is a candidate plane);
+//   4. k_collapse (cooperative): collapse and quantisation one level at a time, eight lanes per 8-wide node.
 // Node slots follow the host builder's layout (a subtree of n triangles occupies slots [s, s + 2n - 1),
 // left child at s + 1, right child at s + 2 * n_left), so the tree needs no slot allocation.  Traversal
 // results do not depend on the tree (order-independent closest-hit rule, outward-rounded boxes).
+//
+// The build is bound by latency (dependent levels) and by the number of instructions per tree node, not by memory.
+// Before, one warp per subtree of 1,024 triangles, depth first, took 3.4 ms whatever the scene's size, a thread per
+// 8-wide node 0.07 ms a level, every level a round trip to the host, and the host made the leaf records.  Whole
+// commits now take (then): 22 triangles 0.15 (0.81) ms, 163,842 1.7 (9.6), 655,362 3.2 (18.5), 5,242,882 14.5 (109),
+// of which the upload and these kernels 0.15 (0.54), 1.7 (6.8), 3.1 (8.9), 14.4 (28.5).
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
-#include "scan.cuh"
 #include "sel_internal.h"
 
 namespace sel {
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 constexpr int kBinsD = 32;
+constexpr int kBinWords = 3 * kBinsD * 7;  // per bin: box lo, hi as ordered ints, count
 constexpr uint32_t kMaxLeafLimit = kMaxLeafRecords;  // leaves beyond a node's 32 records move one level down
 constexpr int kMedianDepthD = 40;
-constexpr uint32_t kSmall = 1024;   // subtrees at or below this many triangles are built by one warp
-constexpr int kWarpStack = 32;
-constexpr int kChunk = 2048;        // triangles per block in the large-task kernels (256 threads x 8)
-constexpr uint32_t kErrBuildStack = 1u;
+constexpr uint32_t kSmall = 1024;   // subtrees at or below this many triangles are built by one block
+constexpr uint32_t kChunk = 2048;   // triangles a block bins or partitions at a time (256 threads x 8)
+constexpr int kSmallWarps = 8;
+constexpr uint32_t kErrTooDeep = 1u, kErrNonFinite = 2u, kErrIndex = 4u;
 
 __device__ __forceinline__ int f2o(float f) {  // float -> int with the same order
     const int i = __float_as_int(f);
@@ -46,170 +57,119 @@ __device__ __forceinline__ float box_area(float3 lo, float3 hi) {
     const float dx = hi.x - lo.x, dy = hi.y - lo.y, dz = hi.z - lo.z;
     return 2.0f * (dx * dy + dy * dz + dz * dx);
 }
-
-struct Build {
-    const float4* soup;   // input triangles, 3 x float4 (TriRecord layout), input order
-    float4* plo;          // per triangle: box lo, w = input index bits
-    float4* phi;          // per triangle: box hi
-    uint32_t* idx;        // triangle order (subtree ranges)
-    uint32_t* idx_tmp;    // partition scratch
-    float4* nlo;          // binary nodes: box lo, w = left slot bits (leaf: all ones)
-    float4* nhi;          // box hi, w = right slot bits
-    uint2* nrange;        // first, count (count > 0: leaf)
-    uint4* tasks[2];      // large tasks: first, count, slot, depth
-    uint4* small;         // small subtrees
-    int* tbox;            // per large task: box lo/hi, centroid box lo/hi (ordered ints), 12 each
-    int* tbins;           // per large task: 3 axes x 32 bins x (6 box ints + count)
-    uint4* tsplit;        // per large task: mode (0 bins, 1 position), axis, bin, n_left
-    uint32_t* tcursor;    // per large task: left / right partition cursors
-    uint32_t* counters;   // [0] next large tasks, [1] small tasks, [2] max large count, [3] depth, [4] error
-    int* scene_box;       // 6 ordered ints
-    uint32_t n;
-    uint32_t max_leaf;    // triangles per leaf, 1..kMaxLeafLimit
-};
-
-__global__ void k_init_counters(Build B) {
-    if (threadIdx.x < 8) B.counters[threadIdx.x] = 0;
-    if (threadIdx.x < 6) B.scene_box[threadIdx.x] = threadIdx.x < 3 ? f2o(INFINITY) : f2o(-INFINITY);
+__device__ __forceinline__ float comp(const float4& v, int axis) { return axis == 0 ? v.x : (axis == 1 ? v.y : v.z); }
+__device__ __forceinline__ float centre(const float4& l, const float4& h, int axis) {
+    return 0.5f * (comp(l, axis) + comp(h, axis));
 }
-
-__global__ void __launch_bounds__(256) k_prims(Build B) {
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < B.n; i += gridDim.x * blockDim.x) {
-        const float4 a = B.soup[size_t(i) * 3], b = B.soup[size_t(i) * 3 + 1], c = B.soup[size_t(i) * 3 + 2];
-        const float3 l = make_float3(fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fminf(fminf(a.z, b.z), c.z));
-        const float3 h = make_float3(fmaxf(fmaxf(a.x, b.x), c.x), fmaxf(fmaxf(a.y, b.y), c.y), fmaxf(fmaxf(a.z, b.z), c.z));
-        B.plo[i] = make_float4(l.x, l.y, l.z, __uint_as_float(i));
-        B.phi[i] = make_float4(h.x, h.y, h.z, 0.0f);
-        B.idx[i] = i;
-        lo[0] = fminf(lo[0], l.x); lo[1] = fminf(lo[1], l.y); lo[2] = fminf(lo[2], l.z);
-        hi[0] = fmaxf(hi[0], h.x); hi[1] = fmaxf(hi[1], h.y); hi[2] = fmaxf(hi[2], h.z);
-    }
-    for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
-    }
-    if ((threadIdx.x & 31) == 0)
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(&B.scene_box[a], f2o(lo[a]));
-            atomicMax(&B.scene_box[3 + a], f2o(hi[a]));
-        }
-}
-
-__device__ __forceinline__ float centroid(const Build& B, uint32_t prim, int axis) {
-    const float4 l = B.plo[prim], h = B.phi[prim];
-    const float lo = axis == 0 ? l.x : (axis == 1 ? l.y : l.z);
-    const float hi = axis == 0 ? h.x : (axis == 1 ? h.y : h.z);
-    return 0.5f * (lo + hi);
-}
-
-// ---------------------------------------------------------------------------------------------------
-// Large tasks (more than kSmall triangles), one level at a time.
-// ---------------------------------------------------------------------------------------------------
-__global__ void k_task_init(Build B, int cur, uint32_t ntasks) {
-    const uint32_t words_box = 12, words_bins = 3 * kBinsD * 7;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ntasks * words_bins; i += gridDim.x * blockDim.x) {
-        const uint32_t w = i % 7;
-        B.tbins[i] = w < 3 ? f2o(INFINITY) : (w < 6 ? f2o(-INFINITY) : 0);
-    }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ntasks * words_box; i += gridDim.x * blockDim.x) {
-        const uint32_t w = i % 12;
-        B.tbox[i] = (w % 6) < 3 ? f2o(INFINITY) : f2o(-INFINITY);
-    }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * ntasks; i += gridDim.x * blockDim.x) B.tcursor[i] = 0;
-    (void)cur;
-}
-
-// Block-wide min/max of 12 floats (box lo/hi, centroid lo/hi), then one atomic per value.
-__global__ void __launch_bounds__(256) k_task_bounds(Build B, int cur) {
-    const uint4 t = B.tasks[cur][blockIdx.y];
-    const uint32_t first = t.x, count = t.y;
-    const uint32_t begin = blockIdx.x * kChunk;
-    if (begin >= count) return;
-    const uint32_t end = min(count, begin + kChunk);
-    float v[12];
-    for (int k = 0; k < 12; ++k) v[k] = (k % 6) < 3 ? INFINITY : -INFINITY;
-    for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        const uint32_t p = B.idx[first + i];
-        const float4 l = B.plo[p], h = B.phi[p];
-        const float c[3] = {0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z)};
-        v[0] = fminf(v[0], l.x); v[1] = fminf(v[1], l.y); v[2] = fminf(v[2], l.z);
-        v[3] = fmaxf(v[3], h.x); v[4] = fmaxf(v[4], h.y); v[5] = fmaxf(v[5], h.z);
-        v[6] = fminf(v[6], c[0]); v[7] = fminf(v[7], c[1]); v[8] = fminf(v[8], c[2]);
-        v[9] = fmaxf(v[9], c[0]); v[10] = fmaxf(v[10], c[1]); v[11] = fmaxf(v[11], c[2]);
-    }
-    __shared__ float red[12][8];
-    for (int k = 0; k < 12; ++k) {
-        for (int o = 16; o > 0; o >>= 1) {
-            const float y = __shfl_xor_sync(0xffffffffu, v[k], o);
-            v[k] = (k % 6) < 3 ? fminf(v[k], y) : fmaxf(v[k], y);
-        }
-        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = v[k];
-    }
-    __syncthreads();
-    if (threadIdx.x < 12) {
-        const int k = threadIdx.x;
-        float r = red[k][0];
-        for (int w = 1; w < 8; ++w) r = (k % 6) < 3 ? fminf(r, red[k][w]) : fmaxf(r, red[k][w]);
-        int* dst = B.tbox + size_t(blockIdx.y) * 12 + k;
-        if ((k % 6) < 3) atomicMin(dst, f2o(r));
-        else atomicMax(dst, f2o(r));
-    }
-}
-
 __device__ __forceinline__ int bin_of(float c, float lo, float k) {
     int b = int((c - lo) * k);
     return b < 0 ? 0 : (b > kBinsD - 1 ? kBinsD - 1 : b);
 }
+__device__ __forceinline__ float bin_scale(float ext) { return ext > 0.0f ? float(kBinsD) * (1.0f - 1e-6f) / ext : 0.0f; }
 
-__global__ void __launch_bounds__(256) k_task_bin(Build B, int cur) {
-    __shared__ int bins[3 * kBinsD * 7];
-    for (int i = threadIdx.x; i < 3 * kBinsD * 7; i += blockDim.x) {
-        const int w = i % 7;
-        bins[i] = w < 3 ? f2o(INFINITY) : (w < 6 ? f2o(-INFINITY) : 0);
-    }
-    __syncthreads();
-    const uint4 t = B.tasks[cur][blockIdx.y];
-    const uint32_t first = t.x, count = t.y;
-    const uint32_t begin = blockIdx.x * kChunk;
-    const int* tb = B.tbox + size_t(blockIdx.y) * 12;
-    float clo[3], kk[3];
-    for (int a = 0; a < 3; ++a) {
-        clo[a] = o2f(tb[6 + a]);
-        const float ext = o2f(tb[9 + a]) - clo[a];
-        kk[a] = ext > 0.0f ? float(kBinsD) * (1.0f - 1e-6f) / ext : 0.0f;
-    }
-    if (begin < count) {
-        const uint32_t end = min(count, begin + kChunk);
-        for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
-            const uint32_t p = B.idx[first + i];
-            const float4 l = B.plo[p], h = B.phi[p];
-            const float c[3] = {0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z)};
-            const int lo[3] = {f2o(l.x), f2o(l.y), f2o(l.z)}, hi[3] = {f2o(h.x), f2o(h.y), f2o(h.z)};
+// A mesh's arrays in HBM and its first triangle in the scene.
+struct MeshDev {
+    const float* vertices;
+    const uint32_t* indices;
+    uint32_t first, vertex_count, geom, kind;
+};
+
+// A subtree of more than kSmall triangles.
+struct TopTask {
+    uint32_t first, count, slot, depth;
+    uint32_t chunk0, pad[3];  // its first chunk in the level's chunk list
+    int box[6], cbox[6];      // bounds of the boxes and of the centroids (ordered ints)
+    uint32_t axis, bin, left_count, by_position;  // the split
+    uint32_t cursor[2];                           // triangles moved left / right so far
+    uint32_t child[2];                            // their tasks in the next level's list (all ones: small)
+};
+
+struct Counters {
+    uint32_t tasks[2], chunks[2], small, depth, err, pad;
+    int box[6], cbox[6];
+    uint32_t wide, tris, levels, pad2;
+};
+
+struct Build {
+    const MeshDev* meshes;
+    uint32_t mesh_count;
+    float4* soup;            // leaf records in input order, 3 x float4 (TriRecord)
+    float4* lo[2];           // per triangle: box lo, w = input index bits; partitions ping-pong
+    float4* hi[2];
+    uint32_t* idx;           // triangle order of the leaves
+    float4* nlo;             // binary nodes: box lo, w = left slot bits (leaf: all ones)
+    float4* nhi;             // box hi, w = right slot bits
+    uint2* nrange;           // first, count (count > 0: leaf)
+    TopTask* tasks[2];
+    int* bins;               // per task of the level
+    uint32_t* chunk_task[2]; // task of each chunk of the level
+    uint4* small;            // first, count, slot, depth | buffer << 31
+    Counters* ctr;
+    uint32_t n, max_leaf;
+};
+
+// ---------------------------------------------------------------------------------------------------
+// 1. Leaf records and bounds.
+// ---------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_records(Build B) {
+    float v[12];
+    for (int k = 0; k < 12; ++k) v[k] = (k % 6) < 3 ? INFINITY : -INFINITY;
+    uint32_t err = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < B.n; i += gridDim.x * blockDim.x) {
+        uint32_t m = 0, top = B.mesh_count;  // the last mesh whose first triangle is at or below i
+        while (top - m > 1) {
+            const uint32_t mid = (m + top) >> 1;
+            if (B.meshes[mid].first <= i) m = mid;
+            else top = mid;
+        }
+        const MeshDev& M = B.meshes[m];
+        const uint32_t t = i - M.first;
+        float p[3][3];
+        for (int k = 0; k < 3; ++k) {
+            uint32_t vi = M.indices[3 * size_t(t) + k];
+            if (vi >= M.vertex_count) {
+                err |= kErrIndex;
+                vi = 0;
+            }
             for (int a = 0; a < 3; ++a) {
-                int* b = bins + (a * kBinsD + bin_of(c[a], clo[a], kk[a])) * 7;
-                for (int q = 0; q < 3; ++q) {
-                    atomicMin(b + q, lo[q]);
-                    atomicMax(b + 3 + q, hi[q]);
-                }
-                atomicAdd(b + 6, 1);
+                p[k][a] = M.vertices[3 * size_t(vi) + a];
+                if (!isfinite(p[k][a])) err |= kErrNonFinite;
             }
         }
+        float4* rec = B.soup + size_t(i) * 3;
+        rec[0] = make_float4(p[0][0], p[0][1], p[0][2], __uint_as_float(t));
+        rec[1] = make_float4(p[1][0], p[1][1], p[1][2], __uint_as_float(M.geom));
+        rec[2] = make_float4(p[2][0], p[2][1], p[2][2], __uint_as_float(M.kind));
+        float l[3], h[3];
+        for (int a = 0; a < 3; ++a) {
+            l[a] = fminf(fminf(p[0][a], p[1][a]), p[2][a]);
+            h[a] = fmaxf(fmaxf(p[0][a], p[1][a]), p[2][a]);
+            const float c = 0.5f * (l[a] + h[a]);
+            v[a] = fminf(v[a], l[a]);
+            v[3 + a] = fmaxf(v[3 + a], h[a]);
+            v[6 + a] = fminf(v[6 + a], c);
+            v[9 + a] = fmaxf(v[9 + a], c);
+        }
+        B.lo[0][i] = make_float4(l[0], l[1], l[2], __uint_as_float(i));
+        B.hi[0][i] = make_float4(h[0], h[1], h[2], 0.0f);
     }
-    __syncthreads();
-    int* g = B.tbins + size_t(blockIdx.y) * 3 * kBinsD * 7;
-    for (int i = threadIdx.x; i < 3 * kBinsD * 7; i += blockDim.x) {
-        const int w = i % 7;
-        if (w < 3) atomicMin(g + i, bins[i]);
-        else if (w < 6) atomicMax(g + i, bins[i]);
-        else if (bins[i]) atomicAdd(g + i, bins[i]);
+    if (err) atomicOr(&B.ctr->err, err);
+    for (int k = 0; k < 12; ++k) {
+        const int o = (k % 6) < 3 ? __reduce_min_sync(0xffffffffu, f2o(v[k])) : __reduce_max_sync(0xffffffffu, f2o(v[k]));
+        int* dst = k < 6 ? &B.ctr->box[k] : &B.ctr->cbox[k - 6];
+        if ((threadIdx.x & 31) == 0) {
+            if ((k % 6) < 3) atomicMin(dst, o);
+            else atomicMax(dst, o);
+        }
     }
 }
 
-// SAH over 32 bins of one axis, lane b = bin b: returns the lane-0 view of (cost, n_left) of the best split
-// after bin b for each lane (cost +inf where a side is empty).
+// ---------------------------------------------------------------------------------------------------
+// 2. Subtrees of more than kSmall triangles, level by level.
+// ---------------------------------------------------------------------------------------------------
+
+// SAH over the 32 bins of one axis, lane b = bin b: the cost of splitting after bin b (infinite where a side is
+// empty) and the triangles left of it.
 __device__ __forceinline__ void sah_sweep(const int* bins, int lane, float& cost, uint32_t& nleft) {
     const int* b = bins + lane * 7;
     float lo[3] = {o2f(b[0]), o2f(b[1]), o2f(b[2])}, hi[3] = {o2f(b[3]), o2f(b[4]), o2f(b[5])};
@@ -247,695 +207,924 @@ __device__ __forceinline__ void sah_sweep(const int* bins, int lane, float& cost
     }
 }
 
-__global__ void k_task_split(Build B, int cur, uint32_t ntasks) {
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= ntasks) return;
-    const uint4 t = B.tasks[cur][warp];
-    const uint32_t first = t.x, count = t.y, slot = t.z, depth = t.w;
-    const int* tb = B.tbox + size_t(warp) * 12;
-    float lo[3], hi[3], clo[3], chi[3];
+// The best binned split of a part with centroid bounds clo..chi: its axis (-1: none), bin, left count and cost.
+__device__ __forceinline__ int best_bin_split(const int* bins, const float* clo, const float* chi, int lane,
+                                              uint32_t& bin, uint32_t& nl, float& best) {
+    best = INFINITY;
+    int best_axis = -1;
     for (int a = 0; a < 3; ++a) {
-        lo[a] = o2f(tb[a]); hi[a] = o2f(tb[3 + a]); clo[a] = o2f(tb[6 + a]); chi[a] = o2f(tb[9 + a]);
+        if (!(chi[a] > clo[a])) continue;
+        float cost;
+        uint32_t n_left;
+        sah_sweep(bins + a * kBinsD * 7, lane, cost, n_left);
+        const int key = f2o(cost);
+        const int least = __reduce_min_sync(0xffffffffu, key);
+        const int bb = __ffs(__ballot_sync(0xffffffffu, key == least)) - 1;  // ties to the lower bin
+        const float bc = o2f(least);
+        const uint32_t nlb = __shfl_sync(0xffffffffu, n_left, bb);
+        if (bc < best) {
+            best = bc;
+            best_axis = a;
+            bin = uint32_t(bb);
+            nl = nlb;
+        }
+    }
+    return best_axis;
+}
+
+__device__ __forceinline__ void clear_bins(int* bins, int i0, int step) {
+    for (int i = i0; i < kBinWords; i += step) {
+        const int w = i % 7;
+        bins[i] = w < 3 ? f2o(INFINITY) : (w < 6 ? f2o(-INFINITY) : 0);
+    }
+}
+
+__device__ __forceinline__ void bin_prim(int* bins, const float4& l, const float4& h, const float* clo, const float* kk) {
+    const int lo[3] = {f2o(l.x), f2o(l.y), f2o(l.z)}, hi[3] = {f2o(h.x), f2o(h.y), f2o(h.z)};
+    for (int a = 0; a < 3; ++a) {
+        int* b = bins + (a * kBinsD + bin_of(centre(l, h, a), clo[a], kk[a])) * 7;
+        for (int q = 0; q < 3; ++q) {
+            atomicMin(b + q, lo[q]);
+            atomicMax(b + 3 + q, hi[q]);
+        }
+        atomicAdd(b + 6, 1);
+    }
+}
+
+// Adds a subtree to the next level's list, or to the small ones (one lane).  Returns its task index.
+__device__ uint32_t add_task(const Build& B, int next, uint32_t first, uint32_t count, uint32_t slot, uint32_t depth,
+                             int buffer) {
+    if (count <= kSmall) {
+        B.small[atomicAdd(&B.ctr->small, 1u)] = make_uint4(first, count, slot, depth | (uint32_t(buffer) << 31));
+        return 0xffffffffu;
+    }
+    const uint32_t q = atomicAdd(&B.ctr->tasks[next], 1u);
+    const uint32_t chunks = (count + kChunk - 1) / kChunk;
+    const uint32_t c0 = atomicAdd(&B.ctr->chunks[next], chunks);
+    TopTask& t = B.tasks[next][q];
+    t.first = first;
+    t.count = count;
+    t.slot = slot;
+    t.depth = depth;
+    t.chunk0 = c0;
+    for (int k = 0; k < 6; ++k) t.box[k] = t.cbox[k] = k < 3 ? f2o(INFINITY) : f2o(-INFINITY);
+    t.cursor[0] = t.cursor[1] = 0;
+    for (uint32_t k = 0; k < chunks; ++k) B.chunk_task[next][c0 + k] = q;
+    return q;
+}
+
+__device__ void split_task(const Build& B, int cur, uint32_t index, int lane) {
+    TopTask& t = B.tasks[cur][index];
+    const uint32_t count = t.count, depth = t.depth;
+    float clo[3], chi[3];
+    for (int a = 0; a < 3; ++a) {
+        clo[a] = o2f(t.cbox[a]);
+        chi[a] = o2f(t.cbox[3 + a]);
     }
     int axis = 0;
     for (int a = 1; a < 3; ++a)
         if (chi[a] - clo[a] > chi[axis] - clo[axis]) axis = a;
     const bool degenerate = !(chi[axis] > clo[axis]);
-    const int* bins = B.tbins + size_t(warp) * 3 * kBinsD * 7;
-    uint32_t mode = 1, split_axis = uint32_t(axis), split_bin = 0, nl = count / 2;
+    const int* bins = B.bins + size_t(index) * kBinWords;
+    uint32_t by_position = 1, split_axis = uint32_t(axis), bin = 0, nl = count / 2;
     if (!degenerate && int(depth) < kMedianDepthD) {
-        float best = INFINITY;
-        for (int a = 0; a < 3; ++a) {
-            if (!(chi[a] > clo[a])) continue;
-            float cost;
-            uint32_t n_left;
-            sah_sweep(bins + a * kBinsD * 7, lane, cost, n_left);
-            // warp argmin, ties to the lower bin
-            float bc = cost;
-            int bb = lane;
-            for (int o = 16; o > 0; o >>= 1) {
-                const float oc = __shfl_xor_sync(0xffffffffu, bc, o);
-                const int ob = __shfl_xor_sync(0xffffffffu, bb, o);
-                if (oc < bc || (oc == bc && ob < bb)) { bc = oc; bb = ob; }
-            }
-            const uint32_t nlb = __shfl_sync(0xffffffffu, n_left, bb);
-            if (bc < best) {
-                best = bc;
-                mode = 0;
-                split_axis = uint32_t(a);
-                split_bin = uint32_t(bb);
-                nl = nlb;
-            }
+        float cost;
+        const int a = best_bin_split(bins, clo, chi, lane, bin, nl, cost);
+        if (a >= 0) {
+            split_axis = uint32_t(a);
+            by_position = 0;
         }
     } else if (!degenerate) {
         // object median through the bins of the widest axis: the bin where half of the triangles is reached
-        uint32_t c = uint32_t(bins[(axis * kBinsD + lane) * 7 + 6]), incl = c;
+        uint32_t incl = uint32_t(bins[(axis * kBinsD + lane) * 7 + 6]);
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += u;
         }
         const uint32_t ok = __ballot_sync(0xffffffffu, incl >= count / 2 && incl < count);
         if (ok) {
-            const int bb = __ffs(ok) - 1;
-            mode = 0;
-            split_bin = uint32_t(bb);
-            nl = __shfl_sync(0xffffffffu, incl, bb);
+            by_position = 0;
+            bin = uint32_t(__ffs(ok) - 1);
+            nl = __shfl_sync(0xffffffffu, incl, int(bin));
         }
     }
-    if (nl == 0 || nl >= count) { mode = 1; nl = count / 2; }
+    if (nl == 0 || nl >= count) {
+        by_position = 1;
+        nl = count / 2;
+    }
     if (lane == 0) {
-        B.tsplit[warp] = make_uint4(mode, split_axis, split_bin, nl);
-        const uint32_t nr = count - nl;
-        const uint32_t left = slot + 1, right = slot + 2 * nl;
-        B.nlo[slot] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(left));
-        B.nhi[slot] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(right));
-        B.nrange[slot] = make_uint2(first, 0);
-        atomicMax(&B.counters[3], depth + 1);
-        const uint4 kids[2] = {make_uint4(first, nl, left, depth + 1), make_uint4(first + nl, nr, right, depth + 1)};
-        for (int k = 0; k < 2; ++k) {
-            if (kids[k].y > kSmall) {
-                const uint32_t q = atomicAdd(&B.counters[0], 1u);
-                B.tasks[cur ^ 1][q] = kids[k];
-                atomicMax(&B.counters[2], kids[k].y);
-            } else {
-                const uint32_t q = atomicAdd(&B.counters[1], 1u);
-                B.small[q] = kids[k];
-            }
-        }
+        t.axis = split_axis;
+        t.bin = bin;
+        t.left_count = nl;
+        t.by_position = by_position;
+        const uint32_t left = t.slot + 1, right = t.slot + 2 * nl;
+        B.nlo[t.slot] = make_float4(o2f(t.box[0]), o2f(t.box[1]), o2f(t.box[2]), __uint_as_float(left));
+        B.nhi[t.slot] = make_float4(o2f(t.box[3]), o2f(t.box[4]), o2f(t.box[5]), __uint_as_float(right));
+        B.nrange[t.slot] = make_uint2(t.first, 0);
+        const int next = cur ^ 1;  // the triangles move to the other buffer with the level
+        t.child[0] = add_task(B, next, t.first, nl, left, depth + 1, next);
+        t.child[1] = add_task(B, next, t.first + nl, count - nl, right, depth + 1, next);
     }
 }
 
-__global__ void __launch_bounds__(256) k_task_partition(Build B, int cur) {
-    const uint4 t = B.tasks[cur][blockIdx.y];
-    const uint32_t first = t.x, count = t.y;
-    const uint4 sp = B.tsplit[blockIdx.y];
-    const int* tb = B.tbox + size_t(blockIdx.y) * 12;
-    const int a = int(sp.y);
-    const float clo = o2f(tb[6 + a]);
-    const float ext = o2f(tb[9 + a]) - clo;
-    const float k = ext > 0.0f ? float(kBinsD) * (1.0f - 1e-6f) / ext : 0.0f;
-    const uint32_t begin = blockIdx.x * kChunk;
-    if (begin >= count) return;
-    const uint32_t end = min(count, begin + kChunk);
+// Moves a chunk's triangles to their sides in the other buffer and grows the bounds of the children's tasks.
+__device__ void partition_chunk(const Build& B, int cur, uint32_t chunk) {
+    __shared__ uint32_t warp_left[8], warp_right[8], base_left, base_right;
+    __shared__ int child_box[2][12];
+    const TopTask& t = B.tasks[cur][B.chunk_task[cur][chunk]];
+    const uint32_t begin = (chunk - t.chunk0) * kChunk, end = min(t.count, begin + kChunk);
+    const int a = int(t.axis), lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const float clo = o2f(t.cbox[a]), kk = bin_scale(o2f(t.cbox[3 + a]) - clo);
+    if (threadIdx.x < 24) child_box[threadIdx.x / 12][threadIdx.x % 12] = (threadIdx.x % 6) < 3 ? f2o(INFINITY) : f2o(-INFINITY);
+    float4 l[8], h[8];
+    uint32_t left = 0, n_left = 0, n_right = 0;  // bit k: the thread's k-th triangle goes left
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t i = begin + uint32_t(k) * 256u + threadIdx.x;
+        if (i >= end) continue;
+        l[k] = B.lo[cur][t.first + i];
+        h[k] = B.hi[cur][t.first + i];
+        const bool go = t.by_position ? i < t.left_count : bin_of(centre(l[k], h[k], a), clo, kk) <= int(t.bin);
+        left |= uint32_t(go) << k;
+        n_left += go;
+        n_right += !go;
+    }
+    // exclusive offsets of the threads' triangles within the block
+    uint32_t il = n_left, ir = n_right;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, il, o), y = __shfl_up_sync(0xffffffffu, ir, o);
+        if (lane >= o) {
+            il += x;
+            ir += y;
+        }
+    }
+    if (lane == 31) {
+        warp_left[w] = il;
+        warp_right[w] = ir;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t sl = 0, sr = 0;
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t x = warp_left[k], y = warp_right[k];
+            warp_left[k] = sl;
+            warp_right[k] = sr;
+            sl += x;
+            sr += y;
+        }
+        TopTask& out = B.tasks[cur][B.chunk_task[cur][chunk]];
+        base_left = sl ? atomicAdd(&out.cursor[0], sl) : 0u;
+        base_right = sr ? atomicAdd(&out.cursor[1], sr) : 0u;
+    }
+    __syncthreads();
+    uint32_t at_left = t.first + base_left + warp_left[w] + il - n_left;
+    uint32_t at_right = t.first + t.left_count + base_right + warp_right[w] + ir - n_right;
+    int v[2][12];
+    for (int c = 0; c < 2; ++c)
+        for (int k = 0; k < 12; ++k) v[c][k] = (k % 6) < 3 ? f2o(INFINITY) : f2o(-INFINITY);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const uint32_t i = begin + uint32_t(k) * 256u + threadIdx.x;
+        if (i >= end) continue;
+        const int c = (left >> k) & 1u ? 0 : 1;
+        const uint32_t dst = c == 0 ? at_left++ : at_right++;
+        B.lo[cur ^ 1][dst] = l[k];
+        B.hi[cur ^ 1][dst] = h[k];
+        for (int q = 0; q < 3; ++q) {
+            const int lo = f2o(comp(l[k], q)), hi = f2o(comp(h[k], q)), ce = f2o(centre(l[k], h[k], q));
+            for (int side = 0; side < 2; ++side) {
+                if (side != c) continue;
+                v[side][q] = min(v[side][q], lo);
+                v[side][3 + q] = max(v[side][3 + q], hi);
+                v[side][6 + q] = min(v[side][6 + q], ce);
+                v[side][9 + q] = max(v[side][9 + q], ce);
+            }
+        }
+    }
+    for (int c = 0; c < 2; ++c) {
+        if (t.child[c] == 0xffffffffu) continue;  // small subtrees find their bounds themselves
+        for (int k = 0; k < 12; ++k) {
+            const int r = (k % 6) < 3 ? __reduce_min_sync(0xffffffffu, v[c][k]) : __reduce_max_sync(0xffffffffu, v[c][k]);
+            if (lane == 0) {
+                if ((k % 6) < 3) atomicMin(&child_box[c][k], r);
+                else atomicMax(&child_box[c][k], r);
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 24) {
+        const int c = threadIdx.x / 12, k = threadIdx.x % 12;
+        if (t.child[c] != 0xffffffffu) {
+            TopTask& child = B.tasks[cur ^ 1][t.child[c]];
+            int* dst = k < 6 ? &child.box[k] : &child.cbox[k - 6];
+            if ((k % 6) < 3) atomicMin(dst, child_box[c][k]);
+            else atomicMax(dst, child_box[c][k]);
+        }
+    }
+    __syncthreads();  // the shared words are the next chunk's
+}
+
+__global__ void __launch_bounds__(256, 2) k_top(Build B) {
+    if (B.ctr->err) return;  // bad input, found by k_records
+    cg::grid_group grid = cg::this_grid();
+    __shared__ int bins[kBinWords];
     const int lane = threadIdx.x & 31;
-    for (uint32_t base = begin; base < end; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        const bool valid = i < end;
-        uint32_t p = 0;
-        bool left = false;
-        if (valid) {
-            p = B.idx[first + i];
-            left = sp.x == 0 ? bin_of(centroid(B, p, a), clo, k) <= int(sp.z) : i < sp.w;
-        }
-        const uint32_t lm = __ballot_sync(0xffffffffu, valid && left), rm = __ballot_sync(0xffffffffu, valid && !left);
-        uint32_t lb = 0, rb = 0;
-        if (lane == 0) {
-            if (lm) lb = atomicAdd(&B.tcursor[2 * blockIdx.y], __popc(lm));
-            if (rm) rb = atomicAdd(&B.tcursor[2 * blockIdx.y + 1], __popc(rm));
-        }
-        lb = __shfl_sync(0xffffffffu, lb, 0);
-        rb = __shfl_sync(0xffffffffu, rb, 0);
-        const uint32_t below = (1u << lane) - 1u;
-        if (valid) {
-            const uint32_t dst = left ? first + lb + __popc(lm & below) : first + sp.w + rb + __popc(rm & below);
-            B.idx_tmp[dst] = p;
-        }
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the root
+        const uint32_t q = add_task(B, 0, 0, B.n, 0, 0, 0);
+        if (q != 0xffffffffu)
+            for (int k = 0; k < 6; ++k) {
+                B.tasks[0][q].box[k] = B.ctr->box[k];
+                B.tasks[0][q].cbox[k] = B.ctr->cbox[k];
+            }
     }
-}
-
-__global__ void __launch_bounds__(256) k_task_copy_back(Build B, int cur) {
-    const uint4 t = B.tasks[cur][blockIdx.y];
-    const uint32_t first = t.x, count = t.y;
-    const uint32_t begin = blockIdx.x * kChunk;
-    if (begin >= count) return;
-    const uint32_t end = min(count, begin + kChunk);
-    for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) B.idx[first + i] = B.idx_tmp[first + i];
-}
-
-// ---------------------------------------------------------------------------------------------------
-// Small subtrees: one warp each, depth first (the larger child waits on the stack, so it holds at most
-// log2(kSmall) entries).
-// ---------------------------------------------------------------------------------------------------
-constexpr int kSmallWarps = 4;
-
-__global__ void __launch_bounds__(32 * kSmallWarps) k_small(Build B) {
-    __shared__ int sbins[kSmallWarps][3 * kBinsD * 7];
-    __shared__ uint4 sstack[kSmallWarps][kWarpStack];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int* bins = sbins[w];
-    uint4* stack = sstack[w];
-    const uint32_t ntasks = B.counters[1];
-    for (uint32_t task = blockIdx.x * kSmallWarps + w; task < ntasks; task += gridDim.x * kSmallWarps) {
-        int sp = 0;
-        uint4 t = B.small[task];
-        for (;;) {
-            const uint32_t first = t.x, count = t.y, slot = t.z, depth = t.w;
-            float v[12];
-            for (int k = 0; k < 12; ++k) v[k] = (k % 6) < 3 ? INFINITY : -INFINITY;
-            for (uint32_t i = lane; i < count; i += 32) {
-                const uint32_t p = B.idx[first + i];
-                const float4 l = B.plo[p], h = B.phi[p];
-                const float c[3] = {0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z)};
-                v[0] = fminf(v[0], l.x); v[1] = fminf(v[1], l.y); v[2] = fminf(v[2], l.z);
-                v[3] = fmaxf(v[3], h.x); v[4] = fmaxf(v[4], h.y); v[5] = fmaxf(v[5], h.z);
-                v[6] = fminf(v[6], c[0]); v[7] = fminf(v[7], c[1]); v[8] = fminf(v[8], c[2]);
-                v[9] = fmaxf(v[9], c[0]); v[10] = fmaxf(v[10], c[1]); v[11] = fmaxf(v[11], c[2]);
+    grid.sync();
+    for (int cur = 0;; cur ^= 1) {
+        const uint32_t ntasks = *(volatile uint32_t*)&B.ctr->tasks[cur];
+        const uint32_t nchunks = *(volatile uint32_t*)&B.ctr->chunks[cur];
+        if (ntasks == 0) break;
+        for (uint32_t t = blockIdx.x; t < ntasks; t += gridDim.x)
+            clear_bins(B.bins + size_t(t) * kBinWords, threadIdx.x, 256);
+        if (blockIdx.x == 0 && threadIdx.x == 0) B.ctr->tasks[cur ^ 1] = B.ctr->chunks[cur ^ 1] = 0;
+        grid.sync();
+        for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+            const uint32_t index = B.chunk_task[cur][c];
+            const TopTask& t = B.tasks[cur][index];
+            const uint32_t begin = (c - t.chunk0) * kChunk, end = min(t.count, begin + kChunk);
+            float clo[3], kk[3];
+            for (int a = 0; a < 3; ++a) {
+                clo[a] = o2f(t.cbox[a]);
+                kk[a] = bin_scale(o2f(t.cbox[3 + a]) - clo[a]);
             }
-            for (int k = 0; k < 12; ++k)
-                for (int o = 16; o > 0; o >>= 1) {
-                    const float y = __shfl_xor_sync(0xffffffffu, v[k], o);
-                    v[k] = (k % 6) < 3 ? fminf(v[k], y) : fmaxf(v[k], y);
-                }
-            if (lane == 0) atomicMax(&B.counters[3], depth + 1);
-            bool leaf = count <= 1;
-            uint32_t mode = 1, split_axis = 0, split_bin = 0, nl = count / 2;
-            int axis = 0;
-            for (int a = 1; a < 3; ++a)
-                if (v[9 + a] - v[6 + a] > v[9 + axis] - v[6 + axis]) axis = a;
-            split_axis = uint32_t(axis);
-            const bool degenerate = !(v[9 + axis] > v[6 + axis]);
-            if (!leaf && (degenerate || int(depth) >= kMedianDepthD)) {
-                leaf = count <= B.max_leaf;  // otherwise split by position
-            } else if (!leaf) {
-                for (int i = lane; i < 3 * kBinsD * 7; i += 32) {
-                    const int q = i % 7;
-                    bins[i] = q < 3 ? f2o(INFINITY) : (q < 6 ? f2o(-INFINITY) : 0);
-                }
-                __syncwarp();
-                float kk[3];
-                for (int a = 0; a < 3; ++a) {
-                    const float ext = v[9 + a] - v[6 + a];
-                    kk[a] = ext > 0.0f ? float(kBinsD) * (1.0f - 1e-6f) / ext : 0.0f;
-                }
-                for (uint32_t i = lane; i < count; i += 32) {
-                    const uint32_t p = B.idx[first + i];
-                    const float4 l = B.plo[p], h = B.phi[p];
-                    const float c[3] = {0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z)};
-                    const int lo[3] = {f2o(l.x), f2o(l.y), f2o(l.z)}, hi[3] = {f2o(h.x), f2o(h.y), f2o(h.z)};
-                    for (int a = 0; a < 3; ++a) {
-                        if (!(v[9 + a] > v[6 + a])) continue;
-                        int* b = bins + (a * kBinsD + bin_of(c[a], v[6 + a], kk[a])) * 7;
-                        for (int q = 0; q < 3; ++q) {
-                            atomicMin(b + q, lo[q]);
-                            atomicMax(b + 3 + q, hi[q]);
-                        }
-                        atomicAdd(b + 6, 1);
-                    }
-                }
-                __syncwarp();
-                float best = INFINITY;
-                int best_axis = -1;
-                for (int a = 0; a < 3; ++a) {
-                    if (!(v[9 + a] > v[6 + a])) continue;
-                    float cost;
-                    uint32_t n_left;
-                    sah_sweep(bins + a * kBinsD * 7, lane, cost, n_left);
-                    float bc = cost;
-                    int bb = lane;
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const float oc = __shfl_xor_sync(0xffffffffu, bc, o);
-                        const int ob = __shfl_xor_sync(0xffffffffu, bb, o);
-                        if (oc < bc || (oc == bc && ob < bb)) { bc = oc; bb = ob; }
-                    }
-                    const uint32_t nlb = __shfl_sync(0xffffffffu, n_left, bb);
-                    if (bc < best) {
-                        best = bc;
-                        best_axis = a;
-                        split_bin = uint32_t(bb);
-                        nl = nlb;
-                    }
-                }
-                const float parent = box_area(make_float3(v[0], v[1], v[2]), make_float3(v[3], v[4], v[5]));
-                const float leaf_cost = parent * float(count);
-                const float split_cost = parent + best;
-                if (count <= B.max_leaf && (best_axis < 0 || split_cost >= leaf_cost)) {
-                    leaf = true;
-                } else if (best_axis >= 0) {
-                    mode = 0;
-                    split_axis = uint32_t(best_axis);
-                }
-                __syncwarp();
+            clear_bins(bins, threadIdx.x, 256);
+            __syncthreads();
+            for (uint32_t i = begin + threadIdx.x; i < end; i += 256)
+                bin_prim(bins, B.lo[cur][t.first + i], B.hi[cur][t.first + i], clo, kk);
+            __syncthreads();
+            int* g = B.bins + size_t(index) * kBinWords;
+            for (int i = threadIdx.x; i < kBinWords; i += 256) {
+                if (!bins[i - i % 7 + 6]) continue;  // an empty bin
+                const int w = i % 7;
+                if (w < 3) atomicMin(g + i, bins[i]);
+                else if (w < 6) atomicMax(g + i, bins[i]);
+                else atomicAdd(g + i, bins[i]);
             }
-            if (!leaf && (nl == 0 || nl >= count)) { mode = 1; nl = count / 2; }
-            if (leaf) {
-                if (lane == 0) {
-                    B.nlo[slot] = make_float4(v[0], v[1], v[2], __uint_as_float(0xffffffffu));
-                    B.nhi[slot] = make_float4(v[3], v[4], v[5], __uint_as_float(0xffffffffu));
-                    B.nrange[slot] = make_uint2(first, count);
-                }
-            } else {
-                // stable partition into the scratch range, then back
-                const float ext = v[9 + split_axis] - v[6 + split_axis];
-                const float k = ext > 0.0f ? float(kBinsD) * (1.0f - 1e-6f) / ext : 0.0f;
-                uint32_t lcount = 0, rcount = 0;
-                for (uint32_t base = 0; base < count; base += 32) {
-                    const uint32_t i = base + lane;
-                    const bool valid = i < count;
-                    uint32_t p = 0;
-                    bool left = false;
-                    if (valid) {
-                        p = B.idx[first + i];
-                        left = mode == 0 ? bin_of(centroid(B, p, int(split_axis)), v[6 + split_axis], k) <= int(split_bin)
-                                         : i < nl;
-                    }
-                    const uint32_t lm = __ballot_sync(0xffffffffu, valid && left);
-                    const uint32_t rm = __ballot_sync(0xffffffffu, valid && !left);
-                    const uint32_t below = (1u << lane) - 1u;
-                    if (valid) {
-                        const uint32_t dst = left ? first + lcount + __popc(lm & below)
-                                                  : first + nl + rcount + __popc(rm & below);
-                        if (dst < first + count) B.idx_tmp[dst] = p;
-                    }
-                    lcount += __popc(lm);
-                    rcount += __popc(rm);
-                }
-                __syncwarp();
-                for (uint32_t i = lane; i < count; i += 32) B.idx[first + i] = B.idx_tmp[first + i];
-                __syncwarp();
-                const uint32_t nr = count - nl;
-                const uint32_t left = slot + 1, right = slot + 2 * nl;
-                if (lane == 0) {
-                    B.nlo[slot] = make_float4(v[0], v[1], v[2], __uint_as_float(left));
-                    B.nhi[slot] = make_float4(v[3], v[4], v[5], __uint_as_float(right));
-                    B.nrange[slot] = make_uint2(first, 0);
-                }
-                const uint4 l4 = make_uint4(first, nl, left, depth + 1), r4 = make_uint4(first + nl, nr, right, depth + 1);
-                const bool left_smaller = nl <= nr;
-                if (sp >= kWarpStack) {  // cannot happen (depth-first on the smaller child): record, stop
-                    if (lane == 0) atomicOr(&B.counters[4], kErrBuildStack);
-                    break;
-                }
-                if (lane == 0) stack[sp] = left_smaller ? r4 : l4;
-                __syncwarp();
-                ++sp;
-                t = left_smaller ? l4 : r4;
-                continue;
-            }
-            if (sp == 0) break;
-            --sp;
-            __syncwarp();
-            t = stack[sp];
-            __syncwarp();
+            __syncthreads();
         }
+        grid.sync();
+        for (uint32_t t = warp; t < ntasks; t += warps) split_task(B, cur, t, lane);
+        grid.sync();
+        for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) partition_chunk(B, cur, c);
+        grid.sync();
     }
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Collapse to 8-wide nodes and quantisation, one level at a time.
+// 3. Subtrees of at most kSmall triangles, one block each.
 // ---------------------------------------------------------------------------------------------------
-struct Collapse {
-    const uint2* level;   // (wide index, binary node)
-    uint2* next;
-    int* slots;           // per entry: 8 binary children in slot order (-1 empty)
-    uint32_t* cnt_int;    // internal children per entry
-    uint32_t* cnt_tri;    // leaf triangles per entry
-    uint32_t* off_int;
-    uint32_t* off_tri;
-    WideNode* nodes;
-    TriRecord* tris;
+
+// A part of the subtree: first and count within the block's order array, depth, node slot.
+__device__ __forceinline__ uint2 pack_part(uint32_t first, uint32_t count, uint32_t depth, uint32_t slot) {
+    return make_uint2(first | (count << 10) | (depth << 21), slot);
+}
+
+constexpr uint32_t kBigParts = kSmall / 17 + 1, kMidParts = kSmall / 9 + 1, kTinyParts = kSmall / 2;
+
+struct SmallShared {
+    float box[6][kSmall];            // lo x y z, hi x y z of triangle k
+    uint32_t tri[kSmall];            // its input index
+    uint16_t order[2][kSmall];       // order and partition scratch
+    int bins[kSmallWarps][kBinWords];
+    uint2 big[2][kBigParts], mid[2][kMidParts], tiny[2][kTinyParts];
+    uint32_t counts[2][3];
 };
 
-__device__ __forceinline__ bool is_leaf(const Build& B, int n) { return B.nrange[n].y > 0; }
-
-__global__ void __launch_bounds__(128) k_collapse_gather(Build B, Collapse C, uint32_t count) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const int root = int(C.level[i].y);
-    int children[8];
-    int nc = 0;
-    if (is_leaf(B, root)) {
-        children[nc++] = root;
-    } else {
-        children[nc++] = int(__float_as_uint(B.nlo[root].w));
-        children[nc++] = int(__float_as_uint(B.nhi[root].w));
-        while (nc < 8) {
-            int best = -1;
-            float best_area = -1.0f;
-            for (int k = 0; k < nc; ++k) {
-                if (is_leaf(B, children[k])) continue;
-                const float4 l = B.nlo[children[k]], h = B.nhi[children[k]];
-                const float a = box_area(make_float3(l.x, l.y, l.z), make_float3(h.x, h.y, h.z));
-                if (a > best_area) { best_area = a; best = k; }
-            }
-            if (best < 0) break;
-            const int opened = children[best];
-            children[best] = int(__float_as_uint(B.nlo[opened].w));
-            children[nc++] = int(__float_as_uint(B.nhi[opened].w));
-        }
-    }
-    // slot assignment by octant direction (the host builder's rule): candidates (cost, child, slot) in
-    // ascending cost, ties in (child, slot) order as a stable sort of child-major candidates leaves them
-    float nlo[3] = {INFINITY, INFINITY, INFINITY}, nhi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    float3 cen[8];
-    for (int k = 0; k < nc; ++k) {
-        const float4 l = B.nlo[children[k]], h = B.nhi[children[k]];
-        nlo[0] = fminf(nlo[0], l.x); nlo[1] = fminf(nlo[1], l.y); nlo[2] = fminf(nlo[2], l.z);
-        nhi[0] = fmaxf(nhi[0], h.x); nhi[1] = fmaxf(nhi[1], h.y); nhi[2] = fmaxf(nhi[2], h.z);
-        cen[k] = make_float3(0.5f * (l.x + h.x), 0.5f * (l.y + h.y), 0.5f * (l.z + h.z));
-    }
-    const float pc[3] = {0.5f * (nlo[0] + nhi[0]), 0.5f * (nlo[1] + nhi[1]), 0.5f * (nlo[2] + nhi[2])};
-    int slot_child[8];
-    bool done[8] = {false, false, false, false, false, false, false, false};
-    for (int s = 0; s < 8; ++s) slot_child[s] = -1;
-    for (int round = 0; round < nc; ++round) {
-        float best = INFINITY;
-        int bc = -1, bs = -1;
-        for (int k = 0; k < nc; ++k) {
-            if (done[k]) continue;
-            const float off[3] = {cen[k].x - pc[0], cen[k].y - pc[1], cen[k].z - pc[2]};
-            for (int s = 0; s < 8; ++s) {
-                if (slot_child[s] >= 0) continue;
-                const float d = (s & 4 ? off[0] : -off[0]) + (s & 2 ? off[1] : -off[1]) + (s & 1 ? off[2] : -off[2]);
-                const float cost = -d;
-                if (cost < best) { best = cost; bc = k; bs = s; }
-            }
-        }
-        if (bc < 0) break;
-        slot_child[bs] = children[bc];
-        done[bc] = true;
-    }
-    // A node's leaf children hold 32 records at most (the traversal's record mask).  With leaves of more than
-    // 4 triangles eight of them can hold more: the largest leaf (the lowest slot among equals) then becomes an
-    // internal child, a node of its own one level down whose single slot is that leaf, until the rest fit.
-    // Such a demoted leaf is stored as -(child + 2) in the slot table.
-    uint32_t nt = 0;
-    for (int s = 0; s < 8; ++s)
-        if (slot_child[s] >= 0 && is_leaf(B, slot_child[s])) nt += B.nrange[slot_child[s]].y;
-    while (nt > kMaxNodeRecords) {
-        int big = -1;
-        for (int s = 0; s < 8; ++s)
-            if (slot_child[s] >= 0 && is_leaf(B, slot_child[s]) &&
-                (big < 0 || B.nrange[slot_child[s]].y > B.nrange[slot_child[big]].y))
-                big = s;
-        nt -= B.nrange[slot_child[big]].y;
-        slot_child[big] = -(slot_child[big] + 2);
-    }
-    uint32_t ni = 0;
-    for (int s = 0; s < 8; ++s) {
-        C.slots[size_t(i) * 8 + s] = slot_child[s];
-        if (slot_child[s] <= -2 || (slot_child[s] >= 0 && !is_leaf(B, slot_child[s]))) ++ni;
-    }
-    C.cnt_int[i] = ni;
-    C.cnt_tri[i] = nt;
+__device__ __forceinline__ void write_node(const Build& B, uint32_t slot, const float* v, uint32_t left, uint32_t right,
+                                           uint32_t first, uint32_t leaf_count) {
+    B.nlo[slot] = make_float4(v[0], v[1], v[2], __uint_as_float(left));
+    B.nhi[slot] = make_float4(v[3], v[4], v[5], __uint_as_float(right));
+    B.nrange[slot] = make_uint2(first, leaf_count);
 }
 
-// Outward 8-bit quantisation of the child boxes on one axis (the host builder's rule, in double precision).
-__device__ void quantise_axis(int a, float nlo, float nhi, const float* clo, const float* chi, const bool* present,
-                              WideNode& node) {
+__device__ __forceinline__ void add_part(SmallShared& S, int next, uint32_t first, uint32_t count, uint32_t depth,
+                                         uint32_t slot) {
+    if (count < 2) return;  // single triangles became leaves as they were partitioned
+    const int kind = count > 16 ? 0 : (count > 8 ? 1 : 2);
+    const uint32_t q = atomicAdd(&S.counts[next][kind], 1u);
+    uint2* list = kind == 0 ? S.big[next] : (kind == 1 ? S.mid[next] : S.tiny[next]);
+    list[q] = pack_part(first, count, depth, slot);
+}
+
+// A part of more than 16 triangles by one warp: binned SAH, stable partition.
+__device__ void split_big(const Build& B, SmallShared& S, int* bins, int next, uint2 part, uint32_t global_first) {
+    const uint32_t first = part.x & 1023u, count = (part.x >> 10) & 2047u, depth = part.x >> 21, slot = part.y;
+    const uint32_t lane = threadIdx.x & 31u;
+    float v[12];
+    for (int k = 0; k < 12; ++k) v[k] = (k % 6) < 3 ? INFINITY : -INFINITY;
+    for (uint32_t i = lane; i < count; i += 32) {
+        const uint32_t p = S.order[0][first + i];
+        for (int a = 0; a < 3; ++a) {
+            const float l = S.box[a][p], h = S.box[3 + a][p], c = 0.5f * (l + h);
+            v[a] = fminf(v[a], l);
+            v[3 + a] = fmaxf(v[3 + a], h);
+            v[6 + a] = fminf(v[6 + a], c);
+            v[9 + a] = fmaxf(v[9 + a], c);
+        }
+    }
+    for (int k = 0; k < 12; ++k) {
+        const int o = f2o(v[k]);
+        v[k] = o2f((k % 6) < 3 ? __reduce_min_sync(0xffffffffu, o) : __reduce_max_sync(0xffffffffu, o));
+    }
+    int axis = 0;
+    for (int a = 1; a < 3; ++a)
+        if (v[9 + a] - v[6 + a] > v[9 + axis] - v[6 + axis]) axis = a;
+    const bool degenerate = !(v[9 + axis] > v[6 + axis]);
+    uint32_t nl = count / 2, bin = 0;
+    bool by_position = true;
+    if (!degenerate && int(depth) < kMedianDepthD) {
+        clear_bins(bins, int(lane), 32);
+        __syncwarp();
+        float kk[3];
+        for (int a = 0; a < 3; ++a) kk[a] = bin_scale(v[9 + a] - v[6 + a]);
+        for (uint32_t i = lane; i < count; i += 32) {
+            const uint32_t p = S.order[0][first + i];
+            bin_prim(bins, make_float4(S.box[0][p], S.box[1][p], S.box[2][p], 0.0f),
+                     make_float4(S.box[3][p], S.box[4][p], S.box[5][p], 0.0f), v + 6, kk);
+        }
+        __syncwarp();
+        float cost;
+        const int a = best_bin_split(bins, v + 6, v + 9, int(lane), bin, nl, cost);
+        if (a >= 0 && nl > 0 && nl < count) {
+            axis = a;
+            by_position = false;
+        }
+        __syncwarp();
+    }
+    if (by_position) nl = count / 2;
+    const float lo = v[6 + axis], k = bin_scale(v[9 + axis] - v[6 + axis]);
+    const uint32_t left = slot + 1, right = slot + 2 * nl, below = (1u << lane) - 1u;
+    uint32_t lcount = 0, rcount = 0;
+    for (uint32_t base = 0; base < count; base += 32) {
+        const uint32_t i = base + lane;
+        uint32_t p = 0;
+        bool go = false;
+        if (i < count) {
+            p = S.order[0][first + i];
+            go = by_position ? i < nl : bin_of(0.5f * (S.box[axis][p] + S.box[3 + axis][p]), lo, k) <= int(bin);
+        }
+        const uint32_t lm = __ballot_sync(0xffffffffu, i < count && go), rm = __ballot_sync(0xffffffffu, i < count && !go);
+        if (i < count) {
+            S.order[1][go ? first + lcount + __popc(lm & below) : first + nl + rcount + __popc(rm & below)] = uint16_t(p);
+            if ((go ? nl : count - nl) == 1) {  // a leaf of one triangle
+                const float b[6] = {S.box[0][p], S.box[1][p], S.box[2][p], S.box[3][p], S.box[4][p], S.box[5][p]};
+                write_node(B, go ? left : right, b, ~0u, ~0u, global_first + (go ? first : first + nl), 1);
+            }
+        }
+        lcount += __popc(lm);
+        rcount += __popc(rm);
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < count; i += 32) S.order[0][first + i] = S.order[1][first + i];
+    if (lane == 0) {
+        write_node(B, slot, v, left, right, global_first + first, 0);
+        add_part(S, next, first, nl, depth + 1, left);
+        add_part(S, next, first + nl, count - nl, depth + 1, right);
+    }
+}
+
+// A part of at most G triangles by G lanes (an aligned group): exact SAH over every centroid plane of every axis,
+// lane i's candidates being the planes through its triangle's centroid.
+template <int G>
+__device__ void split_group(const Build& B, SmallShared& S, int next, uint2 part, uint32_t global_first) {
+    const uint32_t lane = threadIdx.x & 31u, gl = lane & uint32_t(G - 1), g0 = lane & ~uint32_t(G - 1);
+    const uint32_t mask = (G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u)) << g0;
+    const uint32_t first = part.x & 1023u, count = (part.x >> 10) & 2047u, depth = part.x >> 21, slot = part.y;
+    const bool mine = gl < count;
+    const uint32_t p = mine ? S.order[0][first + gl] : 0u;
+    float b[6];  // this lane's box; lanes past the part repeat nothing
+    for (int k = 0; k < 6; ++k) b[k] = mine ? S.box[k][p] : (k < 3 ? INFINITY : -INFINITY);
+    const float c[3] = {0.5f * (b[0] + b[3]), 0.5f * (b[1] + b[4]), 0.5f * (b[2] + b[5])};
+    float llo[3][3], lhi[3][3], rlo[3][3], rhi[3][3];  // per candidate axis: left and right boxes
+    uint32_t nleft[3] = {0, 0, 0};
+    float v[6];
+    for (int a = 0; a < 3; ++a)
+        for (int q = 0; q < 3; ++q) {
+            llo[a][q] = rlo[a][q] = INFINITY;
+            lhi[a][q] = rhi[a][q] = -INFINITY;
+        }
+    for (int q = 0; q < 3; ++q) {
+        v[q] = INFINITY;
+        v[3 + q] = -INFINITY;
+    }
+    for (uint32_t j = 0; j < count; ++j) {
+        float o[6];
+        for (int k = 0; k < 6; ++k) o[k] = __shfl_sync(mask, b[k], int(g0 + j));
+        for (int q = 0; q < 3; ++q) {
+            v[q] = fminf(v[q], o[q]);
+            v[3 + q] = fmaxf(v[3 + q], o[3 + q]);
+        }
+        for (int a = 0; a < 3; ++a) {
+            const bool l = 0.5f * (o[a] + o[3 + a]) <= c[a];
+            nleft[a] += l;
+            for (int q = 0; q < 3; ++q) {
+                llo[a][q] = fminf(llo[a][q], l ? o[q] : INFINITY);
+                lhi[a][q] = fmaxf(lhi[a][q], l ? o[3 + q] : -INFINITY);
+                rlo[a][q] = fminf(rlo[a][q], l ? INFINITY : o[q]);
+                rhi[a][q] = fmaxf(rhi[a][q], l ? -INFINITY : o[3 + q]);
+            }
+        }
+    }
+    float cost = INFINITY;
+    int axis = -1;
+    for (int a = 0; a < 3; ++a) {
+        if (!mine || nleft[a] >= count) continue;
+        const float la = box_area(make_float3(llo[a][0], llo[a][1], llo[a][2]), make_float3(lhi[a][0], lhi[a][1], lhi[a][2]));
+        const float ra = box_area(make_float3(rlo[a][0], rlo[a][1], rlo[a][2]), make_float3(rhi[a][0], rhi[a][1], rhi[a][2]));
+        const float x = la * float(nleft[a]) + ra * float(count - nleft[a]);
+        if (x < cost) {
+            cost = x;
+            axis = a;
+        }
+    }
+    const int key = f2o(cost);
+    const int least = __reduce_min_sync(mask, key);
+    const uint32_t win = __ffs(__ballot_sync(mask, key == least)) - 1;
+    axis = __shfl_sync(mask, axis, int(win));
+    const float plane = axis < 0 ? 0.0f : (axis == 0 ? c[0] : (axis == 1 ? c[1] : c[2]));
+    const float threshold = __shfl_sync(mask, plane, int(win));
+    const float best = o2f(least);
+    const float area = box_area(make_float3(v[0], v[1], v[2]), make_float3(v[3], v[4], v[5]));
+    const bool median = axis < 0 || int(depth) >= kMedianDepthD;
+    const bool leaf = count <= B.max_leaf && (median || area + best >= area * float(count));
+    if (leaf) {
+        if (gl == 0) write_node(B, slot, v, ~0u, ~0u, global_first + first, count);
+        return;
+    }
+    bool go = gl < count / 2;
+    if (!median) go = (axis == 0 ? c[0] : (axis == 1 ? c[1] : c[2])) <= threshold;
+    const uint32_t lm = (__ballot_sync(mask, mine && go) >> g0), rm = (__ballot_sync(mask, mine && !go) >> g0);
+    const uint32_t nl = __popc(lm), below = (1u << gl) - 1u;
+    const uint32_t left = slot + 1, right = slot + 2 * nl;
+    if (mine) {
+        S.order[0][go ? first + __popc(lm & below) : first + nl + __popc(rm & below)] = uint16_t(p);
+        if ((go ? nl : count - nl) == 1)
+            write_node(B, go ? left : right, b, ~0u, ~0u, global_first + (go ? first : first + nl), 1);
+    }
+    if (gl == 0) {
+        write_node(B, slot, v, left, right, global_first + first, 0);
+        add_part(S, next, first, nl, depth + 1, left);
+        add_part(S, next, first + nl, count - nl, depth + 1, right);
+    }
+}
+
+__global__ void __launch_bounds__(32 * kSmallWarps, 2) k_small(Build B) {
+    extern __shared__ __align__(16) unsigned char small_shared[];
+    SmallShared& S = *reinterpret_cast<SmallShared*>(small_shared);
+    if (B.ctr->err) return;
+    const uint32_t ntasks = B.ctr->small;
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    for (uint32_t task = blockIdx.x; task < ntasks; task += gridDim.x) {
+        const uint4 t = B.small[task];
+        const uint32_t first = t.x, count = t.y;
+        const int buffer = int(t.w >> 31);
+        for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) {
+            const float4 l = B.lo[buffer][first + i], h = B.hi[buffer][first + i];
+            S.box[0][i] = l.x; S.box[1][i] = l.y; S.box[2][i] = l.z;
+            S.box[3][i] = h.x; S.box[4][i] = h.y; S.box[5][i] = h.z;
+            S.tri[i] = __float_as_uint(l.w);
+            S.order[0][i] = uint16_t(i);
+        }
+        if (threadIdx.x < 6) S.counts[threadIdx.x / 3][threadIdx.x % 3] = 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (count == 1) {
+                const float b[6] = {S.box[0][0], S.box[1][0], S.box[2][0], S.box[3][0], S.box[4][0], S.box[5][0]};
+                write_node(B, t.z, b, ~0u, ~0u, first, 1);
+            }
+            add_part(S, 0, 0, count, t.w & 0x7fffffffu, t.z);
+        }
+        __syncthreads();
+        for (int cur = 0;; cur ^= 1) {
+            const uint32_t nb = S.counts[cur][0], nm = S.counts[cur][1], nt = S.counts[cur][2];
+            if (nb + nm + nt == 0) break;
+            for (uint32_t k = w; k < nb; k += kSmallWarps) split_big(B, S, S.bins[w], cur ^ 1, S.big[cur][k], first);
+            for (uint32_t k = 2 * w; k < nm; k += 2 * kSmallWarps)
+                if (k + (lane >> 4) < nm) split_group<16>(B, S, cur ^ 1, S.mid[cur][k + (lane >> 4)], first);
+            for (uint32_t k = 4 * w; k < nt; k += 4 * kSmallWarps)
+                if (k + (lane >> 3) < nt) split_group<8>(B, S, cur ^ 1, S.tiny[cur][k + (lane >> 3)], first);
+            __syncthreads();
+            if (threadIdx.x < 3) S.counts[cur][threadIdx.x] = 0;
+            __syncthreads();
+        }
+        for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) B.idx[first + i] = S.tri[S.order[0][i]];
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------
+// 4. Collapse to 8-wide nodes and quantisation, one level at a time, eight lanes per node.
+// ---------------------------------------------------------------------------------------------------
+struct Collapse {
+    int* binary;        // binary node of each 8-wide node; -(node + 2): a demoted leaf, alone in a node of its own
+    WideNode* nodes;
+    float4* tris;
+    uint32_t max_wide;
+};
+
+// Outward 8-bit quantisation of the child boxes on one axis (the host builder's rule, in double precision), lane s
+// the child in slot s: the node's origin and exponent, this child's planes.
+__device__ __forceinline__ void quantise_axis(uint32_t mask, bool present, float clo, float chi, float& origin, int& exponent,
+                                              uint32_t& qlo, uint32_t& qhi) {
+    const float nlo = o2f(__reduce_min_sync(mask, f2o(present ? clo : INFINITY)));
+    const float nhi = o2f(__reduce_max_sync(mask, f2o(present ? chi : -INFINITY)));
     const double ext = double(nhi) - double(nlo);
     const double mag = fmax(fabs(double(nlo)), fabs(double(nhi)));
-    const double min_q = fmax(ldexp(mag, -20), ldexp(1.0, -60));
-    int e;
-    frexp(fmax(ext / 250.0, min_q), &e);
+    const double min_q = fmax(mag * (1.0 / 1048576.0), ldexp(1.0, -60));
+    const double least = fmax(ext / 250.0, min_q);
+    // 2^e >= least: the exponent frexp returns for a positive normal number
+    int e = int((__double2hiint(least) >> 20) & 0x7ff) - 1022;
     for (int guard = 0; guard < 2100; ++guard, ++e) {
-        const double scale = ldexp(1.0, e);
+        const double scale = __hiloint2double((e + 1023) << 20, 0), inv = __hiloint2double((1023 - e) << 20, 0);
         float p = float(double(nlo) - scale);
         if (double(p) > double(nlo) - scale) p = nextafterf(p, -INFINITY);
         bool ok = true;
-        for (int s = 0; s < 8; ++s) {
-            if (!present[s]) {
-                node.qlo[a][s] = 255;
-                node.qhi[a][s] = 0;
-                continue;
-            }
-            double lo = floor((double(clo[s]) - p) / scale) - 1.0;
-            double hi = ceil((double(chi[s]) - p) / scale) + 1.0;
-            while (lo > 0.0 && double(p) + lo * scale > double(clo[s]) - 0.5 * scale) lo -= 1.0;
-            while (double(p) + hi * scale < double(chi[s]) + 0.5 * scale) hi += 1.0;
-            if (lo < 0.0 || hi > 255.0 || double(p) + lo * scale > double(clo[s]) - 0.5 * scale) {
-                ok = false;
-                break;
-            }
-            node.qlo[a][s] = uint8_t(lo);
-            node.qhi[a][s] = uint8_t(hi);
+        double lo = 255.0, hi = 0.0;
+        if (present) {
+            lo = floor((double(clo) - p) * inv) - 1.0;
+            hi = ceil((double(chi) - p) * inv) + 1.0;
+            while (lo > 0.0 && double(p) + lo * scale > double(clo) - 0.5 * scale) lo -= 1.0;
+            while (double(p) + hi * scale < double(chi) + 0.5 * scale) hi += 1.0;
+            ok = !(lo < 0.0 || hi > 255.0 || double(p) + lo * scale > double(clo) - 0.5 * scale);
         }
-        if (ok) {
-            node.p[a] = p;
-            node.e[a] = uint8_t(e + 127);
+        if (__all_sync(mask, ok)) {
+            origin = p;
+            exponent = e;
+            qlo = uint32_t(lo);
+            qhi = uint32_t(hi);
             return;
         }
     }
+    origin = nlo;
+    exponent = 127;
+    qlo = present ? 0u : 255u;
+    qhi = present ? 255u : 0u;
 }
 
-__global__ void __launch_bounds__(128) k_collapse_emit(Build B, Collapse C, uint32_t count, uint32_t next_base,
-                                                       uint32_t tri_base) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    int slot_child[8];
-    bool present[8];
-    float lo[3][8], hi[3][8];
-    float nlo[3] = {INFINITY, INFINITY, INFINITY}, nhi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    bool demoted[8];
-    for (int s = 0; s < 8; ++s) {
-        slot_child[s] = C.slots[size_t(i) * 8 + s];
-        demoted[s] = slot_child[s] <= -2;
-        if (demoted[s]) slot_child[s] = -slot_child[s] - 2;
-        present[s] = slot_child[s] >= 0;
-        if (!present[s]) continue;
-        const float4 l = B.nlo[slot_child[s]], h = B.nhi[slot_child[s]];
-        lo[0][s] = l.x; lo[1][s] = l.y; lo[2][s] = l.z;
-        hi[0][s] = h.x; hi[1][s] = h.y; hi[2][s] = h.z;
-        for (int a = 0; a < 3; ++a) { nlo[a] = fminf(nlo[a], lo[a][s]); nhi[a] = fmaxf(nhi[a], hi[a][s]); }
+// One 8-wide node by an aligned group of eight lanes, lane k first a child, then a slot.
+__device__ void collapse_node(const Build& B, const Collapse& C, uint32_t wide) {
+    const uint32_t lane = threadIdx.x & 31u, k = lane & 7u, g0 = lane & 24u, mask = 0xffu << g0;
+    const int entry = C.binary[wide];
+    const int root = entry <= -2 ? -entry - 2 : entry;
+    // children: the root's two (or the root itself, a leaf), then the largest internal one opened until there are 8
+    int child = -1;
+    float4 l = make_float4(0, 0, 0, 0), h = l;
+    uint2 range = make_uint2(0, 0);
+    auto load = [&](int node) {
+        child = node;
+        l = B.nlo[node];
+        h = B.nhi[node];
+        range = B.nrange[node];
+    };
+    auto open_key = [&]() -> int {  // area of an internal child as an ordered int; -1: not to be opened
+        return child >= 0 && range.y == 0
+                   ? __float_as_int(fmaxf(box_area(make_float3(l.x, l.y, l.z), make_float3(h.x, h.y, h.z)), 0.0f))
+                   : -1;
+    };
+    uint32_t nc = 1;
+    if (k == 0) load(root);
+    for (;;) {
+        const int key = open_key();
+        const int most = __reduce_max_sync(mask, key);
+        if (most < 0 || nc >= 8 || (entry <= -2)) break;
+        const uint32_t w = __ffs(__ballot_sync(mask, key == most)) - 1;
+        const int left = __shfl_sync(mask, int(__float_as_uint(l.w)), int(w));
+        const int right = __shfl_sync(mask, int(__float_as_uint(h.w)), int(w));
+        if (lane == w) load(left);
+        if (k == nc) load(right);
+        ++nc;
     }
-    WideNode node;
-    memset(&node, 0, sizeof(node));
-    memset(node.meta, int(kLeafNone), sizeof(node.meta));
-    for (int a = 0; a < 3; ++a) quantise_axis(a, nlo[a], nhi[a], lo[a], hi[a], present, node);
-    node.child_base = next_base + C.off_int[i];
-    node.tri_base = tri_base + C.off_tri[i];
-    uint32_t ni = 0, offset = 0;
-    for (int s = 0; s < 8; ++s) {
-        const int c = slot_child[s];
-        if (c < 0) continue;
-        if (demoted[s] || !is_leaf(B, c)) {
-            node.imask |= uint8_t(1u << s);
-            C.next[C.off_int[i] + ni] = make_uint2(node.child_base + ni, uint32_t(c));
-            ++ni;
-            continue;
-        }
-        const uint2 r = B.nrange[c];
-        node.meta[s] = uint8_t(((r.y - 1u) << 5) | offset);
-        for (uint32_t k = 0; k < r.y; ++k) {
-            const uint32_t tri = __float_as_uint(B.plo[B.idx[r.x + k]].w);
-            const float4* src = B.soup + size_t(tri) * 3;
-            float4* dst = reinterpret_cast<float4*>(C.tris + node.tri_base + offset + k);
-            dst[0] = src[0];
-            dst[1] = src[1];
-            dst[2] = src[2];
-        }
-        offset += r.y;
+    // slots by octant direction (the host builder's rule): the cheapest (child, slot) pair of those left, ties in
+    // (child, slot) order
+    const bool real = child >= 0;
+    const float blo[3] = {l.x, l.y, l.z}, bhi[3] = {h.x, h.y, h.z};
+    float off[3];
+    for (int a = 0; a < 3; ++a) {
+        const float nlo = o2f(__reduce_min_sync(mask, f2o(real ? blo[a] : INFINITY)));
+        const float nhi = o2f(__reduce_max_sync(mask, f2o(real ? bhi[a] : -INFINITY)));
+        off[a] = 0.5f * (blo[a] + bhi[a]) - 0.5f * (nlo + nhi);
     }
-    C.nodes[C.level[i].x] = node;
+    uint32_t taken = 0, my_slot = 0xffu;
+    for (uint32_t round = 0; round < nc; ++round) {
+        float best = INFINITY;
+        uint32_t bs = 8;
+        if (real && my_slot == 0xffu)
+            for (uint32_t s = 0; s < 8; ++s) {
+                if ((taken >> s) & 1u) continue;
+                const float d = (s & 4u ? off[0] : -off[0]) + (s & 2u ? off[1] : -off[1]) + (s & 1u ? off[2] : -off[2]);
+                if (-d < best) {
+                    best = -d;
+                    bs = s;
+                }
+            }
+        const int key = f2o(__fadd_rn(best, 0.0f));
+        const int least = __reduce_min_sync(mask, key);
+        const uint32_t who = __ballot_sync(mask, bs < 8 && key == least);
+        if (!who) break;
+        const uint32_t w = __ffs(who) - 1;
+        const uint32_t s = __shfl_sync(mask, bs, int(w));
+        if (lane == w) my_slot = s;
+        taken |= 1u << s;
+    }
+    // lane s takes the child of slot s
+    uint32_t from = 0xffu;
+    for (uint32_t j = 0; j < 8; ++j)
+        if (__shfl_sync(mask, my_slot, int(g0 + j)) == k) from = j;
+    const int src = int(g0 + (from < 8 ? from : 0u));
+    const int sc = __shfl_sync(mask, child, src);
+    const uint32_t rx = __shfl_sync(mask, range.x, src), ry = __shfl_sync(mask, range.y, src);
+    float slo[3], shi[3];
+    for (int a = 0; a < 3; ++a) {
+        slo[a] = __shfl_sync(mask, blo[a], src);
+        shi[a] = __shfl_sync(mask, bhi[a], src);
+    }
+    const bool present = from < 8;
+    bool leaf = present && ry > 0;
+    // A node's leaf children hold 32 records at most (the traversal's record mask).  With leaves of more than
+    // 4 triangles eight of them can hold more: the largest leaf (the lowest slot among equals) then becomes an
+    // internal child, a node of its own one level down whose single slot is that leaf, until the rest fit.
+    bool demoted = false;
+    for (int guard = 0; guard < 8; ++guard) {
+        const uint32_t total = __reduce_add_sync(mask, leaf ? ry : 0u);
+        if (total <= kMaxNodeRecords) break;
+        const uint32_t big = __reduce_max_sync(mask, leaf ? ry : 0u);
+        const uint32_t w = __ffs(__ballot_sync(mask, leaf && ry == big)) - 1;
+        if (lane == w) {
+            leaf = false;
+            demoted = true;
+        }
+    }
+    const bool inner = present && !leaf;
+    const uint32_t inner_mask = (__ballot_sync(mask, inner) >> g0) & 0xffu;
+    // records of the leaf slots, in slot order
+    uint32_t incl = leaf ? ry : 0u;
+    for (int o = 1; o < 8; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(mask, incl, o, 8);
+        if (int(k) >= o) incl += x;
+    }
+    const uint32_t records = __shfl_sync(mask, incl, int(g0 + 7u)), offset = incl - (leaf ? ry : 0u);
+    uint32_t child_base = 0, tri_base = 0;
+    if (k == 0) {
+        child_base = atomicAdd(&B.ctr->wide, __popc(inner_mask));
+        tri_base = atomicAdd(&B.ctr->tris, records);
+    }
+    child_base = __shfl_sync(mask, child_base, int(g0));
+    tri_base = __shfl_sync(mask, tri_base, int(g0));
+    unsigned char* node = reinterpret_cast<unsigned char*>(C.nodes + wide);
+    for (int a = 0; a < 3; ++a) {
+        float p;
+        int e;
+        uint32_t qlo, qhi;
+        quantise_axis(mask, present, slo[a], shi[a], p, e, qlo, qhi);
+        if (k == 0) {
+            reinterpret_cast<float*>(node)[a] = p;
+            node[12 + a] = uint8_t(e + 127);
+        }
+        node[32 + 8 * a + k] = uint8_t(qlo);
+        node[56 + 8 * a + k] = uint8_t(qhi);
+    }
+    if (k == 0) {
+        node[15] = uint8_t(inner_mask);
+        reinterpret_cast<uint32_t*>(node)[4] = child_base;
+        reinterpret_cast<uint32_t*>(node)[5] = tri_base;
+    }
+    node[24 + k] = uint8_t(leaf ? ((ry - 1u) << 5) | offset : kLeafNone);
+    if (inner) {
+        const uint32_t at = child_base + __popc(inner_mask & ((1u << k) - 1u));
+        if (at < C.max_wide) C.binary[at] = demoted ? -(sc + 2) : sc;
+    }
+    if (leaf)
+        for (uint32_t j = 0; j < ry; ++j) {
+            const uint32_t at = tri_base + offset + j;
+            if (at >= B.n) break;  // reported as lost triangles
+            const float4* rec = B.soup + size_t(B.idx[rx + j]) * 3;
+            float4* dst = C.tris + size_t(at) * 3;
+            dst[0] = rec[0];
+            dst[1] = rec[1];
+            dst[2] = rec[2];
+        }
 }
 
-template <typename T>
-cudaError_t dalloc(T*& p, size_t count) {
-    return cudaMalloc(reinterpret_cast<void**>(&p), sizeof(T) * (count ? count : 1));
+__global__ void __launch_bounds__(256, 2) k_collapse(Build B, Collapse C) {
+    if (B.ctr->err) return;  // set before this launch, or by the last level of it
+    cg::grid_group grid = cg::this_grid();
+    const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, groups = (gridDim.x * blockDim.x) >> 3;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        C.binary[0] = 0;
+        B.ctr->wide = 1;
+        B.ctr->tris = 0;
+    }
+    grid.sync();
+    uint32_t begin = 0;
+    for (uint32_t level = 1;; ++level) {
+        const uint32_t end = min(*(volatile uint32_t*)&B.ctr->wide, C.max_wide);
+        if (begin >= end) break;
+        if (level > uint32_t(kWideStack)) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&B.ctr->err, kErrTooDeep);
+            break;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) B.ctr->levels = level;
+        grid.sync();  // every thread has read the level's end
+        for (uint32_t i = begin + group; i < end; i += groups) collapse_node(B, C, i);
+        begin = end;
+        grid.sync();
+    }
 }
 
 }  // namespace
 
 std::string build_wide_device(const std::vector<MeshInput>& meshes, uint32_t max_leaf, DeviceBuild& out) {
     if (max_leaf < 1 || max_leaf > kMaxLeafLimit) return "leaf size must lie in 1..8";
-    std::vector<TriRecord> soup;
-    size_t total = 0;
-    for (const MeshInput& m : meshes) total += m.indices.size() / 3;
+    size_t total = 0, vertex_total = 0;
+    for (const MeshInput& m : meshes) {
+        total += m.indices.size() / 3;
+        vertex_total += m.vertices.size();
+    }
     if (total == 0) return "scene has no triangles";
     if (total > (size_t(1) << 30)) return "too many triangles";
-    soup.reserve(total);
-    for (const MeshInput& m : meshes) {
-        const size_t nv = m.vertices.size() / 3;
-        const size_t nt = m.indices.size() / 3;
-        for (size_t t = 0; t < nt; ++t) {
-            TriRecord r;
-            float* dst[3] = {r.v0, r.v1, r.v2};
-            for (int k = 0; k < 3; ++k) {
-                const uint32_t vi = m.indices[3 * t + k];
-                if (vi >= nv) return "triangle index out of range";
-                std::memcpy(dst[k], &m.vertices[3 * size_t(vi)], 12);
-                for (int a = 0; a < 3; ++a)
-                    if (!std::isfinite(dst[k][a])) return "non-finite vertex";
-            }
-            r.prim = uint32_t(t);
-            r.geom = m.geomID;
-            r.kind = m.quads ? kTriQuadHalf : (m.curves ? kTriCurve : kTriPlain);
-            soup.push_back(r);
-        }
-    }
     const uint32_t n = uint32_t(total);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaStream_t s = nullptr;
-    cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
     const auto t0 = std::chrono::steady_clock::now();
 
-    Build B;
-    std::memset(&B, 0, sizeof(B));
-    B.n = n;
-    B.max_leaf = max_leaf;
-    const uint32_t max_large = n / kSmall + 2;
-    const size_t max_nodes = 2 * size_t(n);
-    std::vector<void*> owned;
-    cudaError_t e = cudaSuccess;
-    auto take = [&](auto*& p, size_t count) {
-        if (e == cudaSuccess) e = dalloc(p, count);
-        if (e == cudaSuccess) owned.push_back(static_cast<void*>(p));
-    };
-    float4* soup_d = nullptr;
-    take(soup_d, size_t(n) * 3);
-    B.soup = soup_d;
-    take(B.plo, n);
-    take(B.phi, n);
-    take(B.idx, n);
-    take(B.idx_tmp, n);
-    take(B.nlo, max_nodes);
-    take(B.nhi, max_nodes);
-    take(B.nrange, max_nodes);
-    take(B.tasks[0], max_large);
-    take(B.tasks[1], max_large);
-    take(B.small, n);
-    take(B.tbox, size_t(max_large) * 12);
-    take(B.tbins, size_t(max_large) * 3 * kBinsD * 7);
-    take(B.tsplit, max_large);
-    take(B.tcursor, size_t(max_large) * 2);
-    take(B.counters, 16);
-    take(B.scene_box, 8);
-    uint32_t* h_counters = nullptr;
-    if (e == cudaSuccess) e = cudaMallocHost(&h_counters, 16 * sizeof(uint32_t));
-    auto cleanup = [&]() {
-        for (void* p : owned) cudaFree(p);
-        if (h_counters) cudaFreeHost(h_counters);
-        cudaStreamDestroy(s);
-    };
-    if (e != cudaSuccess) {
-        cleanup();
-        return std::string("device BVH build: ") + cudaGetErrorString(e);
-    }
-    e = cudaMemcpyAsync(soup_d, soup.data(), sizeof(TriRecord) * n, cudaMemcpyHostToDevice, s);
-    k_init_counters<<<1, 32, 0, s>>>(B);
-    k_prims<<<sms * 8, 256, 0, s>>>(B);
-    const auto read_counters = [&]() {
-        cudaMemcpyAsync(h_counters, B.counters, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        return cudaStreamSynchronize(s);
-    };
-    // root task
-    const uint4 root = make_uint4(0, n, 0, 0);
-    int cur = 0;
-    uint32_t ntasks = 0, max_count = 0;
-    if (n > kSmall) {
-        cudaMemcpyAsync(B.tasks[0], &root, sizeof(root), cudaMemcpyHostToDevice, s);
-        ntasks = 1;
-        max_count = n;
-    } else {
-        cudaMemcpyAsync(B.small, &root, sizeof(root), cudaMemcpyHostToDevice, s);
-        const uint32_t one = 1;
-        cudaMemcpyAsync(B.counters + 1, &one, sizeof(one), cudaMemcpyHostToDevice, s);
-    }
-    while (ntasks > 0 && e == cudaSuccess) {
-        if (ntasks > 65535) {  // one grid row per task
-            cleanup();
-            return "device BVH build: too many large tasks in one level (use the host builder)";
-        }
-        const dim3 grid((max_count + kChunk - 1) / kChunk, ntasks);
-        k_task_init<<<sms * 4, 256, 0, s>>>(B, cur, ntasks);
-        k_task_bounds<<<grid, 256, 0, s>>>(B, cur);
-        k_task_bin<<<grid, 256, 0, s>>>(B, cur);
-        cudaMemsetAsync(B.counters, 0, sizeof(uint32_t), s);      // next large tasks
-        cudaMemsetAsync(B.counters + 2, 0, sizeof(uint32_t), s);  // their largest count
-        k_task_split<<<(ntasks * 32 + 127) / 128, 128, 0, s>>>(B, cur, ntasks);
-        k_task_partition<<<grid, 256, 0, s>>>(B, cur);
-        k_task_copy_back<<<grid, 256, 0, s>>>(B, cur);
-        e = read_counters();
-        ntasks = h_counters[0];
-        max_count = h_counters[2];
-        cur ^= 1;
-    }
-    if (e == cudaSuccess) {
-        k_small<<<sms * 8, 32 * kSmallWarps, 0, s>>>(B);
-        e = read_counters();
-    }
-    if (e == cudaSuccess && h_counters[4]) e = cudaErrorUnknown;
-    const uint32_t binary_depth = h_counters[3];
-
-    // collapse, level by level
-    std::vector<uint32_t> level_sizes;
-    WideNode* nodes = nullptr;
-    TriRecord* tris = nullptr;
-    Collapse C;
-    std::memset(&C, 0, sizeof(C));
-    uint2 *lvl_a = nullptr, *lvl_b = nullptr;
-    uint32_t* scan_tmp = nullptr;
-    uint32_t *cnt_int = nullptr, *cnt_tri = nullptr, *off_int = nullptr, *off_tri = nullptr;
-    int* slots = nullptr;
     // 8-wide nodes: each has at least two slots except the single-leaf nodes of demoted leaves (at most one per
     // five triangles, as only a leaf of five or more is demoted), so at most n + n / 5 + 1 of them
-    const size_t max_wide = max_leaf > 4 ? n + n / 5 + 1 : n;
-    take(nodes, max_wide);
-    take(tris, n);
-    take(lvl_a, max_wide);
-    take(lvl_b, max_wide);
-    take(slots, max_wide * 8);
-    take(cnt_int, max_wide);
-    take(cnt_tri, max_wide);
-    take(off_int, max_wide + 1);
-    take(off_tri, max_wide + 1);
-    take(scan_tmp, scan_scratch_words(max_wide));
-    std::string err;
-    uint32_t node_count = 0, tri_count = 0, depth = 0;
-    if (e == cudaSuccess) {
-        const uint2 r = make_uint2(0, 0);
-        cudaMemcpyAsync(lvl_a, &r, sizeof(r), cudaMemcpyHostToDevice, s);
-        uint32_t count = 1, base = 0;
-        while (count > 0 && e == cudaSuccess) {
-            if (++depth > uint32_t(kWideStack)) {
-                err = "8-wide BVH deeper than the traversal stack";
-                break;
-            }
-            C.level = lvl_a;
-            C.next = lvl_b;
-            C.slots = slots;
-            C.cnt_int = cnt_int;
-            C.cnt_tri = cnt_tri;
-            C.off_int = off_int;
-            C.off_tri = off_tri;
-            C.nodes = nodes;
-            C.tris = tris;
-            k_collapse_gather<<<(count + 127) / 128, 128, 0, s>>>(B, C, count);
-            scan_exclusive(cnt_int, count, off_int, scan_tmp, s);
-            scan_exclusive(cnt_tri, count, off_tri, scan_tmp, s);
-            k_collapse_emit<<<(count + 127) / 128, 128, 0, s>>>(B, C, count, base + count, tri_count);
-            uint32_t totals[2] = {0, 0};
-            cudaMemcpyAsync(&totals[0], off_int + count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-            cudaMemcpyAsync(&totals[1], off_tri + count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-            e = cudaStreamSynchronize(s);
-            base += count;
-            tri_count += totals[1];
-            count = totals[0];
-            std::swap(lvl_a, lvl_b);
+    const size_t max_wide = max_leaf > 4 ? size_t(n) + n / 5 + 1 : n;
+    const size_t max_top = size_t(n) / kSmall + 2;         // subtrees of more than kSmall triangles in one level
+    const size_t max_chunks = size_t(n) / kChunk + max_top;
+    Build B;
+    Collapse C;
+    std::memset(&B, 0, sizeof(B));
+    std::memset(&C, 0, sizeof(C));
+    B.n = n;
+    B.max_leaf = max_leaf;
+    B.mesh_count = uint32_t(meshes.size());
+    C.max_wide = uint32_t(max_wide);
+    float* vertices = nullptr;
+    uint32_t* indices = nullptr;
+    MeshDev* mesh_table = nullptr;
+    // one scratch block for everything but the result: sized on the first walk, carved on the second
+    size_t scratch_bytes = 0;
+    char* scratch = nullptr;
+    for (int walk = 0; walk < 2; ++walk) {
+        size_t at = 0;
+        auto take = [&](auto*& p, size_t count) {
+            using T = std::remove_reference_t<decltype(*p)>;
+            if (walk) p = reinterpret_cast<T*>(scratch + at);
+            at += (sizeof(T) * std::max<size_t>(count, 1) + 255) & ~size_t(255);
+        };
+        take(B.ctr, 1);
+        take(mesh_table, meshes.size());
+        take(vertices, vertex_total);
+        take(indices, 3 * total);
+        take(B.soup, size_t(n) * 3);
+        for (int k = 0; k < 2; ++k) {
+            take(B.lo[k], n);
+            take(B.hi[k], n);
+            take(B.tasks[k], max_top);
+            take(B.chunk_task[k], max_chunks);
         }
-        node_count = base;
+        take(B.idx, n);
+        take(B.nlo, 2 * size_t(n));
+        take(B.nhi, 2 * size_t(n));
+        take(B.nrange, 2 * size_t(n));
+        take(B.bins, max_top * kBinWords);
+        take(B.small, size_t(n));
+        take(C.binary, max_wide);
+        take(C.nodes, max_wide);
+        if (!walk) {
+            scratch_bytes = at;
+            const cudaError_t e = cudaMalloc(&scratch, scratch_bytes);
+            if (e != cudaSuccess) return std::string("device BVH build: ") + cudaGetErrorString(e);
+        }
     }
-    if (e == cudaSuccess && err.empty() && tri_count != n) err = "device BVH build lost triangles";
-    if (e == cudaSuccess) e = cudaGetLastError();
-    int box[8] = {0};
+    B.meshes = mesh_table;
+    cudaStream_t s = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMalloc(&C.tris, sizeof(TriRecord) * size_t(n));
+
+    // the meshes' arrays: large ones are copied from where they lie, small ones gathered into one copy
+    constexpr size_t kDirectBytes = 64 * 1024;
+    std::vector<MeshDev> table;
+    std::vector<uint32_t> packed;  // small meshes: vertices (as bits) and indices, in the order of their places
+    size_t vat = 0, iat = 0;
+    uint32_t first = 0;
+    for (const MeshInput& m : meshes) {
+        MeshDev d;
+        d.vertices = vertices + vat;
+        d.indices = indices + iat;
+        d.first = first;
+        d.vertex_count = uint32_t(m.vertices.size() / 3);
+        d.geom = m.geomID;
+        d.kind = m.quads ? kTriQuadHalf : (m.curves ? kTriCurve : kTriPlain);
+        if (!m.indices.empty()) table.push_back(d);
+        vat += m.vertices.size();
+        iat += m.indices.size();
+        first += uint32_t(m.indices.size() / 3);
+    }
+    auto upload = [&](void* dst, auto array_of) {  // runs of small arrays together
+        char* run = static_cast<char*>(dst);
+        auto flush = [&]() {
+            if (!packed.empty() && e == cudaSuccess)
+                e = cudaMemcpyAsync(run, packed.data(), packed.size() * 4, cudaMemcpyHostToDevice, s);
+            if (!packed.empty() && e == cudaSuccess) e = cudaStreamSynchronize(s);  // packed is refilled
+            run += packed.size() * 4;
+            packed.clear();
+        };
+        for (const MeshInput& m : meshes) {
+            const auto& a = array_of(m);
+            const size_t bytes = a.size() * 4;
+            if (bytes < kDirectBytes) {
+                const uint32_t* w = reinterpret_cast<const uint32_t*>(a.data());
+                packed.insert(packed.end(), w, w + a.size());
+                continue;
+            }
+            flush();
+            if (e == cudaSuccess) e = cudaMemcpyAsync(run, a.data(), bytes, cudaMemcpyHostToDevice, s);
+            run += bytes;
+        }
+        flush();
+    };
+    upload(vertices, [](const MeshInput& m) -> const std::vector<float>& { return m.vertices; });
+    upload(indices, [](const MeshInput& m) -> const std::vector<uint32_t>& { return m.indices; });
+    B.mesh_count = uint32_t(table.size());
+    Counters ctr;
+    std::memset(&ctr, 0, sizeof(ctr));
+    for (int k = 0; k < 6; ++k) {
+        // +-infinity as ordered ints
+        ctr.box[k] = ctr.cbox[k] = k < 3 ? 0x7f800000 : int(0xff800000u ^ 0x7fffffffu);
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(mesh_table, table.data(), sizeof(MeshDev) * table.size(), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(B.ctr, &ctr, sizeof(ctr), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        cudaMemcpyAsync(box, B.scene_box, 6 * sizeof(int), cudaMemcpyDeviceToHost, s);
-        e = cudaStreamSynchronize(s);
+        const int records_grid = int(std::min<size_t>((size_t(n) + 255) / 256, size_t(sms) * 8));
+        k_records<<<records_grid, 256, 0, s>>>(B);
+        void* top_args[] = {&B};
+        void* collapse_args[] = {&B, &C};
+        // as many blocks as run at once, fewer for small scenes (a grid barrier costs less)
+        auto cooperative = [&](const void* kernel, size_t work, void** args) {
+            int per_sm = 0;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0);
+            const size_t most = size_t(sms) * size_t(std::max(per_sm, 1));
+            const unsigned blocks = unsigned(std::min(most, std::max<size_t>(work, 1)));
+            if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(256), args, 0, s);
+        };
+        if (n > kSmall) {
+            cooperative(reinterpret_cast<const void*>(&k_top), (size_t(n) + kChunk - 1) / kChunk, top_args);
+        } else {  // the scene is one small subtree
+            const uint4 root = make_uint4(0, n, 0, 0);
+            const uint32_t one = 1;
+            e = cudaMemcpyAsync(B.small, &root, sizeof(root), cudaMemcpyHostToDevice, s);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(&B.ctr->small, &one, sizeof(one), cudaMemcpyHostToDevice, s);
+        }
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SmallShared)));
+        if (e == cudaSuccess) {
+            const int small_grid = int(std::min<size_t>((size_t(n) + 63) / 64, size_t(sms) * 16));
+            k_small<<<small_grid, 32 * kSmallWarps, sizeof(SmallShared), s>>>(B);
+            e = cudaGetLastError();
+        }
+        if (e == cudaSuccess)
+            cooperative(reinterpret_cast<const void*>(&k_collapse), (size_t(n) + 127) / 128, collapse_args);
     }
-    const auto t1 = std::chrono::steady_clock::now();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&ctr, B.ctr, sizeof(ctr), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    std::string err;
+    if (e == cudaSuccess) {
+        if (ctr.err & kErrIndex) err = "triangle index out of range";
+        else if (ctr.err & kErrNonFinite) err = "non-finite vertex";
+        else if (ctr.err & kErrTooDeep) err = "8-wide BVH deeper than the traversal stack";
+        else if (ctr.tris != n || ctr.wide > max_wide) err = "device BVH build lost triangles";
+    }
+    WideNode* nodes = nullptr;
+    if (e == cudaSuccess && err.empty()) {
+        e = cudaMalloc(&nodes, sizeof(WideNode) * size_t(ctr.wide));
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(nodes, C.nodes, sizeof(WideNode) * size_t(ctr.wide), cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
+    if (s) cudaStreamDestroy(s);
+    cudaFree(scratch);
     if (e != cudaSuccess || !err.empty()) {
-        cleanup();
+        cudaGetLastError();
+        if (nodes) cudaFree(nodes);
+        if (C.tris) cudaFree(C.tris);
         return err.empty() ? std::string("device BVH build: ") + cudaGetErrorString(e) : err;
     }
-    // hand the node and triangle arrays to the caller, free the rest
+    const auto t1 = std::chrono::steady_clock::now();
     out.d_nodes = nodes;
-    out.d_tris = tris;
-    for (void* p : owned)
-        if (p != nodes && p != tris) cudaFree(p);
-    cudaFreeHost(h_counters);
-    cudaStreamDestroy(s);
+    out.d_tris = C.tris;
     auto o2f_host = [](int i) {
         const int b = i >= 0 ? i : i ^ 0x7fffffff;
         float f;
@@ -943,13 +1132,12 @@ std::string build_wide_device(const std::vector<MeshInput>& meshes, uint32_t max
         return f;
     };
     for (int a = 0; a < 3; ++a) {
-        out.lo[a] = o2f_host(box[a]);
-        out.hi[a] = o2f_host(box[3 + a]);
+        out.lo[a] = o2f_host(ctr.box[a]);
+        out.hi[a] = o2f_host(ctr.box[3 + a]);
     }
-    out.node_count = node_count;
-    out.tri_count = tri_count;
-    out.max_depth = depth;
-    out.binary_depth = binary_depth;
+    out.node_count = ctr.wide;
+    out.tri_count = n;
+    out.max_depth = ctr.levels;
     out.build_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
     return "";
 }

@@ -94,7 +94,7 @@ std::string build_bvh(const std::vector<MeshInput>& meshes, int kind, BuiltBvh& 
 struct DeviceBuild {
     void* d_nodes = nullptr;  // WideNode[node_count]
     void* d_tris = nullptr;   // TriRecord[tri_count], leaf order
-    uint32_t node_count = 0, tri_count = 0, max_depth = 0, binary_depth = 0;
+    uint32_t node_count = 0, tri_count = 0, max_depth = 0;
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
     double build_ms = 0.0;    // upload of the triangles + all build kernels
 };
