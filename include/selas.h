@@ -115,11 +115,12 @@ enum {
                                      the batch's neighbouring rays run nearly parallel; 0 (default): queue
                                      and record order */
     SEL_OPTION_ZERO_COPY = 4      /* 1 (default): the host-memory queries (sel_intersect1M etc.) trace records
-                                     that lie in page-locked host memory the GPU can address (cudaHostAlloc /
-                                     cudaHostRegister) in place, the kernel reading rays and writing hits over
-                                     the host link, except batches of more than 524,288 records whose rays
-                                     run nearly parallel record to record (camera rays: their traversal is
-                                     too short to hide the link, so full-duplex staged copies are faster);
+                                     that lie in host memory the GPU can address (page-locked memory; any host
+                                     memory where the GPU walks the host's page tables) in place, the kernel
+                                     reading rays and writing hits over the host link, except closest-hit
+                                     batches of more than 2,097,152 page-locked records whose rays run nearly
+                                     parallel record to record (camera rays: their traversal is too short to
+                                     hide the link, so full-duplex staged copies are faster);
                                      0: always stage them through HBM with pipelined copies */
 };
 int sel_device_set_option(SelDevice device, int option, int value);

@@ -49,14 +49,13 @@ int ensure_scratch(SelSceneTy* sc, size_t bytes) {
     return SEL_OK;
 }
 
+// The kernels' error word lies in page-locked host memory: once their stream is done it is a plain read.
 int read_error_word(SelDeviceTy* dev, cudaStream_t s) {
-    uint32_t word = 0;
-    cudaError_t e = cudaMemcpyAsync(&word, dev->d_err, sizeof(word), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(e, "reading device error word");
+    if (__atomic_load_n(dev->h_err, __ATOMIC_RELAXED) == 0) return SEL_OK;
+    const uint32_t word = __atomic_exchange_n(dev->h_err, 0u, __ATOMIC_RELAXED);
     if (word) {
-        cudaMemsetAsync(dev->d_err, 0, sizeof(uint32_t), s);
-        cudaStreamSynchronize(s);
         const char* what = (word & 2u)    ? "traversal stack overflow"
                            : (word & 4u)  ? "Ptex filter frame stack overflow"
                            : (word & 8u)  ? "render queue overflow"
@@ -122,8 +121,18 @@ int sel_device_new(int cuda_device, SelDevice* out_device) {
     e = cudaStreamCreateWithFlags(&dev->stream, cudaStreamNonBlocking);
     for (int k = 0; k < 4 && e == cudaSuccess; ++k) e = cudaStreamCreateWithFlags(&dev->qstream[k], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&dev->sm_count, cudaDevAttrMultiProcessorCount, cuda_device);
-    if (e == cudaSuccess) e = cudaMalloc(&dev->d_err, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(dev->d_err, 0, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaHostAlloc(&dev->h_err, sizeof(uint32_t), cudaHostAllocMapped);
+    if (e == cudaSuccess) {
+        *dev->h_err = 0;
+        e = cudaHostGetDevicePointer(&dev->d_err, dev->h_err, 0);
+    }
+    if (e == cudaSuccess) {
+        int pageable = 0, host_tables = 0;
+        e = cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, cuda_device);
+        if (e == cudaSuccess)
+            e = cudaDeviceGetAttribute(&host_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, cuda_device);
+        dev->pageable_access = pageable && host_tables;
+    }
     // The allocation-free query's staging array: resolving its address here loads its module (and so
     // creates the array) while the device is being set up, not inside the first allocation-free call.
     if (e == cudaSuccess && resolve_noalloc_staging(dev) != SEL_OK) e = cudaErrorInvalidSymbol;
@@ -143,7 +152,7 @@ int sel_device_new(int cuda_device, SelDevice* out_device) {
         if (dev->stream) cudaStreamDestroy(dev->stream);
         for (cudaStream_t q : dev->qstream)
             if (q) cudaStreamDestroy(q);
-        if (dev->d_err) cudaFree(dev->d_err);
+        if (dev->h_err) cudaFreeHost(dev->h_err);
         delete dev;
         return cuda_fail(e, "device setup");
     }
@@ -160,7 +169,7 @@ int sel_device_release(SelDevice device) {
         cudaStreamSynchronize(q);
         cudaStreamDestroy(q);
     }
-    cudaFree(device->d_err);
+    cudaFreeHost(device->h_err);
     if (device->order_pool) cudaMemPoolDestroy(device->order_pool);  // released once its last block is freed
     delete device;
     return SEL_OK;
@@ -741,10 +750,15 @@ static int check_query(SelScene scene) {
     return SEL_OK;
 }
 
-// The device address of `bytes` of host memory at p when the whole range is page-locked memory that the current
-// device can address (cudaHostAlloc / cudaMallocHost / cudaHostRegister under unified addressing): both ends
-// must belong to pinned memory mapped contiguously into the device's address space.
-static bool mapped_host_range(const void* p, size_t bytes, int device, void** dptr) {
+// The device address of `bytes` of host memory at p that the current device can address: any host memory when the
+// GPU walks the host's page tables (Grace), else page-locked memory (cudaHostAlloc / cudaMallocHost /
+// cudaHostRegister under unified addressing) whose both ends are mapped contiguously into the device's address space.
+static bool mapped_host_range(const void* p, size_t bytes, const SelDeviceTy* dev, void** dptr) {
+    if (dev->pageable_access) {
+        *dptr = const_cast<void*>(p);
+        return true;
+    }
+    const int device = dev->cuda_device;
     cudaPointerAttributes a{}, b{};
     const char* first = static_cast<const char*>(p);
     const char* last = first + bytes - 1;
@@ -761,11 +775,22 @@ static bool mapped_host_range(const void* p, size_t bytes, int device, void** dp
     return true;
 }
 
+static bool page_locked(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+}
+
 // Whether a batch's rays run nearly parallel from one record to the next (camera rays in pixel order): sampled
 // pairs of neighbouring records, directions within about 2.5 degrees.  Such rays traverse so fast that moving
-// the records over the host link is the whole cost, and the copy engines' full-duplex staging moves them
-// fastest; incoherent rays traverse long enough to hide the link's latency, and the query kernel reads and
-// writes them in place.
+// the records over the host link is the whole cost, and for page-locked records the copy engines' full-duplex
+// staging moves large closest-hit batches fastest (0.6 M, 1 M, 4.2 M camera rays: 0.61, 0.92, 3.08 ms staged
+// against 0.45, 0.75, 3.41 in place, so from about 2 M on; any hit 0.39, 0.53, 1.73 against 0.29, 0.46, 1.70);
+// incoherent rays traverse long enough to hide the link's latency.  Copies of pageable records are slower than
+// either: 4.2 M camera rays 6.6 ms staged, 3.4 in place.
 static bool coherent_batch(const void* recs, size_t byte_stride, unsigned int M) {
     constexpr unsigned kPairs = 256;
     if (M < 2) return false;
@@ -797,18 +822,21 @@ static int host_query(SelScene scene, Rec* recs, unsigned int M, size_t byte_str
     const size_t bytes = size_t(M) * sizeof(Rec);
     const bool dense = byte_stride == sizeof(Rec);
     cudaError_t e = cudaSuccess;
-    // Records in page-locked host memory the GPU can address (over NVLink-C2C on Grace): the query kernel reads
-    // each ray and writes each hit in place, so only the fields it touches cross the link and no staging buffer
-    // or copy is needed.  Any 16-byte aligned stride that is a multiple of 16 works.  Large dense batches of
-    // coherent rays take the staged pipeline below instead (coherent_batch).
-    constexpr unsigned kChunk = 1u << 18;
+    // Records in host memory the GPU can address (over NVLink-C2C on Grace): the query kernel reads each ray and
+    // writes each hit in place, so only the fields it touches cross the link and no staging buffer or copy is
+    // needed.  Any 16-byte aligned stride that is a multiple of 16 works.  Pageable records too, where the GPU walks
+    // the host's page tables: one ray 15 us a call against 21 staged (43 with the copies, two synchronisations and a
+    // read-back of the error word that a call took before), 300,000 incoherent rays 0.36 against 0.63 ms.  Closest-hit
+    // batches of more than 2 M coherent rays in page-locked memory take the staged pipeline below (coherent_batch).
+    constexpr unsigned kChunk = 1u << 18, kStageCoherent = 1u << 21;
     const bool staged_pipeline = dense && M > 2 * kChunk;
+    const bool staged_faster = kHit && dense && M > kStageCoherent && page_locked(recs) &&
+                               coherent_batch(recs, byte_stride, M);
     void* mapped = nullptr;
     if (dev->zero_copy && byte_stride % 16 == 0 && (reinterpret_cast<uintptr_t>(recs) & 15u) == 0 &&
-        !(staged_pipeline && coherent_batch(recs, byte_stride, M)) &&
-        mapped_host_range(recs, size_t(M - 1) * byte_stride + sizeof(Rec), dev->cuda_device, &mapped)) {
+        !staged_faster &&
+        mapped_host_range(recs, size_t(M - 1) * byte_stride + sizeof(Rec), dev, &mapped)) {
         e = launch_query_strided(!kHit, device_bvh(scene), mapped, byte_stride, M, dev->d_err, dev->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(dev->stream);
         if (e != cudaSuccess) return cuda_fail(e, "zero-copy query");
         return read_error_word(dev, dev->stream);
     }

@@ -16,7 +16,9 @@ struct SelDeviceTy {
     cudaStream_t stream = nullptr;  // internal stream for the host-memory entry points
     cudaStream_t qstream[4] = {nullptr, nullptr, nullptr, nullptr};  // pipelined host-memory queries (chunk k on k % 4)
     int sm_count = 1;
-    uint32_t* d_err = nullptr;      // kernel error word (iteration cap / stack overflow bits)
+    uint32_t* h_err = nullptr;      // kernel error word (iteration cap / stack overflow bits), page-locked host memory
+    uint32_t* d_err = nullptr;      // its device address
+    bool pageable_access = false;   // the GPU reads and writes any host memory through the host's page tables
     cudaMemPool_t order_pool = nullptr;  // stream-ordered scratch of ordered queries (keeps freed memory)
     bool graph_replay = true;       // SEL_OPTION_GRAPH_REPLAY
     bool material_sort = true;      // SEL_OPTION_MATERIAL_SORT
