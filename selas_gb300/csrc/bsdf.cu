@@ -26,6 +26,7 @@ __device__ __forceinline__ Surface load_surface(const SelSurface& r) {
     s.scatter_distance = r.scatterDistance;
     s.ior = r.ior;
     s.shader = r.shader;
+    disney::derive(s);
     return s;
 }
 

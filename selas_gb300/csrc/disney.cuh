@@ -31,6 +31,8 @@ struct Surface {
     float anisotropic, relative_ior, specular_tint, roughness;
     float scatter_distance, ior;
     int shader;
+    float alpha_x, alpha_y;                 // aniso(roughness, anisotropic)
+    float p_spec, p_diff, p_coat, p_trans;  // lobe_pdfs
 };
 
 struct BsdfSampleOut {
@@ -103,24 +105,31 @@ SEL_HD float ggx_d(float3 wm, float ax, float ay) {
     const float ax2 = sqr(ax), ay2 = sqr(ay);
     return 1.0f / (kPi * ax * ay * sqr(hx2 / ax2 + hy2 / ay2 + c2));
 }
-// Heitz 2018 visible-normal sampling (Ggx.cpp:105-128)
-SEL_HD float3 sample_vndf(float3 wo, float ax, float ay, float u1, float u2) {
-    const float3 v = normalize(f3(wo.x * ax, wo.y, wo.z * ay));
-    const float3 t1 = (v.y < 0.9999f) ? normalize(cross(v, f3(0.0f, 1.0f, 0.0f))) : f3(1.0f, 0.0f, 0.0f);
-    const float3 t2 = cross(t1, v);
-    const float a = 1.0f / (1.0f + v.y);
-    const float r = sqrtf(u1);
-    const float phi = (u2 < a) ? (u2 / a) * kPi : kPi + (u2 - a) / (1.0f - a) * kPi;
-    const float p1 = r * cosf(phi);
-    const float p2 = r * sinf(phi) * ((u2 < a) ? 1.0f : v.y);
-    const float3 n = p1 * t1 + p2 * t2 + sqrtf(fmaxf(0.0f, 1.0f - p1 * p1 - p2 * p2)) * v;
+// Heitz 2018 visible-normal sampling (Ggx.cpp:105-128) in two halves around the sine and cosine of its angle
+// (which the diffuse lobe needs too).
+struct VndfSetup {
+    float3 v, t1, t2;
+    float a, phi;
+};
+SEL_HD VndfSetup vndf_begin(float3 wo, float ax, float ay, float u2) {
+    VndfSetup q;
+    q.v = normalize(f3(wo.x * ax, wo.y, wo.z * ay));
+    q.t1 = (q.v.y < 0.9999f) ? normalize(cross(q.v, f3(0.0f, 1.0f, 0.0f))) : f3(1.0f, 0.0f, 0.0f);
+    q.t2 = cross(q.t1, q.v);
+    q.a = 1.0f / (1.0f + q.v.y);
+    q.phi = (u2 < q.a) ? (u2 / q.a) * kPi : kPi + (u2 - q.a) / (1.0f - q.a) * kPi;
+    return q;
+}
+SEL_HD float3 vndf_end(const VndfSetup& q, float ax, float ay, float u2, float r, float cos_phi, float sin_phi) {
+    const float p1 = r * cos_phi;
+    const float p2 = r * sin_phi * ((u2 < q.a) ? 1.0f : q.v.y);
+    const float3 n = p1 * q.t1 + p2 * q.t2 + sqrtf(fmaxf(0.0f, 1.0f - p1 * p1 - p2 * p2)) * q.v;
     return normalize(f3(ax * n.x, n.y, ay * n.z));
 }
-// forward and reverse visible-normal pdfs (Ggx.cpp:143-156)
-SEL_HD void vndf_pdfs(float3 wi, float3 wm, float3 wo, float ax, float ay, float& fwd, float& rev) {
-    const float d = ggx_d(wm, ax, ay);
-    fwd = smith_g1(wo, ax, ay) * fabsf(dot(wm, wi)) * d / fabsf(wi.y);
-    rev = smith_g1(wi, ax, ay) * fabsf(dot(wm, wo)) * d / fabsf(wo.y);
+// forward and reverse visible-normal pdfs (Ggx.cpp:143-156) from D and both masking terms
+SEL_HD void vndf_pdfs(float3 wi, float3 wm, float3 wo, float d, float g_wi, float g_wo, float& fwd, float& rev) {
+    fwd = g_wo * fabsf(dot(wm, wi)) * d / fabsf(wi.y);
+    rev = g_wi * fabsf(dot(wm, wo)) * d / fabsf(wo.y);
 }
 
 SEL_HD float3 reflect(float3 n, float3 l) { return 2.0f * dot(n, l) * n - l; }
@@ -157,6 +166,11 @@ SEL_HD void aniso(float r, float anisotropic, float& ax, float& ay) {
     ax = fmaxf(0.001f, sqr(r) / aspect);
     ay = fmaxf(0.001f, sqr(r) * aspect);
 }
+// What the lobes take from the material alone.
+SEL_HD void derive(Surface& s) {
+    aniso(s.roughness, s.anisotropic, s.alpha_x, s.alpha_y);
+    lobe_pdfs(s, s.p_spec, s.p_diff, s.p_coat, s.p_trans);
+}
 SEL_HD float3 tint(float3 c) {
     const float lum = dot(f3(0.3f, 0.6f, 1.0f), c);
     return lum > 0.0f ? c * (1.0f / lum) : f3(1.0f);
@@ -183,39 +197,43 @@ SEL_HD float3 sheen_eval(const Surface& s, float3 wm, float3 wi) {
     const float hl = fabsf(dot(wm, wi));
     return s.sheen * lerp3(f3(1.0f), tint(s.base_color), s.sheen_tint) * schlick_weight(hl);
 }
+// The interpolation ends at the dielectric term when metallic is 0; the Schlick term (a powf and a division) is
+// skipped then unless its operands could make it infinite or NaN, which 0 times it would pass on.
 SEL_HD float3 disney_fresnel(const Surface& s, float3 wo, float3 wm, float3 wi) {
     const float hv = dot(wm, wo);
+    const float fd = dielectric(hv, 1.0f, s.ior);
+    if (s.metallic == 0.0f) {
+        const float lum = dot(f3(0.3f, 0.6f, 1.0f), s.base_color);
+        const float rel = s.relative_ior;
+        const float least = fminf(fminf(s.base_color.x, s.base_color.y), s.base_color.z);
+        const bool tame = (lum == 0.0f || (lum > 1e-30f && lum < 1e30f)) && least >= 0.0f && rel > 0.0f &&
+                          rel < 1e15f && fabsf(s.specular_tint) < 1e15f;
+        if (tame) return f3(fd);
+    }
     float3 r0 = schlick_r0(s.relative_ior) * lerp3(f3(1.0f), tint(s.base_color), s.specular_tint);
     r0 = lerp3(r0, s.base_color, s.metallic);
-    const float fd = dielectric(hv, 1.0f, s.ior);
     const float3 fm = schlick_color(r0, dot(wi, wm));
     return lerp3(f3(fd), fm, s.metallic);
 }
-SEL_HD float3 brdf_eval(const Surface& s, float3 wo, float3 wm, float3 wi, float& fpdf, float& rpdf) {
+// d, gl, gv: ggx_d(wm), smith_g1(wi), smith_g1(wo) at the surface's widths
+SEL_HD float3 brdf_eval(const Surface& s, float3 wo, float3 wm, float3 wi, float d, float gl, float gv,
+                        float& fpdf, float& rpdf) {
     fpdf = 0.0f;
     rpdf = 0.0f;
     const float nl = wi.y, nv = wo.y;
     if (nl <= 0.0f || nv <= 0.0f) return f3(0.0f);
-    float ax, ay;
-    aniso(s.roughness, s.anisotropic, ax, ay);
-    const float d = ggx_d(wm, ax, ay);
-    const float gl = smith_g1(wi, ax, ay);
-    const float gv = smith_g1(wo, ax, ay);
     const float3 f = disney_fresnel(s, wo, wm, wi);
-    vndf_pdfs(wi, wm, wo, ax, ay, fpdf, rpdf);
+    vndf_pdfs(wi, wm, wo, d, gl, gv, fpdf, rpdf);
     fpdf *= (1.0f / (4.0f * fabsf(dot(wo, wm))));
     rpdf *= (1.0f / (4.0f * fabsf(dot(wi, wm))));
     return d * gl * gv * f * (1.0f / (4.0f * nl * nv));
 }
-SEL_HD float3 spec_trans_eval(const Surface& s, float3 wo, float3 wm, float3 wi, float ax, float ay, bool thin) {
+SEL_HD float3 spec_trans_eval(const Surface& s, float3 wo, float3 wm, float3 wi, float d, float gl, float gv, bool thin) {
     const float rel = s.relative_ior;
     const float n2 = rel * rel;
     const float abs_nl = fabsf(wi.y), abs_nv = fabsf(wo.y);
     const float hl = dot(wm, wi), hv = dot(wm, wo);
     const float abs_hl = fabsf(hl), abs_hv = fabsf(hv);
-    const float d = ggx_d(wm, ax, ay);
-    const float gl = smith_g1(wi, ax, ay);
-    const float gv = smith_g1(wo, ax, ay);
     const float f = dielectric(hv, 1.0f, s.ior);
     const float3 color = thin ? sqrt3(s.base_color) : s.base_color;
     const float c = (abs_hl * abs_hv) / (abs_nl * abs_nv);
@@ -260,13 +278,17 @@ SEL_HD float3 evaluate(const Surface& s, float3 v, float3 l, bool thin, float& f
     float3 refl = f3(0.0f);
     fwd = 0.0f;
     rev = 0.0f;
-    float p_brdf, p_diff, p_coat, p_trans;
-    lobe_pdfs(s, p_brdf, p_diff, p_coat, p_trans);
-    float ax, ay;
-    aniso(s.roughness, s.anisotropic, ax, ay);
+    const float p_brdf = s.p_spec, p_diff = s.p_diff, p_coat = s.p_coat, p_trans = s.p_trans;
     const float w_diff = (1.0f - s.metallic) * (1.0f - s.spec_trans);
     const float w_trans = (1.0f - s.metallic) * s.spec_trans;
     const bool upper = nl > 0.0f && nv > 0.0f;
+    // D and masking at the surface's widths, shared by the specular and (solid) transmission lobes and their pdfs
+    float d = 0.0f, gl = 0.0f, gv = 0.0f;
+    if (upper || (!thin && w_trans > 0.0f)) {
+        d = ggx_d(wm, s.alpha_x, s.alpha_y);
+        gl = smith_g1(wi, s.alpha_x, s.alpha_y);
+        gv = smith_g1(wo, s.alpha_x, s.alpha_y);
+    }
     if (upper && s.clearcoat > 0.0f) {
         float fc, rc;
         const float c = clearcoat_eval(s.clearcoat, s.clearcoat_gloss, wo, wm, wi, fc, rc);
@@ -276,27 +298,32 @@ SEL_HD float3 evaluate(const Surface& s, float3 v, float3 l, bool thin, float& f
     }
     if (w_diff > 0.0f) {
         const float fd = fabsf(wi.y), rd = fabsf(wo.y);
-        const float d = diffuse_eval(s, wo, wm, wi, thin);
+        const float df = diffuse_eval(s, wo, wm, wi, thin);
         const float3 sh = sheen_eval(s, wm, wi);
-        refl += w_diff * (d * s.base_color + sh);
+        refl += w_diff * (df * s.base_color + sh);
         fwd += p_diff * fd;
         rev += p_diff * rd;
     }
     if (w_trans > 0.0f) {
-        const float rs = thin ? thin_roughness(s.ior, s.roughness) : s.roughness;
-        float tax, tay;
-        aniso(rs, s.anisotropic, tax, tay);
-        const float3 tr = spec_trans_eval(s, wo, wm, wi, tax, tay, thin);
+        float td = d, tgl = gl, tgv = gv;
+        if (thin) {
+            float tax, tay;
+            aniso(thin_roughness(s.ior, s.roughness), s.anisotropic, tax, tay);
+            td = ggx_d(wm, tax, tay);
+            tgl = smith_g1(wi, tax, tay);
+            tgv = smith_g1(wo, tax, tay);
+        }
+        const float3 tr = spec_trans_eval(s, wo, wm, wi, td, tgl, tgv, thin);
         refl += w_trans * tr;
         float ft, rt;
-        vndf_pdfs(wi, wm, wo, tax, tay, ft, rt);
+        vndf_pdfs(wi, wm, wo, td, tgl, tgv, ft, rt);
         const float lh = dot(wm, wi), vh = dot(wm, wo);
         fwd += p_trans * ft / sqr(lh + s.relative_ior * vh);
         rev += p_trans * rt / sqr(vh + s.relative_ior * lh);
     }
     if (upper) {
         float fm, rm;
-        const float3 sp = brdf_eval(s, wo, wm, wi, fm, rm);
+        const float3 sp = brdf_eval(s, wo, wm, wi, d, gl, gv, fm, rm);
         refl += sp;
         fwd += p_brdf * fm / (4.0f * fabsf(dot(wo, wm)));
         rev += p_brdf * rm / (4.0f * fabsf(dot(wi, wm)));
@@ -311,29 +338,7 @@ SEL_HD void clear_sample(BsdfSampleOut& o) {
     o.wi = f3(0.0f);
 }
 
-// Each sampler below draws its uniforms from u[] in the order the reference draws them.
-SEL_HD bool sample_brdf(const Surface& s, float3 v, const float* u, int& used, BsdfSampleOut& o) {
-    const float3 wo = normalize(to_local(s, v));
-    float ax, ay;
-    aniso(s.roughness, s.anisotropic, ax, ay);
-    const float r0 = u[used++], r1 = u[used++];
-    const float3 wm = sample_vndf(wo, ax, ay, r0, r1);
-    const float3 wi = normalize(reflect(wm, wo));
-    if (wi.y <= 0.0f) {
-        clear_sample(o);
-        return false;
-    }
-    const float3 F = disney_fresnel(s, wo, wm, wi);
-    const float g1v = smith_g1(wo, ax, ay);
-    o.flags = kScatterEvent;
-    o.reflectance = g1v * F;
-    o.wi = normalize(to_world(s, wi));
-    vndf_pdfs(wi, wm, wo, ax, ay, o.forward_pdf, o.reverse_pdf);
-    o.forward_pdf *= (1.0f / (4.0f * fabsf(dot(wo, wm))));
-    o.reverse_pdf *= (1.0f / (4.0f * fabsf(dot(wi, wm))));
-    return true;
-}
-
+// The samplers draw their uniforms from u[] in the order the reference draws them.
 SEL_HD bool sample_clearcoat(const Surface& s, float3 v, const float* u, int& used, BsdfSampleOut& o) {
     const float3 wo = normalize(to_local(s, v));
     const float a = 0.25f, a2 = a * a;
@@ -357,125 +362,141 @@ SEL_HD bool sample_clearcoat(const Surface& s, float3 v, const float* u, int& us
     return true;
 }
 
-SEL_HD bool sample_spec_trans(const Surface& s, float3 v, bool thin, const float* u, int& used, BsdfSampleOut& o) {
-    const float3 wo = to_local(s, v);
-    if (wo.y == 0.0f) {
+// The lobes but the clearcoat (SampleDisneyBRDF, SampleDisneySpecTransmission, SampleDisneyDiffuse), r0, r1 being
+// their first two uniforms.  Shading is bound by the instructions of diverged warps, whose lanes take different lobes:
+// what the lobes share (the sine, cosine and radius, the visible normal with its masking and pdfs, the way back to
+// world space) is written once, so that a warp runs it once.
+SEL_HD bool sample_lobe(const Surface& s, float3 v, bool thin, bool spec, bool diffuse, const float* u, int& used,
+                        BsdfSampleOut& o) {
+    const float3 raw = to_local(s, v);
+    const bool trans = !spec && !diffuse;
+    if (trans && raw.y == 0.0f) {
         clear_sample(o);
         return false;
     }
-    const float rs = thin ? thin_roughness(s.ior, s.roughness) : s.roughness;
-    float tax, tay;
-    aniso(rs, s.anisotropic, tax, tay);
-    const float r0 = u[used++], r1 = u[used++];
-    const float3 wm = sample_vndf(wo, tax, tay, r0, r1);
-    float vh = dot(wo, wm);
-    if (wm.y < 0.0f) vh = -vh;
-    const float ni = wo.y > 0.0f ? 1.0f : s.ior;
-    const float nt = wo.y > 0.0f ? s.ior : 1.0f;
-    const float rel = ni / nt;
-    const float F = dielectric(vh, 1.0f, s.ior);
-    const float g1v = smith_g1(wo, tax, tay);
-    float pdf;
+    const float r0 = u[1], r1 = u[2];
+    used += 2;
+    float ax = s.alpha_x, ay = s.alpha_y;
+    if (thin && trans) aniso(thin_roughness(s.ior, s.roughness), s.anisotropic, ax, ay);
+    const float3 wo = spec ? normalize(raw) : raw;
+    VndfSetup q;
+    float phi = kTwoPi * r1;
+    if (!diffuse) {
+        q = vndf_begin(wo, ax, ay, r1);
+        phi = q.phi;
+    }
+    const float r = sqrtf(r0), cos_p = cosf(phi), sin_p = sinf(phi);
     float3 wi;
-    if (u[used++] <= F) {
-        wi = normalize(reflect(wm, wo));
-        o.flags = kScatterEvent;
-        o.reflectance = g1v * s.base_color;
-        pdf = F / (4.0f * fabsf(dot(wo, wm)));
-    } else {
-        if (thin) {
-            wi = reflect(wm, wo);
-            wi.y = -wi.y;
-            o.reflectance = g1v * sqrt3(s.base_color);
-            o.flags = kScatterEvent;
-        } else {
-            if (transmit(wm, wo, rel, wi)) {
-                o.flags = kTransmissionEvent;
-                o.medium_phase = vh > 0.0f ? 1 : 0;
-                o.extinction = extinction(s.transmittance_color, s.scatter_distance);
+    if (diffuse) {
+        const float sign = wo.y > 0.0f ? 1.0f : (wo.y < 0.0f ? -1.0f : 0.0f);
+        wi = sign * f3(r * cos_p, sqrtf(fmaxf(0.0f, 1.0f - r0)), r * sin_p);
+        const float3 wm = normalize(wi + wo);
+        const float nl = wi.y;
+        if (nl == 0.0f) {
+            clear_sample(o);
+            return false;
+        }
+        const float nv = wo.y;
+        float pdf;
+        unsigned ev = kScatterEvent;
+        float3 color = s.base_color;
+        ++used;
+        if (u[3] <= s.diff_trans) {
+            wi = -wi;
+            pdf = s.diff_trans;
+            if (thin) {
+                color = sqrt3(color);
             } else {
-                o.flags = kScatterEvent;
-                wi = reflect(wm, wo);
+                ev = kTransmissionEvent;
+                o.medium_phase = 1;
+                o.extinction = extinction(s.transmittance_color, s.scatter_distance);
             }
-            o.reflectance = g1v * s.base_color;
-        }
-        wi = normalize(wi);
-        const float lh = fabsf(dot(wi, wm));
-        const float jac = lh / sqr(lh + s.relative_ior * vh);
-        pdf = (1.0f - F) / jac;
-    }
-    if (wi.y == 0.0f) {
-        clear_sample(o);
-        return false;
-    }
-    if (s.roughness < 0.01f) o.flags |= kDiracEvent;
-    vndf_pdfs(wi, wm, wo, tax, tay, o.forward_pdf, o.reverse_pdf);
-    o.forward_pdf *= pdf;
-    o.reverse_pdf *= pdf;
-    o.wi = normalize(to_world(s, wi));
-    return true;
-}
-
-SEL_HD bool sample_diffuse(const Surface& s, float3 v, bool thin, const float* u, int& used, BsdfSampleOut& o) {
-    const float3 wo = to_local(s, v);
-    const float sign = wo.y > 0.0f ? 1.0f : (wo.y < 0.0f ? -1.0f : 0.0f);
-    const float r0 = u[used++], r1 = u[used++];
-    const float rr = sqrtf(r0);
-    const float th = kTwoPi * r1;
-    float3 wi = sign * f3(rr * cosf(th), sqrtf(fmaxf(0.0f, 1.0f - r0)), rr * sinf(th));
-    const float3 wm = normalize(wi + wo);
-    const float nl = wi.y;
-    if (nl == 0.0f) {
-        clear_sample(o);
-        return false;
-    }
-    const float nv = wo.y;
-    float pdf;
-    unsigned ev = kScatterEvent;
-    float3 color = s.base_color;
-    if (u[used++] <= s.diff_trans) {
-        wi = -wi;
-        pdf = s.diff_trans;
-        if (thin) {
-            color = sqrt3(color);
         } else {
-            ev = kTransmissionEvent;
-            o.medium_phase = 1;
-            o.extinction = extinction(s.transmittance_color, s.scatter_distance);
+            pdf = 1.0f - s.diff_trans;
         }
+        const float3 sh = sheen_eval(s, wm, wi);
+        const float d = diffuse_eval(s, wo, wm, wi, thin);
+        o.reflectance = sh + color * (d / pdf);
+        o.forward_pdf = fabsf(nl) * pdf;
+        o.reverse_pdf = fabsf(nv) * pdf;
+        o.flags = ev;
     } else {
-        pdf = 1.0f - s.diff_trans;
+        const float3 wm = vndf_end(q, ax, ay, r1, r, cos_p, sin_p);
+        const float g1v = smith_g1(wo, ax, ay);
+        float pdf = 0.0f;
+        if (spec) {
+            wi = normalize(reflect(wm, wo));
+            if (wi.y <= 0.0f) {
+                clear_sample(o);
+                return false;
+            }
+            const float3 F = disney_fresnel(s, wo, wm, wi);
+            o.flags = kScatterEvent;
+            o.reflectance = g1v * F;
+        } else {
+            float vh = dot(wo, wm);
+            if (wm.y < 0.0f) vh = -vh;
+            const float ni = wo.y > 0.0f ? 1.0f : s.ior;
+            const float nt = wo.y > 0.0f ? s.ior : 1.0f;
+            const float rel = ni / nt;
+            const float F = dielectric(vh, 1.0f, s.ior);
+            ++used;
+            if (u[3] <= F) {
+                wi = normalize(reflect(wm, wo));
+                o.flags = kScatterEvent;
+                o.reflectance = g1v * s.base_color;
+                pdf = F / (4.0f * fabsf(dot(wo, wm)));
+            } else {
+                if (thin) {
+                    wi = reflect(wm, wo);
+                    wi.y = -wi.y;
+                    o.reflectance = g1v * sqrt3(s.base_color);
+                    o.flags = kScatterEvent;
+                } else {
+                    if (transmit(wm, wo, rel, wi)) {
+                        o.flags = kTransmissionEvent;
+                        o.medium_phase = vh > 0.0f ? 1 : 0;
+                        o.extinction = extinction(s.transmittance_color, s.scatter_distance);
+                    } else {
+                        o.flags = kScatterEvent;
+                        wi = reflect(wm, wo);
+                    }
+                    o.reflectance = g1v * s.base_color;
+                }
+                wi = normalize(wi);
+                const float lh = fabsf(dot(wi, wm));
+                const float jac = lh / sqr(lh + s.relative_ior * vh);
+                pdf = (1.0f - F) / jac;
+            }
+            if (wi.y == 0.0f) {
+                clear_sample(o);
+                return false;
+            }
+            if (s.roughness < 0.01f) o.flags |= kDiracEvent;
+        }
+        vndf_pdfs(wi, wm, wo, ggx_d(wm, ax, ay), smith_g1(wi, ax, ay), g1v, o.forward_pdf, o.reverse_pdf);
+        if (spec) {
+            o.forward_pdf *= (1.0f / (4.0f * fabsf(dot(wo, wm))));
+            o.reverse_pdf *= (1.0f / (4.0f * fabsf(dot(wi, wm))));
+        } else {
+            o.forward_pdf *= pdf;
+            o.reverse_pdf *= pdf;
+        }
     }
-    const float3 sh = sheen_eval(s, wm, wi);
-    const float d = diffuse_eval(s, wo, wm, wi, thin);
-    o.reflectance = sh + color * (d / pdf);
     o.wi = normalize(to_world(s, wi));
-    o.forward_pdf = fabsf(nl) * pdf;
-    o.reverse_pdf = fabsf(nv) * pdf;
-    o.flags = ev;
     return true;
 }
 
 // SampleDisney (Disney.cpp:617-659)
 SEL_HD bool sample(const Surface& s, float3 v, bool thin, const float* u, int& used, BsdfSampleOut& o) {
-    float p_spec, p_diff, p_coat, p_trans;
-    lobe_pdfs(s, p_spec, p_diff, p_coat, p_trans);
-    bool ok;
-    float p_lobe;
-    const float p = u[used++];
-    if (p <= p_spec) {
-        ok = sample_brdf(s, v, u, used, o);
-        p_lobe = p_spec;
-    } else if (p <= p_spec + p_coat) {
-        ok = sample_clearcoat(s, v, u, used, o);
-        p_lobe = p_coat;
-    } else if (p <= p_spec + p_coat + p_diff) {
-        ok = sample_diffuse(s, v, thin, u, used, o);
-        p_lobe = p_diff;
-    } else {
-        ok = sample_spec_trans(s, v, thin, u, used, o);
-        p_lobe = p_trans;
-    }
+    const float p = u[0];
+    ++used;
+    const float p_spec = s.p_spec, p_coat = s.p_coat, p_diff = s.p_diff, p_trans = s.p_trans;
+    const bool spec = p <= p_spec;
+    const bool coat = !spec && p <= p_spec + p_coat;
+    const bool diffuse = !spec && !coat && p <= p_spec + p_coat + p_diff;
+    const bool ok = coat ? sample_clearcoat(s, v, u, used, o) : sample_lobe(s, v, thin, spec, diffuse, u, used, o);
+    const float p_lobe = spec ? p_spec : (coat ? p_coat : (diffuse ? p_diff : p_trans));
     if (p_lobe > 0.0f) {
         o.reflectance = o.reflectance * (1.0f / p_lobe);
         o.forward_pdf *= p_lobe;

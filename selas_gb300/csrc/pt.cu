@@ -448,6 +448,7 @@ __global__ void __launch_bounds__(kBlock) k_texture(PtParams P, int cur, const u
             base = tex2d_base_colour(m, geom < r.attr_count ? r.attrs + geom : nullptr, __float_as_uint(p0.w), hit.y,
                                      hit.z);
         }
+        base = pow3(base, 2.2f);
         P.st.base[s] = make_float4(base.x, base.y, base.z, 0.0f);
     }
     if (status) atomicOr(P.err, status);
@@ -523,12 +524,12 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
                 // RayPick error bound (PathTracer.cpp:134-136)
                 const float err = 32.0f * 1.19209e-07f *
                                   fmaxf(fmaxf(fabsf(pos.x), fabsf(pos.y)), fmaxf(fabsf(pos.z), hit.x));
-                float3 base = ld3(m.base_color);
+                float3 base = ld3(m.base_linear);
                 if (m.flags & kMaterialTextured) {  // filtered or sampled by k_texture for this hit
                     const float4 b = P.st.base[s];
                     base = f3(b.x, b.y, b.z);
                 }
-                const Surface sf = make_surface_frame(m, ft, fn, fb, -d, pow3(base, 2.2f));
+                const Surface sf = make_surface_frame(m, ft, fn, fb, -d, base);
                 // Next-event estimation to the surface's light set (AreaLighting.cpp:353-373)
                 LightSample ls;
                 ls.radiance = f3(0.0f);
@@ -601,14 +602,18 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
                         }
                     }
                 }
-                // BSDF sampling: draw ahead from a copy of the stream, then advance by what was used
+                // BSDF sampling: draw ahead, then keep the stream's state after the draws that were used (every shader
+                // uses at least one)
                 float u4[4];
-                Pcg32 ahead = rng;
-                for (int k = 0; k < 4; ++k) u4[k] = pcg_float(ahead);
+                uint64_t state[4];  // after 1..4 draws
+                for (int k = 0; k < 4; ++k) {
+                    u4[k] = pcg_float(rng);
+                    state[k] = rng.state;
+                }
                 int used = 0;
                 BsdfSampleOut bs;
                 const bool ok = bsdf_sample_as<kShader>(sf, -d, u4, used, bs);
-                for (int k = 0; k < used; ++k) pcg_next(rng);
+                rng.state = used <= 1 ? state[0] : (used == 2 ? state[1] : (used == 3 ? state[2] : state[3]));
                 if (!ok) {
                     alive = false;
                 } else if (deferred) {

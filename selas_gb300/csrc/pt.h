@@ -107,7 +107,7 @@ struct PtState {
     uint32_t* queue_sorted;  // the current queue ordered by material class (counting sort; textured scenes:
                              // class, then Ptex face, by radix sort)
     uint32_t* cls;    // material class of each current queue entry
-    float4* base;     // Ptex base colour (authored, before the 2.2 power) of the path's current hit
+    float4* base;     // textured base colour (linear) of the path's current hit
     float4* sh_o;     // shadow rays (2 per path slot): origin, tnear
     float4* sh_d;     // direction, tfar
     float4* sh_c;     // contribution, (job << 28 | pixel) bits

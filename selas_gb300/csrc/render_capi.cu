@@ -10,6 +10,7 @@
 #include "ibl.cuh"
 #include "pt.h"
 #include "ptex_quad.cuh"
+#include "shading.cuh"
 #include "vcm.h"
 
 using namespace sel;
@@ -54,6 +55,15 @@ SelMaterial default_material() {
     m.baseColor[0] = m.baseColor[1] = m.baseColor[2] = 0.6f;
     m.ior = 1.5f;
     return m;
+}
+
+__global__ void k_derive_materials(MaterialDev* m, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) derive_material(m[i]);
+}
+__global__ void k_derive_lights(QuadLight* l, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) derive_light(l[i]);
 }
 
 template <typename T>
@@ -348,6 +358,13 @@ int sync_shading(SelSceneTy* sc) {
     if (int rc = upload(sc->d_materials, mats.data(), mats.size())) return rc;
     if (int rc = upload(sc->d_lights, lights.data(), lights.size())) return rc;
     if (int rc = upload(sc->d_light_sets, sets.data(), sets.size())) return rc;
+    k_derive_materials<<<unsigned((mats.size() + 127) / 128), 128>>>(static_cast<MaterialDev*>(sc->d_materials),
+                                                                     uint32_t(mats.size()));
+    if (!lights.empty())
+        k_derive_lights<<<unsigned((lights.size() + 127) / 128), 128>>>(static_cast<QuadLight*>(sc->d_lights),
+                                                                        uint32_t(lights.size()));
+    if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return cuda_fail(e, "deriving shading data");
+    if (cudaError_t e = cudaStreamSynchronize(nullptr); e != cudaSuccess) return cuda_fail(e, "deriving shading data");
     if (int rc = upload_ibl(sc)) return rc;
     if (int rc = upload_attrs(sc)) return rc;
     if (sc->d_view) {

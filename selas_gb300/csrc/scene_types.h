@@ -8,13 +8,18 @@
 namespace sel {
 
 // SceneLight as NextEventEstimation reads it (SceneLib/SceneResource.h; AreaLighting.cpp:113-153):
-// centre, facing direction, full edge vectors x and z, emitted radiance.
+// centre, facing direction, full edge vectors x and z, emitted radiance.  The rest is derived once per light on the
+// device (derive_light), as every sample would compute it: the corner, the edges' lengths and unit vectors and
+// their cross product.
 struct QuadLight {
     float3 position, direction, x, z, radiance;
+    float3 corner, unit_x, unit_z, unit_n;
+    float length_x, length_z;
 };
 
-// Per-geometry material record in HBM (128 bytes): the MaterialResourceData fields the shading reads
-// (SceneLib/ModelResource.h:68-88) plus the geometry's light set and Ptex face range.
+// Per-geometry material record in HBM (160 bytes): the MaterialResourceData fields the shading reads
+// (SceneLib/ModelResource.h:68-88), the geometry's light set and Ptex face range, and what the shading derives from
+// the material alone, computed once on the device (derive_material) with the operations a hit would run.
 struct MaterialDev {
     int shader;
     uint32_t flags;      // kMaterialTransparent | kMaterialUsesPtex | kMaterialUsesTexture
@@ -26,9 +31,12 @@ struct MaterialDev {
     float anisotropic, specular_tint, roughness, scatter_distance, ior;
     uint32_t tex_lo, tex_hi;        // kMaterialUsesTexture: the base-colour image (float4 texels, row-major)
     uint32_t tex_width, tex_height;
-    float pad[5];
+    float base_linear[3];                    // base_color to the power 2.2
+    float alpha_x, alpha_y;                  // the microfacet widths
+    float p_spec, p_diff, p_coat, p_trans;   // the lobes' sampling probabilities
+    float pad[4];
 };
-static_assert(sizeof(MaterialDev) == 128, "MaterialDev must be 128 bytes");
+static_assert(sizeof(MaterialDev) == 160, "MaterialDev must be 160 bytes");
 
 // Shading data of one scene as the integrators read it for hits inside instances of that scene (the model data
 // ModelDataFromRayIds finds, SceneResource.cpp:362-378): one fixed device record per scene, rewritten whenever

@@ -62,13 +62,23 @@ struct RectSampler {
     float z0, z0sq, x0, y0, y0sq, x1, y1, y1sq, b0, b1, b0sq, k, S;
 };
 
-SEL_HD void rect_init(float3 s, float3 ex, float3 ey, float3 o, RectSampler& r) {
+// What rect_init needs of a light that does not depend on the shaded point.
+SEL_HD void derive_light(QuadLight& L) {
+    L.corner = L.position - 0.5f * L.x - 0.5f * L.z;
+    L.length_x = length(L.x);
+    L.length_z = length(L.z);
+    L.unit_x = L.x * (1.0f / L.length_x);
+    L.unit_z = L.z * (1.0f / L.length_z);
+    L.unit_n = cross(L.unit_x, L.unit_z);
+}
+
+SEL_HD void rect_init(const QuadLight& L, float3 o, RectSampler& r) {
     r.o = o;
-    const float exl = length(ex), eyl = length(ey);
-    r.x = ex * (1.0f / exl);
-    r.y = ey * (1.0f / eyl);
-    r.z = cross(r.x, r.y);
-    const float3 d = s - o;
+    const float exl = L.length_x, eyl = L.length_z;
+    r.x = L.unit_x;
+    r.y = L.unit_z;
+    r.z = L.unit_n;
+    const float3 d = L.corner - o;
     r.z0 = dot(d, r.z);
     if (r.z0 > 0.0f) {
         r.z = -r.z;
@@ -117,9 +127,8 @@ struct LightSample {
 // SampleRectangleLightSolidAngle (AreaLighting.cpp:113-153): radiance already carries cos(theta_light)/d^2
 // and cos(theta_surface) (as the reference computes it), pdf is (1/solid angle) * cos(theta_light)/d^2.
 SEL_HD void sample_quad_light(const QuadLight& L, float3 p, float3 n, float u, float v, LightSample& s) {
-    const float3 corner = L.position - 0.5f * L.x - 0.5f * L.z;
     RectSampler r;
-    rect_init(corner, L.x, L.z, p, r);
+    rect_init(L, p, r);
     const float pdf = 1.0f / r.S;
     const float3 lp = rect_sample(r, u, v);
     const float3 ul = lp - p;
@@ -250,21 +259,35 @@ SEL_HD Surface make_surface_frame(const MaterialDev& m, float3 t, float3 n, floa
     s.scatter_distance = m.scatter_distance;
     s.ior = m.ior;
     s.shader = m.shader;
+    s.alpha_x = m.alpha_x;
+    s.alpha_y = m.alpha_y;
+    s.p_spec = m.p_spec;
+    s.p_diff = m.p_diff;
+    s.p_coat = m.p_coat;
+    s.p_trans = m.p_trans;
     s.relative_ior = ((m.flags & kMaterialTransparent) && dot(view, n) < 0.0f) ? s.ior : 1.0f / s.ior;
     return s;
 }
 
-// The same for meshes without shading normals or tangents: the frame around the unit geometric normal n.
-SEL_HD Surface make_surface_linear(const MaterialDev& m, float3 n, float3 view, float3 base_color_linear) {
-    float3 t, b;
-    orthonormal_basis(n, t, b);
-    return make_surface_frame(m, t, n, b, view, base_color_linear);
-}
-
-// The same from a hit: frame from the normalised geometric normal, authored base colour raised to the
-// power 2.2.
-SEL_HD Surface make_surface(const MaterialDev& m, float3 ng, float3 view, float3 base_color_authored) {
-    return make_surface_linear(m, normalize(ng), view, pow3(base_color_authored, 2.2f));
+// The derived fields of a material record.
+SEL_HD void derive_material(MaterialDev& m) {
+    const float3 base = pow3(ld3(m.base_color), 2.2f);
+    m.base_linear[0] = base.x;
+    m.base_linear[1] = base.y;
+    m.base_linear[2] = base.z;
+    Surface s;
+    s.metallic = saturate(m.metallic);
+    s.spec_trans = saturate(m.spec_trans);
+    s.clearcoat = m.clearcoat;
+    s.roughness = m.roughness;
+    s.anisotropic = m.anisotropic;
+    disney::derive(s);
+    m.alpha_x = s.alpha_x;
+    m.alpha_y = s.alpha_y;
+    m.p_spec = s.p_spec;
+    m.p_diff = s.p_diff;
+    m.p_coat = s.p_coat;
+    m.p_trans = s.p_trans;
 }
 
 // ContinuationProbability (SurfaceParameters.cpp:420-424)

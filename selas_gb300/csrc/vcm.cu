@@ -275,7 +275,7 @@ __device__ void make_vhit(const VcmParams& P, uint32_t s, float3 org, float3 dir
     const MaterialDev& m = hr.mats[mi];
     h.pos = f3(org.x + hit.x * dir.x, org.y + hit.x * dir.y, org.z + hit.x * dir.z);
     h.err = 32.0f * 1.19209e-07f * fmaxf(fmaxf(fabsf(h.pos.x), fabsf(h.pos.y)), fmaxf(fabsf(h.pos.z), hit.x));
-    float3 base = ld3(m.base_color);
+    float3 base = ld3(m.base_linear);
     const MeshAttrDev* attr = geom < hr.attr_count ? hr.attrs + geom : nullptr;
     if (m.flags & kMaterialTextured) {
         if constexpr (kPretex) {
@@ -283,12 +283,14 @@ __device__ void make_vhit(const VcmParams& P, uint32_t s, float3 org, float3 dir
             base = f3(b.x, b.y, b.z);
         } else if (m.flags & kMaterialUsesPtex) {
             uint32_t pstatus = 0;
+            base = ld3(m.base_color);
             ptex_eval(static_cast<const PtexFace*>(hr.ptex_faces), int(hr.ptex_count),
                       static_cast<const __half*>(hr.ptex_texels), int(m.ptex_base + __float_as_uint(p0.w)), hit.y,
                       hit.z, base, pstatus);
             status |= pstatus;
+            base = pow3(base, 2.2f);
         } else {
-            base = tex2d_base_colour(m, attr, __float_as_uint(p0.w), hit.y, hit.z);
+            base = pow3(tex2d_base_colour(m, attr, __float_as_uint(p0.w), hit.y, hit.z), 2.2f);
         }
     }
     h.view = -dir;
@@ -297,7 +299,7 @@ __device__ void make_vhit(const VcmParams& P, uint32_t s, float3 org, float3 dir
                             : triangle_ng(p0, p1, p2);
     shading_frame(attr, __float_as_uint(p0.w), hit.y, hit.z, ng,
                   [&](float3 x) { return kInst ? world_normal(hr, x) : x; }, fn, ft, fb, h.bsign);
-    h.s = make_surface_frame(m, ft, fn, fb, h.view, pow3(base, 2.2f));
+    h.s = make_surface_frame(m, ft, fn, fb, h.view, base);
     h.n = h.s.n;
     h.cont = continuation_probability(h.s);
     h.mat = &m;
@@ -757,6 +759,7 @@ __global__ void __launch_bounds__(kBlock) k_vtexture(VcmParams P, int cur, const
             base = tex2d_base_colour(m, geom < hr.attr_count ? hr.attrs + geom : nullptr, __float_as_uint(p0.w), hit.y,
                                      hit.z);
         }
+        base = pow3(base, 2.2f);
         P.st.base[s] = make_float4(base.x, base.y, base.z, 0.0f);
     }
     if (status) atomicOr(P.err, status);

@@ -48,7 +48,7 @@ struct VcmState {
     uint32_t* queue[2];   // live path slots, ping-pong between bounces
     uint32_t* queue_sorted;  // the current queue ordered by material class (counting sort)
     uint32_t* cls;        // material class of each current queue entry
-    float4* base;         // Ptex base colour (authored) of the path's current hit, filtered before shading
+    float4* base;         // textured base colour (linear) of the path's current hit, filtered before shading
     // shadow queue: light tracing, next-event and connection segments with their contributions
     float4* so;           // origin, tnear
     float4* sd;           // direction, tfar
