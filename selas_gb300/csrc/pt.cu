@@ -456,14 +456,19 @@ __global__ void __launch_bounds__(kBlock) k_texture(PtParams P, int cur, const u
 
 // kModes: bit 0 path-tracer jobs, bit 1 deferred jobs in the batch (a single-mode batch compiles the other
 // integrator out of the kernel).
-// The path tracer's shading at most 96 registers (5 blocks per SM; a few bytes spill): 2 % faster renders of the
-// room than 102 registers.  The deferred and mixed forms keep 4 blocks per SM (their bigger code would spill).
 // kShader: the shader of every hit the kernel shades (-1: any).  classes = (c0, c1): the kernel shades the
 // entries of material classes c0..c1 of the class-ordered queue (class counts in counters[32 + c]); c0 < 0: the
 // whole queue.
+// Bound by instruction fetches and latency (see even_step): one block per SM, its warps in step.  The frame, base
+// colour and material address are held from stage to stage and the rest of the surface is read again from the
+// material's record, so that little spills.  640 threads at 96 registers against 512 at 128: 1280 x 720 still 21.7 and
+// 22.4 ms, textured room 27.7 and 27.4 ms, deferred sky 5.09 and 5.22 ms; the kernels for any shader spill too much at 96.
+template <uint32_t kModes, int kShader>
+constexpr int kShadeBlock = kModes == 3u || kShader < 0 ? 512 : 640;
+
 template <uint32_t kModes, bool kInst, int kShader>
-__global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams P, int cur, uint32_t bounce,
-                                                                        const uint32_t* in_queue, int2 classes) {
+__global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
+    k_shade(PtParams P, int cur, uint32_t bounce, const uint32_t* in_queue, int2 classes) {
     uint32_t lo = 0, hi = P.st.counters[cur];
     if (classes.x >= 0) {
         uint32_t before = 0, upto = 0;
@@ -476,31 +481,31 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
         hi = upto;
     }
     const int next = cur ^ 1;
-    for (uint32_t base = lo + blockIdx.x * blockDim.x; base < hi; base += gridDim.x * blockDim.x) {
+    const uint32_t step = even_step(hi - lo);
+    for (uint32_t base = lo + blockIdx.x * step; base < hi; base += gridDim.x * step) {
         const uint32_t e = base + threadIdx.x;
-        const bool valid = e < hi;
-        bool cont = false, shadow = false, shadow2 = false;
-        uint32_t s = 0;
-        float4 sh_o = make_float4(0, 0, 0, 0), sh_d = sh_o, sh_c = sh_o;
-        float4 sh2_o = sh_o, sh2_d = sh_o, sh2_c = sh_o;  // deferred: the background's shadow ray
+        const bool valid = threadIdx.x < step && e < hi;
+        uint32_t s = 0, job = 0, pixel = 0, light_set = 0, tri = 0xffffffffu;
+        float3 d = f3(0.0f), thr = d, pos = d, fn = d, ft = d, fb = d, base_color = d;
+        const MaterialDev* mat = nullptr;
+        float specular = 0.0f, ray_distance = 0.0f, err = 0.0f;
+        Pcg32 rng;
+        __syncthreads();
         if (valid) {
             s = in_queue[e];
-            const uint32_t job = P.st.job[s];
-            const PtJob& J = P.st.jobs[job];
-            const PtScene& S = J.scene;
-            const uint32_t npix = J.cam.width * J.cam.height;
-            const bool deferred = kModes == 2u || (kModes == 3u && J.mode == kPtModeDeferred);
+            job = P.st.job[s];
+            const PtScene& S = P.st.jobs[job].scene;
             const float4 o4 = P.st.ray_o[s], d4 = P.st.ray_d[s];
-            const float3 o = f3(o4.x, o4.y, o4.z), d = f3(d4.x, d4.y, d4.z);
-            float4 thr4 = P.st.thr[s];
-            float3 thr = f3(thr4.x, thr4.y, thr4.z);
-            float4 med = P.st.medium[s];
+            const float3 o = f3(o4.x, o4.y, o4.z);
+            d = f3(d4.x, d4.y, d4.z);
+            const float4 thr4 = P.st.thr[s], med = P.st.medium[s];
+            thr = f3(thr4.x, thr4.y, thr4.z);
+            specular = thr4.w;
             const float4 hit = P.st.hit[s];
-            const uint32_t tri = __float_as_uint(hit.w);
-            const uint32_t pixel = P.st.pixel[s];
-            Pcg32 rng = load_rng(P.st, s);
-            float ray_distance = hit.x;
-            float3 pos = f3(0.0f);
+            tri = __float_as_uint(hit.w);
+            pixel = P.st.pixel[s];
+            rng = load_rng(P.st, s);
+            ray_distance = hit.x;
             if (tri != 0xffffffffu) {
                 pos = f3(o.x + hit.x * d.x, o.y + hit.x * d.y, o.z + hit.x * d.z);
                 ray_distance = length(pos - o);
@@ -508,100 +513,100 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
             if (med.x != 0.0f) {  // Isotropic::Transmission
                 thr = thr * f3(expf(-med.y * ray_distance), expf(-med.z * ray_distance), expf(-med.w * ray_distance));
             }
-            bool alive = true;
             if (tri != 0xffffffffu) {
                 const HitRef hr = hit_ref<kInst>(P.st, S, s, tri);
                 const float4 p0 = __ldg(hr.tp), p1 = __ldg(hr.tp + 1), p2 = __ldg(hr.tp + 2);
                 const uint32_t geom = __float_as_uint(p1.w);
-                const MaterialDev& m = hr.mats[geom < hr.mat_count ? geom : 0];
+                mat = hr.mats + (geom < hr.mat_count ? geom : 0);
                 const MeshAttrDev* attr = geom < hr.attr_count ? hr.attrs + geom : nullptr;
-                float3 fn, ft, fb;
                 float fsign;
                 const float3 ng = kInst ? record_ng(hr.tp, p0, p1, p2, hr.rec0, hr.rec1, o, d, hit.x, hit.y)
                                         : triangle_ng(p0, p1, p2);
                 shading_frame(attr, __float_as_uint(p0.w), hit.y, hit.z, ng,
                               [&](float3 x) { return kInst ? world_normal(hr, x) : x; }, fn, ft, fb, fsign);
                 // RayPick error bound (PathTracer.cpp:134-136)
-                const float err = 32.0f * 1.19209e-07f *
-                                  fmaxf(fmaxf(fabsf(pos.x), fabsf(pos.y)), fmaxf(fabsf(pos.z), hit.x));
-                float3 base = ld3(m.base_linear);
-                if (m.flags & kMaterialTextured) {  // filtered or sampled by k_texture for this hit
+                err = 32.0f * 1.19209e-07f * fmaxf(fmaxf(fabsf(pos.x), fabsf(pos.y)), fmaxf(fabsf(pos.z), hit.x));
+                base_color = ld3(mat->base_linear);
+                if (mat->flags & kMaterialTextured) {  // filtered or sampled by k_texture for this hit
                     const float4 b = P.st.base[s];
-                    base = f3(b.x, b.y, b.z);
+                    base_color = f3(b.x, b.y, b.z);
                 }
-                const Surface sf = make_surface_frame(m, ft, fn, fb, -d, base);
-                // Next-event estimation to the surface's light set (AreaLighting.cpp:353-373)
-                LightSample ls;
-                ls.radiance = f3(0.0f);
-                if (m.light_set < S.light_set_count) {
-                    const uint2 set = S.light_sets[m.light_set];
-                    if (set.y > 0) {
-                        const float p0u = pcg_float(rng);
-                        uint32_t li = uint32_t(p0u * float(set.y));
-                        li = li < set.y ? li : set.y - 1;
-                        const float u = pcg_float(rng), v = pcg_float(rng);
-                        sample_quad_light(S.lights[set.x + li], pos, sf.n, u, v, ls);
-                        ls.pdf *= 1.0f / float(set.y);
-                    }
+                light_set = mat->light_set;
+            }
+        }
+        const PtJob& J = P.st.jobs[job];
+        const PtScene& S = J.scene;
+        const bool on_surface = tri != 0xffffffffu;
+        const bool deferred = kModes == 2u || (kModes == 3u && J.mode == kPtModeDeferred);
+        // Next-event estimation: to the surface's light set (AreaLighting.cpp:353-373), then, deferred, to the
+        // background; the segments with a contribution are queued (at most 2 records per path).
+#pragma unroll 1
+        for (int pass = 0; pass < ((kModes & 2u) ? 2 : 1); ++pass) {
+            LightSample ls;
+            ls.radiance = f3(0.0f);
+            if (on_surface && pass == 0 && light_set < S.light_set_count) {
+                const uint2 set = S.light_sets[light_set];
+                if (set.y > 0) {
+                    const float p0u = pcg_float(rng);
+                    uint32_t li = uint32_t(p0u * float(set.y));
+                    li = li < set.y ? li : set.y - 1;
+                    const float u = pcg_float(rng), v = pcg_float(rng);
+                    sample_quad_light(S.lights[set.x + li], pos, fn, u, v, ls);
+                    ls.pdf *= 1.0f / float(set.y);
                 }
-                const uint32_t tag = (job << 28) | pixel;
-                if (dot(ls.radiance, f3(1.0f)) > 0.0f) {
-                    float fpdf, rpdf;
-                    const float3 refl = bsdf_evaluate_as<kShader>(sf, -d, ls.direction, fpdf, rpdf);
-                    if (deferred) {
-                        // weight 1 (DeferredPathTracer.cpp:65-88); the shadow ray starts at tnear 0
-                        const float3 smp = 1.0f * refl * ls.radiance * (1.0f / ls.pdf);
-                        if (dot(smp, f3(1.0f)) > 0.0f) {
-                            const float3 so = offset_origin(pos, sf.n, err, ls.direction, 0.1f);
-                            const float3 c = smp * thr;
-                            sh_o = make_float4(so.x, so.y, so.z, 0.0f);
-                            sh_d = make_float4(ls.direction.x, ls.direction.y, ls.direction.z, ls.distance);
-                            sh_c = make_float4(c.x, c.y, c.z, __uint_as_float(tag));
-                            shadow = true;
-                        }
-                    } else if (dot(refl, f3(1.0f)) > 0.0f) {
-                        // OcclusionRay (PathTracer.cpp:71-92): origin offset 0.1 * error, tnear = error
-                        const float3 so = offset_origin(pos, sf.n, err, ls.direction, 0.1f);
-                        const float3 c = refl * ls.radiance * (1.0f / ls.pdf) * thr;
-                        sh_o = make_float4(so.x, so.y, so.z, err);
-                        sh_d = make_float4(ls.direction.x, ls.direction.y, ls.direction.z, ls.distance);
-                        sh_c = make_float4(c.x, c.y, c.z, __uint_as_float(tag));
-                        shadow = true;
-                    }
+            }
+            if ((kModes & 2u) && on_surface && pass == 1 && deferred) {
+                // SampleBackground (AreaLighting.cpp:393-401): with an image DirectIblLightSample (:293-314),
+                // else BackgroundLightSample (:334-350), a uniform sphere direction whose density is recorded
+                // as 1; at distance 1e36
+                const float r0 = pcg_float(rng), r1 = pcg_float(rng);
+                ls.distance = 1e36f;
+                if (S.ibl) {
+                    ibl_sample(*S.ibl, r0, r1, ls.direction, ls.radiance, ls.pdf);
+                } else {
+                    const float uu = 2.0f * r1 - 1.0f;
+                    const float nn = sqrtf(fmaxf(0.0f, 1.0f - uu * uu));
+                    const float th = kTwoPi * r0;
+                    ls.direction = f3(nn * cosf(th), uu, nn * sinf(th));
+                    ls.radiance = f3(S.background[0], S.background[1], S.background[2]);
+                    ls.pdf = 1.0f;
                 }
-                if (deferred) {
-                    // SampleBackground (AreaLighting.cpp:393-401): with an image DirectIblLightSample (:293-314),
-                    // else BackgroundLightSample (:334-350), a uniform sphere direction whose density is recorded
-                    // as 1; at distance 1e36; balance heuristic against the BSDF's density
-                    // (DeferredPathTracer.cpp:90-111)
-                    const float r0 = pcg_float(rng), r1 = pcg_float(rng);
-                    float3 sdir, bg;
-                    float spdf;
-                    if (S.ibl) {
-                        ibl_sample(*S.ibl, r0, r1, sdir, bg, spdf);
-                    } else {
-                        const float uu = 2.0f * r1 - 1.0f;
-                        const float nn = sqrtf(fmaxf(0.0f, 1.0f - uu * uu));
-                        const float th = kTwoPi * r0;
-                        sdir = f3(nn * cosf(th), uu, nn * sinf(th));
-                        bg = f3(S.background[0], S.background[1], S.background[2]);
-                        spdf = 1.0f;
-                    }
-                    if (dot(bg, f3(1.0f)) > 0.0f) {
-                        float fpdf, rpdf;
-                        const float3 refl = bsdf_evaluate_as<kShader>(sf, -d, sdir, fpdf, rpdf);
-                        const float mis = (1.0f * spdf) / (1.0f * spdf + 1.0f * fpdf);
-                        const float3 smp = mis * refl * bg * (1.0f / spdf);
-                        if (dot(smp, f3(1.0f)) > 0.0f) {
-                            const float3 so = offset_origin(pos, sf.n, err, sdir, 0.1f);
-                            const float3 c = smp * thr;
-                            sh2_o = make_float4(so.x, so.y, so.z, 0.0f);
-                            sh2_d = make_float4(sdir.x, sdir.y, sdir.z, 1e36f);
-                            sh2_c = make_float4(c.x, c.y, c.z, __uint_as_float(tag));
-                            shadow2 = true;
-                        }
-                    }
+            }
+            __syncthreads();
+            bool shadow = false;
+            float4 sh_o = make_float4(0, 0, 0, 0), sh_d = sh_o, sh_c = sh_o;
+            if (on_surface && dot(ls.radiance, f3(1.0f)) > 0.0f) {
+                float fpdf, rpdf;
+                const Surface sf = make_surface_frame(*mat, ft, fn, fb, -d, base_color);
+                const float3 refl = bsdf_evaluate_as<kShader>(sf, -d, ls.direction, fpdf, rpdf);
+                // path tracer: OcclusionRay (PathTracer.cpp:71-92), tnear = error.  Deferred: a light weighs 1
+                // (DeferredPathTracer.cpp:65-88), the background by the balance heuristic against the BSDF's density
+                // (:90-111); tnear 0.  Both: origin offset 0.1 * error
+                const float weight = pass == 1 ? (1.0f * ls.pdf) / (1.0f * ls.pdf + 1.0f * fpdf) : 1.0f;
+                const float3 smp = weight * refl * ls.radiance * (1.0f / ls.pdf);
+                if (dot(deferred ? smp : refl, f3(1.0f)) > 0.0f) {
+                    const float3 so = offset_origin(pos, fn, err, ls.direction, 0.1f);
+                    const float3 c = smp * thr;
+                    sh_o = make_float4(so.x, so.y, so.z, deferred ? 0.0f : err);
+                    sh_d = make_float4(ls.direction.x, ls.direction.y, ls.direction.z, ls.distance);
+                    sh_c = make_float4(c.x, c.y, c.z, __uint_as_float((job << 28) | pixel));
+                    shadow = true;
                 }
+            }
+            const uint32_t sslot = warp_append(&P.st.counters[2], shadow);
+            if (shadow) {
+                P.st.sh_o[sslot] = sh_o;
+                P.st.sh_d[sslot] = sh_d;
+                P.st.sh_c[sslot] = sh_c;
+            }
+        }
+        __syncthreads();
+        bool cont = false;
+        if (valid) {
+            const uint32_t npix = J.cam.width * J.cam.height;
+            float4 med = P.st.medium[s];
+            bool alive = true;
+            if (on_surface) {
                 // BSDF sampling: draw ahead, then keep the stream's state after the draws that were used (every shader
                 // uses at least one)
                 float u4[4];
@@ -612,6 +617,7 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
                 }
                 int used = 0;
                 BsdfSampleOut bs;
+                const Surface sf = make_surface_frame(*mat, ft, fn, fb, -d, base_color);
                 const bool ok = bsdf_sample_as<kShader>(sf, -d, u4, used, bs);
                 rng.state = used <= 1 ? state[0] : (used == 2 ? state[1] : (used == 3 ? state[2] : state[3]));
                 if (!ok) {
@@ -621,31 +627,32 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
                     // 404-413: the image's density, else 1 / (4 pi))
                     const float sky_pdf = S.ibl ? ibl_pdf(*S.ibl, bs.wi) : kInv4Pi;
                     const float mis = (1.0f * bs.forward_pdf) / (1.0f * bs.forward_pdf + 1.0f * sky_pdf);
-                    if (!(bs.flags & kDiracEvent)) thr4.w = 0.0f;  // diracScatterOnly
+                    if (!(bs.flags & kDiracEvent)) specular = 0.0f;  // diracScatterOnly
                     const float3 t = mis * thr * bs.reflectance;
                     if (dot(t, t) == 0.0f) {
                         alive = false;
                     } else {
                         thr = t;
-                        const float3 no = offset_origin(pos, sf.n, err, bs.wi, 1.0f);
+                        const float3 no = offset_origin(pos, fn, err, bs.wi, 1.0f);
                         P.st.ray_o[s] = make_float4(no.x, no.y, no.z, 0.0f);
                         P.st.ray_d[s] = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, kFloatMax);
                     }
                 } else {
-                    if (!(bs.flags & kDiracEvent)) thr4.w = 0.0f;
+                    if (!(bs.flags & kDiracEvent)) specular = 0.0f;
                     if (bs.flags == kTransmissionEvent) {
                         if (med.x == 0.0f) med = make_float4(float(bs.medium_phase), bs.extinction.x, bs.extinction.y, bs.extinction.z);
                         else med = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
                     thr = 1.0f * thr * bs.reflectance;
-                    const float3 no = offset_origin(pos, sf.n, err, bs.wi, 1.0f);
+                    const float3 no = offset_origin(pos, fn, err, bs.wi, 1.0f);
                     P.st.ray_o[s] = make_float4(no.x, no.y, no.z, 0.0f);
                     P.st.ray_d[s] = make_float4(bs.wi.x, bs.wi.y, bs.wi.z, kFloatMax);
                     if (bounce == 0) accumulate(J.accum, npix, 0, pixel, bs.reflectance);
                 }
             } else if (!deferred && med.x != 0.0f) {
                 // scatter inside the medium: Isotropic::SampleScatterDirection -> CSampler::UniformSphere
-                const float3 no = o + ray_distance * d;
+                const float4 o4 = P.st.ray_o[s];
+                const float3 no = f3(o4.x, o4.y, o4.z) + ray_distance * d;
                 const float r0 = pcg_float(rng), r1 = pcg_float(rng);
                 const float uu = 2.0f * r1 - 1.0f;
                 const float nn = sqrtf(fmaxf(0.0f, 1.0f - uu * uu));
@@ -657,7 +664,7 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
                 // miss: EvaluateBackgroundMiss for a camera ray or a pure specular chain, else EvaluateBackground
                 // (AreaLighting.cpp:415-436): the image's miss / light texel, or the uniform background
                 float3 bg = f3(S.background[0], S.background[1], S.background[2]);
-                if (S.ibl) bg = thr4.w != 0.0f ? ibl_miss(*S.ibl, d) : ibl_radiance(*S.ibl, d);
+                if (S.ibl) bg = specular != 0.0f ? ibl_miss(*S.ibl, d) : ibl_radiance(*S.ibl, d);
                 accumulate(J.accum, npix, deferred ? 0 : 1, pixel, bg * thr);
                 alive = false;
             }
@@ -676,26 +683,12 @@ __global__ void __launch_bounds__(kBlock, kModes == 1u ? 5 : 4) k_shade(PtParams
                 }
                 cont = alive && nb < J.max_bounces;
             }
-            P.st.thr[s] = make_float4(thr.x, thr.y, thr.z, thr4.w);
+            P.st.thr[s] = make_float4(thr.x, thr.y, thr.z, specular);
             P.st.medium[s] = med;
             P.st.rng[s] = rng.state;
         }
         const uint32_t qslot = warp_append(&P.st.counters[next], cont);
         if (cont) P.st.queue[next][qslot] = s;
-        const uint32_t sslot = warp_append(&P.st.counters[2], shadow);
-        if (shadow) {
-            P.st.sh_o[sslot] = sh_o;
-            P.st.sh_d[sslot] = sh_d;
-            P.st.sh_c[sslot] = sh_c;
-        }
-        if ((kModes & 2u) && __any_sync(0xffffffffu, shadow2)) {  // the queue holds 2 records per path
-            const uint32_t s2 = warp_append(&P.st.counters[2], shadow2);
-            if (shadow2) {
-                P.st.sh_o[s2] = sh2_o;
-                P.st.sh_d[s2] = sh2_d;
-                P.st.sh_c[s2] = sh2_c;
-            }
-        }
     }
 }
 
@@ -867,15 +860,15 @@ void launch_shade_modes(int shader, int grid, cudaStream_t s, const PtParams& P,
                         const uint32_t* q, int2 classes) {
     if constexpr (kModes != 3u) {
         if (shader == 1) {
-            k_shade<kModes, kInst, 1><<<grid, kBlock, 0, s>>>(P, cur, b, q, classes);
+            k_shade<kModes, kInst, 1><<<grid, kShadeBlock<kModes, 1>, 0, s>>>(P, cur, b, q, classes);
             return;
         }
         if (shader == 2) {
-            k_shade<kModes, kInst, 2><<<grid, kBlock, 0, s>>>(P, cur, b, q, classes);
+            k_shade<kModes, kInst, 2><<<grid, kShadeBlock<kModes, 2>, 0, s>>>(P, cur, b, q, classes);
             return;
         }
     }
-    k_shade<kModes, kInst, -1><<<grid, kBlock, 0, s>>>(P, cur, b, q, classes);
+    k_shade<kModes, kInst, -1><<<grid, kShadeBlock<kModes, -1>, 0, s>>>(P, cur, b, q, classes);
 }
 
 void launch_shade(uint32_t modes, bool inst, int shader, int grid, cudaStream_t s, const PtParams& P, int cur,
@@ -952,23 +945,12 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
     };
     const int shade_grid = grid_for(sms, 8);
     const int gen_grid = int((st.capacity + kBlock - 1) / kBlock);
-    // the shading kernel (4 or 5 resident blocks per SM) runs one resident wave of grid-striding blocks, sized by
-    // the occupancy calculator, as VCM's shading kernels do
-    const void* shade_fn = instanced ? (modes == 2u ? reinterpret_cast<const void*>(&k_shade<2, true, -1>)
-                                        : modes == 3u ? reinterpret_cast<const void*>(&k_shade<3, true, -1>)
-                                                      : reinterpret_cast<const void*>(&k_shade<1, true, -1>))
-                                     : (modes == 2u ? reinterpret_cast<const void*>(&k_shade<2, false, -1>)
-                                        : modes == 3u ? reinterpret_cast<const void*>(&k_shade<3, false, -1>)
-                                                      : reinterpret_cast<const void*>(&k_shade<1, false, -1>));
     // shading launches: one kernel for the jobs' single shader over the whole queue; with several shaders and the
     // class order, one per shader over its classes (1 + shader * 4 .. 4 + shader * 4; the misses, class 0, with
     // the thin shader's); else the kernel for every shader
     const uint32_t kinds = shader_kinds & 7u;
     const bool one_kind = kinds != 0u && (kinds & (kinds - 1u)) == 0u;
     const int single = one_kind ? __builtin_ctz(kinds) : -1;
-    int shade_blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&shade_blocks, shade_fn, kBlock, 0);
-    const int wave_grid = sms * std::max(shade_blocks, 1);
     auto enqueue = [&](cudaStream_t s) {
         k_batch_begin<<<1, 32, 0, s>>>(P);
         k_generate<<<gen_grid, kBlock, 0, s>>>(P);
@@ -1015,13 +997,13 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
             else if (texture) k_texture<false, false><<<shade_grid, kBlock, 0, s>>>(P, cur, q);
             const int2 whole = make_int2(-1, -1);
             if (one_kind) {
-                launch_shade(modes, instanced, single, wave_grid, s, P, cur, b, q, whole);
+                launch_shade(modes, instanced, single, sms, s, P, cur, b, q, whole);
             } else if (sort) {
-                launch_shade(modes, instanced, -1, wave_grid, s, P, cur, b, q, make_int2(0, 4));
-                if (kinds & 2u) launch_shade(modes, instanced, 1, wave_grid, s, P, cur, b, q, make_int2(5, 8));
-                if (kinds & 4u) launch_shade(modes, instanced, 2, wave_grid, s, P, cur, b, q, make_int2(9, 12));
+                launch_shade(modes, instanced, -1, sms, s, P, cur, b, q, make_int2(0, 4));
+                if (kinds & 2u) launch_shade(modes, instanced, 1, sms, s, P, cur, b, q, make_int2(5, 8));
+                if (kinds & 4u) launch_shade(modes, instanced, 2, sms, s, P, cur, b, q, make_int2(9, 12));
             } else {
-                launch_shade(modes, instanced, -1, wave_grid, s, P, cur, b, q, whole);
+                launch_shade(modes, instanced, -1, sms, s, P, cur, b, q, whole);
             }
             shadow(s);
             if (ray_sort && b + 1 < bounces) {

@@ -34,7 +34,8 @@ struct MaterialDev {
     float base_linear[3];                    // base_color to the power 2.2
     float alpha_x, alpha_y;                  // the microfacet widths
     float p_spec, p_diff, p_coat, p_trans;   // the lobes' sampling probabilities
-    float pad[4];
+    float inverse_ior;
+    float pad[3];
 };
 static_assert(sizeof(MaterialDev) == 160, "MaterialDev must be 160 bytes");
 

@@ -44,6 +44,8 @@ namespace sel {
 namespace {
 
 constexpr int kBlock = 128;
+constexpr int kVertexBlock = 512;   // one block per SM, at up to 128 registers
+constexpr int kConnectBlock = 640;  // the same at up to 96
 constexpr float kFloatMax = 3.402823466e+38f;
 constexpr int kBoundsBlocks = 256;
 
@@ -597,20 +599,23 @@ __global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_shadow(const __g
 // Light sub-path vertices (EvaluateLightPaths, VCM.cpp:502-561): MIS update, stored vertex, connection to
 // the camera (ConnectLightPathToCamera, VCM.cpp:190-233; tech report sec. 5.3) and scattering.
 template <bool kSorted, bool kInst>
-__global__ void __launch_bounds__(kBlock) k_l_shade(VcmParams P, int cur, const uint32_t* in_queue) {
+__global__ void __launch_bounds__(kVertexBlock, 1) k_l_shade(VcmParams P, int cur, const uint32_t* in_queue) {
     const VcmConsts c = P.st.consts[*P.st.iter];
     const uint32_t n = P.st.counters[cur];
     const uint32_t N = P.npaths;
     const int next = cur ^ 1;
     uint32_t status = 0;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const uint32_t step = even_step(n);
+    for (uint32_t base = blockIdx.x * step; base < n; base += gridDim.x * step) {
         const uint32_t e = base + threadIdx.x;
+        const bool valid = threadIdx.x < step && e < n;
+        __syncthreads();
         bool cont = false, shadow = false;
         uint32_t s = 0, pixel = 0;
         VHit h;
         float3 to_cam = f3(0.0f), contrib = f3(0.0f);
         float sh_tfar = 0.0f;
-        if (e < n) {
+        if (valid) {
             s = in_queue[e];
             const float4 hit = P.st.phit[s];
             if (__float_as_uint(hit.w) != 0xffffffffu) {
@@ -898,14 +903,17 @@ __device__ __forceinline__ CameraVertex load_camera_vertex(const float4* v) {
 }
 
 template <bool kSorted, bool kInst>
-__global__ void __launch_bounds__(kBlock) k_c_shade(VcmParams P, int cur, const uint32_t* in_queue) {
+__global__ void __launch_bounds__(kVertexBlock, 1) k_c_shade(VcmParams P, int cur, const uint32_t* in_queue) {
     const VcmConsts c = P.st.consts[*P.st.iter];
     const uint32_t n = P.st.counters[cur];
     const uint32_t N = P.npaths;
     const int next = cur ^ 1;
     uint32_t status = 0;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const uint32_t step = even_step(n);
+    for (uint32_t base = blockIdx.x * step; base < n; base += gridDim.x * step) {
         const uint32_t e = base + threadIdx.x;
+        const bool valid = threadIdx.x < step && e < n;
+        __syncthreads();
         bool cont = false, hit_ok = false, nee_ray = false, record = false;
         uint32_t s = 0, nvc = 0;
         VHit h;
@@ -915,7 +923,7 @@ __global__ void __launch_bounds__(kBlock) k_c_shade(VcmParams P, int cur, const 
         rng.inc = 1;
         float3 to_l = f3(0.0f), contrib = f3(0.0f);
         float tfar = 0.0f;
-        if (e < n) {
+        if (valid) {
             s = in_queue[e];
             const float4 hit = P.st.phit[s];
             if (__float_as_uint(hit.w) != 0xffffffffu) {
@@ -1042,17 +1050,20 @@ __global__ void __launch_bounds__(kBlock) k_c_shade(VcmParams P, int cur, const 
 // One thread per (camera vertex, light vertex) pair: ConnectPathVertices (VCM.cpp:293-359), with the light
 // side oriented f(v = toward the camera vertex, l = toward the previous light vertex) and the cosine at the
 // connection carried.
-__global__ void __launch_bounds__(kBlock) k_c_connect(VcmParams P) {
+__global__ void __launch_bounds__(kConnectBlock, 1) k_c_connect(VcmParams P) {
     const VcmConsts c = P.st.consts[*P.st.iter];
     const uint32_t n = P.st.counters[6];
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const uint32_t step = even_step(n);
+    for (uint32_t base = blockIdx.x * step; base < n; base += gridDim.x * step) {
         const uint32_t e = base + threadIdx.x;
+        const bool valid = threadIdx.x < step && e < n;
+        __syncthreads();
         bool ray = false;
         float3 dir = f3(0.0f), contrib = f3(0.0f);
         float tfar = 0.0f;
         CameraVertex cv;
         cv.pixel = 0;
-        if (e < n) {
+        if (valid) {
             const uint2 pr = P.st.pairs[e];
             cv = load_camera_vertex(P.st.cverts + size_t(pr.x) * kCamF4);
             const LightVertex lv = load_vertex(P.st.verts + (size_t(cv.pixel) * P.slots + pr.y) * kVertF4);
@@ -1418,15 +1429,6 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
     const bool sort = sc.sort_hint != 0 || inst;
     const bool quads = sc.ptex_quads != 0;
     const bool pretex = sort || quads;
-    const void* l_fn = inst ? reinterpret_cast<const void*>(&k_l_shade<true, true>)
-                            : pretex ? reinterpret_cast<const void*>(&k_l_shade<true, false>)
-                                     : reinterpret_cast<const void*>(&k_l_shade<false, false>);
-    const void* c_fn = inst ? reinterpret_cast<const void*>(&k_c_shade<true, true>)
-                            : pretex ? reinterpret_cast<const void*>(&k_c_shade<true, false>)
-                                     : reinterpret_cast<const void*>(&k_c_shade<false, false>);
-    const int l_grid = wave(l_fn);
-    const int c_grid = wave(c_fn);
-    const int connect_grid = wave(reinterpret_cast<const void*>(&k_c_connect));
     const int merge_grid = wave(reinterpret_cast<const void*>(&k_c_merge));
     // material-class sort and Ptex of a bounce's hits; returns the queue the shading kernel reads
     auto sort_hits = [&](cudaStream_t stream, int cur) -> const uint32_t* {
@@ -1456,9 +1458,9 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
             k_bounce_reset<<<1, 32, 0, stream>>>(st.counters, cur ^ 1);
             extend(stream, cur);
             const uint32_t* q = sort_hits(stream, cur);
-            if (inst) k_l_shade<true, true><<<l_grid, kBlock, 0, stream>>>(P, cur, q);
-            else if (pretex) k_l_shade<true, false><<<l_grid, kBlock, 0, stream>>>(P, cur, q);
-            else k_l_shade<false, false><<<l_grid, kBlock, 0, stream>>>(P, cur, q);
+            if (inst) k_l_shade<true, true><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
+            else if (pretex) k_l_shade<true, false><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
+            else k_l_shade<false, false><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
             shadow(stream);
         }
         // hash grid over the stored vertices
@@ -1485,10 +1487,10 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
             k_bounce_reset<<<1, 32, 0, stream>>>(st.counters, cur ^ 1);
             extend(stream, cur);
             const uint32_t* q = sort_hits(stream, cur);
-            if (inst) k_c_shade<true, true><<<c_grid, kBlock, 0, stream>>>(P, cur, q);
-            else if (pretex) k_c_shade<true, false><<<c_grid, kBlock, 0, stream>>>(P, cur, q);
-            else k_c_shade<false, false><<<c_grid, kBlock, 0, stream>>>(P, cur, q);
-            k_c_connect<<<connect_grid, kBlock, 0, stream>>>(P);
+            if (inst) k_c_shade<true, true><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
+            else if (pretex) k_c_shade<true, false><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
+            else k_c_shade<false, false><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
+            k_c_connect<<<sms, kConnectBlock, 0, stream>>>(P);
             k_c_merge<<<merge_grid, kBlock, 0, stream>>>(P);
             shadow(stream);
         }

@@ -1,8 +1,14 @@
-"""The Disney Fresnel term of a surface with metallic 0 ends at its dielectric part without running the Schlick part.
+"""Shading kernels: what they skip and how they split a queue.
+
+The Disney Fresnel term of a surface with metallic 0 ends at its dielectric part without running the Schlick part.
 
 A denormal metallic runs the whole interpolation, (1 - m) * fd + m * fm, and rounds to the same floats as metallic 0:
 1 - m is 1 and m * fm is far below half an ulp of fd, which is at least 1e-3 for the indices used here.  So both must
 agree bit for bit, in every evaluation and sample.
+
+One block of 512 or 640 threads per SM steps through the queue, all blocks with equally many entries a step (a multiple
+of 32).  However a batch falls into blocks and steps, its paths are the same: only the order of the FP64 additions to a
+pixel differs (about 1e-15 relative each), so images agree to one rounding of the result to FP32, 2^-23.
 """
 from pathlib import Path
 
@@ -46,3 +52,23 @@ def test_metallic_zero_equals_denormal_metallic(base, tint):
             surf[:, METALLIC] = metallic
             got.append(_run(name, surf, golden[f"wo_{kind}"], golden[second], width))
         assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
+
+
+# batches around one warp, around the wave of 512- and 640-thread blocks on 152 SMs, and two steps with a remainder
+@pytest.mark.gpu
+@pytest.mark.parametrize("size,batch", [((9, 7), 1), ((9, 7), 31), ((9, 7), 33), ((400, 250), 77823), ((400, 250), 77825),
+                                        ((400, 250), 97279), ((400, 250), 97281)])
+def test_batches_of_any_size_give_one_image(device, size, batch):
+    import selas_gb300 as sel
+    from selas_gb300 import scenes
+    rs = scenes.textured_spheres(count=4, level=3)
+    sc = rs.build(sel, device)
+    cam = rs.sel_camera(sel, *size)
+    imgs = []
+    for paths in (batch, 0):
+        st, df = sel.pt_settings(1, 5, seed=3), sel.deferred_settings(1, 6, seed=3)
+        st.pathsInFlight = df.pathsInFlight = paths
+        imgs.append((sc.pt_generate_image(cam, st), sc.deferred_generate_image(cam, df)))
+    sc.release()
+    for got, want in zip(*imgs):
+        np.testing.assert_allclose(got, want, rtol=2.0 ** -22, atol=1e-12)
