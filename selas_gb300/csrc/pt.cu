@@ -128,15 +128,12 @@ __global__ void k_batch_end(PtParams P) {
     if (threadIdx.x < kMaxPtJobs) c.next[threadIdx.x] += c.count[threadIdx.x];
 }
 
-__global__ void k_bounce_reset(uint32_t* counters, int next) {
-    // next queue length, shadow queue length and both fetch cursors restart each bounce
-    if (threadIdx.x == 0) {
-        counters[next] = 0u;
-        counters[2] = 0u;
-        counters[3] = 0u;
-        counters[4] = 0u;
-    }
+// The next bounce's queue length, its shadow queue's and both fetch cursors restart once the bounce is traced: by the
+// kernel that follows the tracing.
+__device__ __forceinline__ void bounce_reset(uint32_t* counters, int cur) {
+    if (threadIdx.x < 4) counters[threadIdx.x == 0 ? cur ^ 1 : threadIdx.x + 1] = 0u;
 }
+__global__ void k_bounce_reset(uint32_t* counters, int cur) { bounce_reset(counters, cur); }
 
 __global__ void __launch_bounds__(kBlock) k_generate(PtParams P) {
     const PtControl& c = *P.st.control;
@@ -277,13 +274,11 @@ template <int K, int B>
 constexpr int kTraceBlocksPerSm = (K == 2 ? 512 : 1024) / B;
 
 template <int K, int B, bool kOne>
-__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_extend(const __grid_constant__ PtParams P, int cur) {
+__device__ __forceinline__ void extend_queue(const PtParams& P, int cur, int* binary_stack, uint32_t& status) {
     const uint32_t n = P.st.counters[cur];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays, (unsigned long long)n);
     const uint32_t* queue = P.st.queue[cur];
-    uint32_t status = 0;
     if constexpr (K == 1) {
-        __shared__ int stack_mem[kBinaryStack * B];
         for (;;) {
             uint32_t base = 0;
             if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[3], 32u);
@@ -296,7 +291,7 @@ __global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_extend(const __g
                 const PtScene& sc = P.st.jobs[P.st.job[s]].scene;
                 QueryHit h;
                 const bool found = trace_binary<false>(static_cast<const float4*>(sc.nodes), sc.tris, q, h,
-                                                       stack_mem + threadIdx.x, B, status);
+                                                       binary_stack + threadIdx.x, B, status);
                 P.st.hit[s] = found ? make_float4(h.t, h.u, h.v, __uint_as_float(h.tri))
                                     : make_float4(q.tfar, 0.0f, 0.0f, __uint_as_float(0xffffffffu));
             }
@@ -308,6 +303,77 @@ __global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_extend(const __g
         else if (short_queue(n)) trace_groups<false>(rays, n, stack, status);
         else trace_stream<false, WideWalk>(rays, stack, status);
     }
+}
+
+// The queued shadow rays of the batch.
+template <bool kOne>
+struct ShadowRays : QueueRanges, LaneScene<kOne> {
+    const PtState& st;
+    __device__ __forceinline__ ShadowRays(const PtParams& P, uint32_t n)
+        : QueueRanges(n, &P.st.counters[4]), LaneScene<kOne>(P), st(P.st) {}
+    __device__ __forceinline__ bool begin(uint32_t e, QueryRay& q) {
+        if constexpr (!kOne) this->take(__float_as_uint(st.sh_c[e].w) >> 28);
+        const float4 o = st.sh_o[e], d = st.sh_d[e];
+        q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = o.w;
+        q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = d.w;
+        return true;
+    }
+    __device__ __forceinline__ void add(uint32_t e) const {
+        const float4 c = st.sh_c[e];
+        const uint32_t tag = __float_as_uint(c.w);
+        const PtJob& J = st.jobs[tag >> 28];
+        accumulate(J.accum, J.cam.width * J.cam.height, J.mode == kPtModeDeferred ? 0 : 1, tag & 0x0fffffffu,
+                   f3(c.x, c.y, c.z));
+    }
+    __device__ __forceinline__ void end(uint32_t e, const WideState& h) const {
+        if (h.hit.tri == 0xffffffffu) add(e);
+    }
+    __device__ __forceinline__ void end(uint32_t e, const InstState& h) const {
+        if (h.hit.tri == 0xffffffffu) add(e);
+    }
+};
+
+template <int K, int B, bool kOne>
+__device__ __forceinline__ void shadow_queue(const PtParams& P, int* binary_stack, uint32_t& status) {
+    const uint32_t n = P.st.counters[2];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays + 1, (unsigned long long)n);
+    if constexpr (K == 1) {
+        for (;;) {
+            uint32_t base = 0;
+            if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[4], 32u);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= n) break;
+            const uint32_t e = base + (threadIdx.x & 31u);
+            if (e < n) {
+                ShadowRays<false> rays(P, n);
+                QueryRay q;
+                rays.begin(e, q);
+                QueryHit h;
+                if (!trace_binary<true>(reinterpret_cast<const float4*>(rays.nodes()), rays.tris(), q, h,
+                                        binary_stack + threadIdx.x, B, status))
+                    rays.add(e);
+            }
+        }
+    } else {
+        ShadowRays<kOne> rays(P, n);
+        const WideStack stack{pt_stack + threadIdx.x, B, P.stack_depth};
+        if constexpr (K == 2) trace_stream<true, InstWalk>(rays, stack, status);
+        else if (short_queue(n)) trace_groups<true>(rays, n, stack, status);
+        else trace_stream<true, WideWalk>(rays, stack, status);
+    }
+}
+
+// A bounce's rays: the closest hits of the queued paths (cur < 0: none, after the last bounce), then the shadow rays
+// that the bounce before queued.  One launch for both: warps that find the first queue empty go on with the second, so
+// the SMs idle at the end of one queue a bounce, not two.  It also clears the class counts, which only kernels
+// between two of these launches use.
+template <int K, int B, bool kOne>
+__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_trace(const __grid_constant__ PtParams P, int cur) {
+    __shared__ int binary_stack[K == 1 ? kBinaryStack * B : 1];
+    if (blockIdx.x == 0 && threadIdx.x < 2 * kPtClasses) P.st.counters[32 + threadIdx.x] = 0u;
+    uint32_t status = 0;
+    if (cur >= 0) extend_queue<K, B, kOne>(P, cur, binary_stack, status);
+    shadow_queue<K, B, kOne>(P, binary_stack, status);
     if (status) atomicOr(P.err, status);
 }
 
@@ -328,10 +394,6 @@ __device__ __forceinline__ uint32_t material_class(const PtParams& P, uint32_t s
     return class_of(r.mats[geom < r.mat_count ? geom : 0]);
 }
 
-__global__ void k_class_reset(uint32_t* counters) {
-    if (threadIdx.x < 2 * kPtClasses) counters[32 + threadIdx.x] = 0u;
-}
-
 template <bool kInst>
 __global__ void __launch_bounds__(kBlock) k_classify(PtParams P, int cur) {
     const uint32_t n = P.st.counters[cur];
@@ -346,17 +408,15 @@ __global__ void __launch_bounds__(kBlock) k_classify(PtParams P, int cur) {
     }
 }
 
-__global__ void k_class_offsets(uint32_t* counters) {
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int c = 0; c < kPtClasses; ++c) {
-            counters[48 + c] = run;
-            run += counters[32 + c];
-        }
-    }
-}
-
 __global__ void __launch_bounds__(kBlock) k_class_scatter(PtParams P, int cur) {
+    __shared__ uint32_t first[kPtClasses];  // the classes' places in the sorted queue
+    if (threadIdx.x < kPtClasses) {
+        uint32_t run = 0;
+        for (uint32_t c = 0; c < threadIdx.x; ++c) run += P.st.counters[32 + c];
+        first[threadIdx.x] = run;
+    }
+    if (blockIdx.x == 0) bounce_reset(P.st.counters, cur);
+    __syncthreads();
     const uint32_t n = P.st.counters[cur];
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t e = base + threadIdx.x;
@@ -366,7 +426,7 @@ __global__ void __launch_bounds__(kBlock) k_class_scatter(PtParams P, int cur) {
         const uint32_t lane = threadIdx.x & 31u;
         const int leader = __ffs(peers) - 1;
         uint32_t at = 0;
-        if (valid && leader == int(lane)) at = atomicAdd(&P.st.counters[48 + c], __popc(peers));
+        if (valid && leader == int(lane)) at = first[c] + atomicAdd(&P.st.counters[48 + c], __popc(peers));
         at = __shfl_sync(0xffffffffu, at, leader);
         if (valid) P.st.queue_sorted[at + __popc(peers & ((1u << lane) - 1u))] = P.st.queue[cur][e];
     }
@@ -381,6 +441,7 @@ __global__ void __launch_bounds__(kBlock) k_class_scatter(PtParams P, int cur) {
 // ranges from the counts; a batch with one shader shades the whole queue and needs none).
 template <bool kInst, bool kCount>
 __global__ void __launch_bounds__(kBlock) k_sort_keys(PtParams P, int cur) {
+    if (blockIdx.x == 0) bounce_reset(P.st.counters, cur);
     const uint32_t n = P.st.counters[cur];
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t e = base + threadIdx.x;
@@ -692,67 +753,6 @@ __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
     }
 }
 
-// The queued shadow rays of the batch.
-template <bool kOne>
-struct ShadowRays : QueueRanges, LaneScene<kOne> {
-    const PtState& st;
-    __device__ __forceinline__ ShadowRays(const PtParams& P, uint32_t n)
-        : QueueRanges(n, &P.st.counters[4]), LaneScene<kOne>(P), st(P.st) {}
-    __device__ __forceinline__ bool begin(uint32_t e, QueryRay& q) {
-        if constexpr (!kOne) this->take(__float_as_uint(st.sh_c[e].w) >> 28);
-        const float4 o = st.sh_o[e], d = st.sh_d[e];
-        q.ox = o.x; q.oy = o.y; q.oz = o.z; q.tnear = o.w;
-        q.dx = d.x; q.dy = d.y; q.dz = d.z; q.tfar = d.w;
-        return true;
-    }
-    __device__ __forceinline__ void add(uint32_t e) const {
-        const float4 c = st.sh_c[e];
-        const uint32_t tag = __float_as_uint(c.w);
-        const PtJob& J = st.jobs[tag >> 28];
-        accumulate(J.accum, J.cam.width * J.cam.height, J.mode == kPtModeDeferred ? 0 : 1, tag & 0x0fffffffu,
-                   f3(c.x, c.y, c.z));
-    }
-    __device__ __forceinline__ void end(uint32_t e, const WideState& h) const {
-        if (h.hit.tri == 0xffffffffu) add(e);
-    }
-    __device__ __forceinline__ void end(uint32_t e, const InstState& h) const {
-        if (h.hit.tri == 0xffffffffu) add(e);
-    }
-};
-
-template <int K, int B, bool kOne>
-__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_shadow(const __grid_constant__ PtParams P) {
-    const uint32_t n = P.st.counters[2];
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays + 1, (unsigned long long)n);
-    uint32_t status = 0;
-    if constexpr (K == 1) {
-        __shared__ int stack_mem[kBinaryStack * B];
-        for (;;) {
-            uint32_t base = 0;
-            if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[4], 32u);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base >= n) break;
-            const uint32_t e = base + (threadIdx.x & 31u);
-            if (e < n) {
-                ShadowRays<false> rays(P, n);
-                QueryRay q;
-                rays.begin(e, q);
-                QueryHit h;
-                if (!trace_binary<true>(reinterpret_cast<const float4*>(rays.nodes()), rays.tris(), q, h,
-                                        stack_mem + threadIdx.x, B, status))
-                    rays.add(e);
-            }
-        }
-    } else {
-        ShadowRays<kOne> rays(P, n);
-        const WideStack stack{pt_stack + threadIdx.x, B, P.stack_depth};
-        if constexpr (K == 2) trace_stream<true, InstWalk>(rays, stack, status);
-        else if (short_queue(n)) trace_groups<true>(rays, n, stack, status);
-        else trace_stream<true, WideWalk>(rays, stack, status);
-    }
-    if (status) atomicOr(P.err, status);
-}
-
 // Sort key of a continuing ray (the batcher's order, PathTracingBatcher.cpp:162-258): direction bin (dominant axis
 // x 2 + sign, 3 bits) above a 12-bit Morton code of the origin in the job scene's bounds (4 bits per axis).
 __device__ __forceinline__ uint32_t spread4(uint32_t x) {
@@ -910,10 +910,8 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
     const int tb = (trace_block == 256 && bvh_kind == 0) ? 256 : 128;
     const size_t stack_bytes = bvh_kind == 0 ? size_t(stack_depth) * size_t(tb) * sizeof(uint2) : 0;
     if (stack_bytes > 48u * 1024u) {  // deep instanced scenes with 256-thread blocks
-        for (const void* f : {reinterpret_cast<const void*>(&k_extend<2, 256, true>),
-                              reinterpret_cast<const void*>(&k_extend<2, 256, false>),
-                              reinterpret_cast<const void*>(&k_shadow<2, 256, true>),
-                              reinterpret_cast<const void*>(&k_shadow<2, 256, false>)}) {
+        for (const void* f : {reinterpret_cast<const void*>(&k_trace<2, 256, true>),
+                              reinterpret_cast<const void*>(&k_trace<2, 256, false>)}) {
             const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                        int(kInstStack * 256 * sizeof(uint2)));
             if (e != cudaSuccess) return e;
@@ -933,14 +931,9 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
         P.insts = one_scene->insts;
     }
     const int trace_grid = grid_for(sms, (instanced ? 512 : 1024) / tb);
-    auto extend = [&](cudaStream_t s, int cur) {
+    auto trace = [&](cudaStream_t s, int cur) {
         launch_trace(bvh_kind, instanced, tb, one_scene != nullptr, [&](auto k, auto b, auto one) {
-            k_extend<k.value, b.value, one.value><<<trace_grid, tb, stack_bytes, s>>>(P, cur);
-        });
-    };
-    auto shadow = [&](cudaStream_t s) {
-        launch_trace(bvh_kind, instanced, tb, one_scene != nullptr, [&](auto k, auto b, auto one) {
-            k_shadow<k.value, b.value, one.value><<<trace_grid, tb, stack_bytes, s>>>(P);
+            k_trace<k.value, b.value, one.value><<<trace_grid, tb, stack_bytes, s>>>(P, cur);
         });
     };
     const int shade_grid = grid_for(sms, 8);
@@ -956,8 +949,7 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
         k_generate<<<gen_grid, kBlock, 0, s>>>(P);
         for (uint32_t b = 0; b < bounces; ++b) {
             const int cur = int(b & 1u);
-            k_bounce_reset<<<1, 32, 0, s>>>(st.counters, cur ^ 1);
-            extend(s, cur);
+            trace(s, cur);
             if (face_order) {
                 // textured scenes, large batches: order by (class, Ptex face, footprint region), three 8-bit
                 // radix passes from the queue to queue_sorted (through rvals)
@@ -965,7 +957,6 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
                     if (instanced) k_sort_keys<true, false><<<shade_grid, kBlock, 0, s>>>(P, cur);
                     else k_sort_keys<false, false><<<shade_grid, kBlock, 0, s>>>(P, cur);
                 } else {
-                    k_class_reset<<<1, 32, 0, s>>>(st.counters);
                     if (instanced) k_sort_keys<true, true><<<shade_grid, kBlock, 0, s>>>(P, cur);
                     else k_sort_keys<false, true><<<shade_grid, kBlock, 0, s>>>(P, cur);
                 }
@@ -983,11 +974,11 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
                     vin = vout;
                 }
             } else if (sort) {
-                k_class_reset<<<1, 32, 0, s>>>(st.counters);
                 if (instanced) k_classify<true><<<shade_grid, kBlock, 0, s>>>(P, cur);
                 else k_classify<false><<<shade_grid, kBlock, 0, s>>>(P, cur);
-                k_class_offsets<<<1, 32, 0, s>>>(st.counters);
                 k_class_scatter<<<shade_grid, kBlock, 0, s>>>(P, cur);
+            } else {
+                k_bounce_reset<<<1, 32, 0, s>>>(st.counters, cur);
             }
             // Ptex base colours of the hits (the shading kernel reads them), in shading order
             const uint32_t* q = sort ? st.queue_sorted : st.queue[cur];
@@ -1005,7 +996,6 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
             } else {
                 launch_shade(modes, instanced, -1, sms, s, P, cur, b, q, whole);
             }
-            shadow(s);
             if (ray_sort && b + 1 < bounces) {
                 // order the next bounce's queue by (direction bin, origin cell): two 8-bit radix passes, the
                 // queue ping-ponging through rvals
@@ -1026,6 +1016,7 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
                 }
             }
         }
+        trace(s, -1);
         k_batch_end<<<1, 32, 0, s>>>(P);
     };
     struct Key {

@@ -323,16 +323,12 @@ __global__ void k_reset(uint32_t* counters) {
     if (threadIdx.x < 8) counters[threadIdx.x] = 0u;
 }
 
-__global__ void k_bounce_reset(uint32_t* counters, int next) {
-    if (threadIdx.x == 0) {
-        counters[next] = 0u;
-        counters[2] = 0u;  // shadow entries
-        counters[3] = 0u;  // extend cursor
-        counters[4] = 0u;  // shadow cursor
-        counters[5] = 0u;  // camera-vertex records
-        counters[6] = 0u;  // connection pairs
-    }
+// Counters that restart once a bounce is traced, by the kernel that follows the tracing: the next queue's length [cur ^ 1],
+// shadow entries [2], both fetch cursors [3], [4], camera-vertex records [5] and connection pairs [6].
+__device__ __forceinline__ void bounce_reset(uint32_t* counters, int cur) {
+    if (threadIdx.x < 6) counters[threadIdx.x == 0 ? cur ^ 1 : threadIdx.x + 1] = 0u;
 }
+__global__ void k_bounce_reset(uint32_t* counters, int cur) { bounce_reset(counters, cur); }
 
 // Concentric map of the unit square onto the unit disc (Shirley and Chiu, "A Low Distortion Map Between Disk and
 // Square", 1997): the disc sample of EmitIblLightSample (AreaLighting.cpp:268-272).
@@ -502,41 +498,6 @@ extern __shared__ uint2 vcm_stack[];
 template <int K, int B>
 constexpr int kTraceBlocksPerSm = (K == 2 ? 512 : 1024) / B;
 
-template <int K, int B>
-__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_extend(const __grid_constant__ VcmParams P, int cur,
-                                                                       int stack_depth) {
-    const uint32_t n = P.st.counters[cur];
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays, (unsigned long long)n);
-    const uint32_t* queue = P.st.queue[cur];
-    uint32_t status = 0;
-    PathRays rays(P, queue, n);
-    if constexpr (K == 1) {
-        __shared__ int stack_mem[kBinaryStack * B];
-        for (;;) {
-            uint32_t base = 0;
-            if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[3], 32u);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base >= n) break;
-            const uint32_t e = base + (threadIdx.x & 31u);
-            if (e < n) {
-                QueryRay q;
-                rays.begin(e, q);
-                QueryHit h;
-                trace_binary<false>(static_cast<const float4*>(P.nodes), P.tris, q, h, stack_mem + threadIdx.x, B,
-                                    status);
-                const float uv[2] = {h.u, h.v};
-                rays.store(queue[e], h.t, uv, h.tri);
-            }
-        }
-    } else {
-        const WideStack stack{vcm_stack + threadIdx.x, B, stack_depth};
-        if constexpr (K == 2) trace_stream<false, InstWalk>(rays, stack, status);
-        else if (short_queue(n)) trace_groups<false>(rays, n, stack, status);
-        else trace_stream<false, WideWalk>(rays, stack, status);
-    }
-    if (status) atomicOr(P.err, status);
-}
-
 // Any-hit of the queued shadow rays; unoccluded ones add their contribution to their pixel.
 struct ShadowRays : QueueRanges {
     const VcmParams& P;
@@ -565,14 +526,43 @@ struct ShadowRays : QueueRanges {
 };
 
 template <int K, int B>
-__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_shadow(const __grid_constant__ VcmParams P,
-                                                                       int stack_depth) {
+__device__ __forceinline__ void extend_queue(const VcmParams& P, int cur, int stack_depth, int* binary_stack,
+                                             uint32_t& status) {
+    const uint32_t n = P.st.counters[cur];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays, (unsigned long long)n);
+    const uint32_t* queue = P.st.queue[cur];
+    PathRays rays(P, queue, n);
+    if constexpr (K == 1) {
+        for (;;) {
+            uint32_t base = 0;
+            if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[3], 32u);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (base >= n) break;
+            const uint32_t e = base + (threadIdx.x & 31u);
+            if (e < n) {
+                QueryRay q;
+                rays.begin(e, q);
+                QueryHit h;
+                trace_binary<false>(static_cast<const float4*>(P.nodes), P.tris, q, h, binary_stack + threadIdx.x, B,
+                                    status);
+                const float uv[2] = {h.u, h.v};
+                rays.store(queue[e], h.t, uv, h.tri);
+            }
+        }
+    } else {
+        const WideStack stack{vcm_stack + threadIdx.x, B, stack_depth};
+        if constexpr (K == 2) trace_stream<false, InstWalk>(rays, stack, status);
+        else if (short_queue(n)) trace_groups<false>(rays, n, stack, status);
+        else trace_stream<false, WideWalk>(rays, stack, status);
+    }
+}
+
+template <int K, int B>
+__device__ __forceinline__ void shadow_queue(const VcmParams& P, int stack_depth, int* binary_stack, uint32_t& status) {
     const uint32_t n = P.st.counters[2];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.st.rays + 1, (unsigned long long)n);
-    uint32_t status = 0;
     ShadowRays rays(P, n);
     if constexpr (K == 1) {
-        __shared__ int stack_mem[kBinaryStack * B];
         for (;;) {
             uint32_t base = 0;
             if ((threadIdx.x & 31u) == 0) base = atomicAdd(&P.st.counters[4], 32u);
@@ -582,7 +572,7 @@ __global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_shadow(const __g
             QueryRay q;
             if (e < n && rays.begin(e, q)) {
                 QueryHit h;
-                if (!trace_binary<true>(static_cast<const float4*>(P.nodes), P.tris, q, h, stack_mem + threadIdx.x, B,
+                if (!trace_binary<true>(static_cast<const float4*>(P.nodes), P.tris, q, h, binary_stack + threadIdx.x, B,
                                         status))
                     rays.add(e);
             }
@@ -593,6 +583,18 @@ __global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_shadow(const __g
         else if (short_queue(n)) trace_groups<true>(rays, n, stack, status);
         else trace_stream<true, WideWalk>(rays, stack, status);
     }
+}
+
+// A bounce's rays: the closest hits of the queued paths (cur < 0: none), then the shadow rays that the bounce before
+// queued, in one launch (as the path tracer's k_trace).  It also clears the class counts.
+template <int K, int B>
+__global__ void __launch_bounds__(B, kTraceBlocksPerSm<K, B>) k_trace(const __grid_constant__ VcmParams P, int cur,
+                                                                      int stack_depth) {
+    __shared__ int binary_stack[K == 1 ? kBinaryStack * B : 1];
+    if (blockIdx.x == 0 && threadIdx.x < 32) P.st.counters[32 + threadIdx.x] = 0u;
+    uint32_t status = 0;
+    if (cur >= 0) extend_queue<K, B>(P, cur, stack_depth, binary_stack, status);
+    shadow_queue<K, B>(P, stack_depth, binary_stack, status);
     if (status) atomicOr(P.err, status);
 }
 
@@ -691,10 +693,6 @@ __device__ __forceinline__ uint32_t vmaterial_class(const VcmParams& P, uint32_t
     return 1u + shader * 4u + ((m.flags & kMaterialTextured) ? 2u : 0u) + ((m.flags & kMaterialTransparent) ? 1u : 0u);
 }
 
-__global__ void k_vclass_reset(uint32_t* counters) {
-    if (threadIdx.x < 32) counters[32 + threadIdx.x] = 0u;
-}
-
 template <bool kInst>
 __global__ void __launch_bounds__(kBlock) k_vclassify(VcmParams P, int cur) {
     const uint32_t n = P.st.counters[cur];
@@ -709,17 +707,15 @@ __global__ void __launch_bounds__(kBlock) k_vclassify(VcmParams P, int cur) {
     }
 }
 
-__global__ void k_vclass_offsets(uint32_t* counters) {
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int c = 0; c < 16; ++c) {
-            counters[48 + c] = run;
-            run += counters[32 + c];
-        }
-    }
-}
-
 __global__ void __launch_bounds__(kBlock) k_vclass_scatter(VcmParams P, int cur) {
+    __shared__ uint32_t first[16];  // the classes' places in the sorted queue
+    if (threadIdx.x < 16) {
+        uint32_t run = 0;
+        for (uint32_t c = 0; c < threadIdx.x; ++c) run += P.st.counters[32 + c];
+        first[threadIdx.x] = run;
+    }
+    if (blockIdx.x == 0) bounce_reset(P.st.counters, cur);
+    __syncthreads();
     const uint32_t n = P.st.counters[cur];
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t e = base + threadIdx.x;
@@ -729,7 +725,7 @@ __global__ void __launch_bounds__(kBlock) k_vclass_scatter(VcmParams P, int cur)
         const uint32_t lane = threadIdx.x & 31u;
         const int leader = __ffs(peers) - 1;
         uint32_t at = 0;
-        if (valid && leader == int(lane)) at = atomicAdd(&P.st.counters[48 + c], __popc(peers));
+        if (valid && leader == int(lane)) at = first[c] + atomicAdd(&P.st.counters[48 + c], __popc(peers));
         at = __shfl_sync(0xffffffffu, at, leader);
         if (valid) P.st.queue_sorted[at + __popc(peers & ((1u << lane) - 1u))] = P.st.queue[cur][e];
     }
@@ -1411,17 +1407,11 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
     const int inst_grid = sms * 4;
     const int depth = int(sc.stack_depth);
     const size_t stack_128 = size_t(depth) * 128 * sizeof(uint2), stack_256 = 2 * stack_128;
-    auto extend = [&](cudaStream_t stream, int cur) {
-        if (inst) k_extend<2, 128><<<inst_grid, 128, stack_128, stream>>>(P, cur, depth);
-        else if (sc.bvh_kind != 0) k_extend<1, 128><<<trace_grid, 128, 0, stream>>>(P, cur, depth);
-        else if (tb == 256) k_extend<0, 256><<<trace_grid, 256, stack_256, stream>>>(P, cur, depth);
-        else k_extend<0, 128><<<trace_grid, 128, stack_128, stream>>>(P, cur, depth);
-    };
-    auto shadow = [&](cudaStream_t stream) {
-        if (inst) k_shadow<2, 128><<<inst_grid, 128, stack_128, stream>>>(P, depth);
-        else if (sc.bvh_kind != 0) k_shadow<1, 128><<<trace_grid, 128, 0, stream>>>(P, depth);
-        else if (tb == 256) k_shadow<0, 256><<<trace_grid, 256, stack_256, stream>>>(P, depth);
-        else k_shadow<0, 128><<<trace_grid, 128, stack_128, stream>>>(P, depth);
+    auto trace = [&](cudaStream_t stream, int cur) {
+        if (inst) k_trace<2, 128><<<inst_grid, 128, stack_128, stream>>>(P, cur, depth);
+        else if (sc.bvh_kind != 0) k_trace<1, 128><<<trace_grid, 128, 0, stream>>>(P, cur, depth);
+        else if (tb == 256) k_trace<0, 256><<<trace_grid, 256, stack_256, stream>>>(P, cur, depth);
+        else k_trace<0, 128><<<trace_grid, 128, stack_128, stream>>>(P, cur, depth);
     };
     // Textures are filtered by the texture pass (k_vtexture) over the sorted queue when the hits are sorted; the
     // plain form (SEL_OPTION_MATERIAL_SORT 0) filters triangle Ptex inline in queue order, and quad-mesh Ptex, which
@@ -1432,16 +1422,16 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
     const int merge_grid = wave(reinterpret_cast<const void*>(&k_c_merge));
     // material-class sort and Ptex of a bounce's hits; returns the queue the shading kernel reads
     auto sort_hits = [&](cudaStream_t stream, int cur) -> const uint32_t* {
-        if (!pretex) return st.queue[cur];
         const uint32_t* q = st.queue[cur];
         if (sort) {
-            k_vclass_reset<<<1, 32, 0, stream>>>(st.counters);
             if (inst) k_vclassify<true><<<shade_grid, kBlock, 0, stream>>>(P, cur);
             else k_vclassify<false><<<shade_grid, kBlock, 0, stream>>>(P, cur);
-            k_vclass_offsets<<<1, 32, 0, stream>>>(st.counters);
             k_vclass_scatter<<<shade_grid, kBlock, 0, stream>>>(P, cur);
             q = st.queue_sorted;
+        } else {
+            k_bounce_reset<<<1, 32, 0, stream>>>(st.counters, cur);
         }
+        if (!pretex) return q;
         if (inst && quads) k_vtexture<true, true><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
         else if (inst) k_vtexture<true, false><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
         else if (quads) k_vtexture<false, true><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
@@ -1455,14 +1445,13 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
         k_l_generate<<<shade_grid, kBlock, 0, stream>>>(P);
         for (uint32_t b = 0; b + 1 < set.max_len; ++b) {
             const int cur = int(b & 1u);
-            k_bounce_reset<<<1, 32, 0, stream>>>(st.counters, cur ^ 1);
-            extend(stream, cur);
+            trace(stream, cur);
             const uint32_t* q = sort_hits(stream, cur);
             if (inst) k_l_shade<true, true><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
             else if (pretex) k_l_shade<true, false><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
             else k_l_shade<false, false><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
-            shadow(stream);
         }
+        trace(stream, -1);
         // hash grid over the stored vertices
         k_bounds<<<kBoundsBlocks, 256, 0, stream>>>(P);
         k_bounds_final<<<1, 32, 0, stream>>>(P, kBoundsBlocks);
@@ -1484,16 +1473,15 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
         k_c_generate<<<shade_grid, kBlock, 0, stream>>>(P);
         for (uint32_t b = 0; b < set.max_len; ++b) {
             const int cur = int(b & 1u);
-            k_bounce_reset<<<1, 32, 0, stream>>>(st.counters, cur ^ 1);
-            extend(stream, cur);
+            trace(stream, cur);
             const uint32_t* q = sort_hits(stream, cur);
             if (inst) k_c_shade<true, true><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
             else if (pretex) k_c_shade<true, false><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
             else k_c_shade<false, false><<<sms, kVertexBlock, 0, stream>>>(P, cur, q);
             k_c_connect<<<sms, kConnectBlock, 0, stream>>>(P);
             k_c_merge<<<merge_grid, kBlock, 0, stream>>>(P);
-            shadow(stream);
         }
+        trace(stream, -1);
         k_pass_end<<<1, 32, 0, stream>>>(st.iter);
     };
     struct Key {
