@@ -1431,7 +1431,7 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
         } else {
             k_bounce_reset<<<1, 32, 0, stream>>>(st.counters, cur);
         }
-        if (!pretex) return q;
+        if (!pretex || !pt_scene_textured(sc)) return q;  // no hit reads a texture
         if (inst && quads) k_vtexture<true, true><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
         else if (inst) k_vtexture<true, false><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
         else if (quads) k_vtexture<false, true><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
