@@ -526,8 +526,17 @@ __global__ void __launch_bounds__(kBlock) k_texture(PtParams P, int cur, const u
 // 22.4 ms, textured room 27.7 and 27.4 ms, deferred sky 5.09 and 5.22 ms; the kernels for any shader spill too much at 96.
 template <uint32_t kModes, int kShader>
 constexpr int kShadeBlock = kModes == 3u || kShader < 0 ? 512 : 640;
+template <uint32_t kModes>
+constexpr uint32_t kParts = (kModes & 2u) ? 3u : 2u;
+template <uint32_t kModes, int kShader>
+constexpr uint32_t shade_share = (kShadeBlock<kModes, kShader> / kParts<kModes>) & ~31u;
 
-template <uint32_t kModes, bool kInst, int kShader>
+// kSplit (batches of at most one share of every block): an entry has a thread for each of its parts, the estimate of the
+// light, the deferred form's of the background, and the next segment, which so run at the same time; the blocks would
+// otherwise be a quarter full.  All set the hit up; a part skips the draws of those before it.  128 x 128 preview: 285 -> 260
+// us.
+// Larger batches keep the plain form: the split costs it registers (1280 x 720 still 21.6 -> 21.9 ms).
+template <uint32_t kModes, bool kInst, int kShader, bool kSplit>
 __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
     k_shade(PtParams P, int cur, uint32_t bounce, const uint32_t* in_queue, int2 classes) {
     uint32_t lo = 0, hi = P.st.counters[cur];
@@ -543,9 +552,13 @@ __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
     }
     const int next = cur ^ 1;
     const uint32_t step = even_step(hi - lo);
+    const uint32_t share = shade_share<kModes, kShader>;
+    const bool split = kSplit && step <= share && gridDim.x * step >= hi - lo;
+    const uint32_t part = split ? threadIdx.x / share : 0u, at = threadIdx.x - part * share;
+    const bool shades = !split || part == kParts<kModes> - 1;
     for (uint32_t base = lo + blockIdx.x * step; base < hi; base += gridDim.x * step) {
-        const uint32_t e = base + threadIdx.x;
-        const bool valid = threadIdx.x < step && e < hi;
+        const uint32_t e = base + at;
+        const bool valid = at < step && e < hi && part < kParts<kModes>;
         uint32_t s = 0, job = 0, pixel = 0, light_set = 0, tri = 0xffffffffu;
         float3 d = f3(0.0f), thr = d, pos = d, fn = d, ft = d, fb = d, base_color = d;
         const MaterialDev* mat = nullptr;
@@ -598,11 +611,13 @@ __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
         const PtJob& J = P.st.jobs[job];
         const PtScene& S = J.scene;
         const bool on_surface = tri != 0xffffffffu;
+        if constexpr (kSplit) __syncthreads();  // every part has read the path's state
         const bool deferred = kModes == 2u || (kModes == 3u && J.mode == kPtModeDeferred);
         // Next-event estimation: to the surface's light set (AreaLighting.cpp:353-373), then, deferred, to the
         // background; the segments with a contribution are queued (at most 2 records per path).
 #pragma unroll 1
-        for (int pass = 0; pass < ((kModes & 2u) ? 2 : 1); ++pass) {
+        for (uint32_t pass = 0; pass < kParts<kModes> - 1; ++pass) {
+            const bool mine = on_surface && (!split || part == pass);
             LightSample ls;
             ls.radiance = f3(0.0f);
             if (on_surface && pass == 0 && light_set < S.light_set_count) {
@@ -612,8 +627,10 @@ __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
                     uint32_t li = uint32_t(p0u * float(set.y));
                     li = li < set.y ? li : set.y - 1;
                     const float u = pcg_float(rng), v = pcg_float(rng);
-                    sample_quad_light(S.lights[set.x + li], pos, fn, u, v, ls);
-                    ls.pdf *= 1.0f / float(set.y);
+                    if (mine) {
+                        sample_quad_light(S.lights[set.x + li], pos, fn, u, v, ls);
+                        ls.pdf *= 1.0f / float(set.y);
+                    }
                 }
             }
             if ((kModes & 2u) && on_surface && pass == 1 && deferred) {
@@ -622,7 +639,8 @@ __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
                 // as 1; at distance 1e36
                 const float r0 = pcg_float(rng), r1 = pcg_float(rng);
                 ls.distance = 1e36f;
-                if (S.ibl) {
+                if (!mine) {
+                } else if (S.ibl) {
                     ibl_sample(*S.ibl, r0, r1, ls.direction, ls.radiance, ls.pdf);
                 } else {
                     const float uu = 2.0f * r1 - 1.0f;
@@ -633,10 +651,10 @@ __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
                     ls.pdf = 1.0f;
                 }
             }
-            __syncthreads();
+            if (!split) __syncthreads();
             bool shadow = false;
             float4 sh_o = make_float4(0, 0, 0, 0), sh_d = sh_o, sh_c = sh_o;
-            if (on_surface && dot(ls.radiance, f3(1.0f)) > 0.0f) {
+            if (mine && dot(ls.radiance, f3(1.0f)) > 0.0f) {
                 float fpdf, rpdf;
                 const Surface sf = make_surface_frame(*mat, ft, fn, fb, -d, base_color);
                 const float3 refl = bsdf_evaluate_as<kShader>(sf, -d, ls.direction, fpdf, rpdf);
@@ -661,9 +679,9 @@ __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
                 P.st.sh_c[sslot] = sh_c;
             }
         }
-        __syncthreads();
+        if (!split) __syncthreads();
         bool cont = false;
-        if (valid) {
+        if (valid && shades) {
             const uint32_t npix = J.cam.width * J.cam.height;
             float4 med = P.st.medium[s];
             bool alive = true;
@@ -855,32 +873,31 @@ size_t pt_state_block_bytes(uint32_t paths) {
 
 // Shader-specific kernels for the solid and Dirac shaders of single-integrator batches; thin surfaces and mixed
 // batches take the kernel for every shader (each specialisation is compiled once per integrator and instancing).
+// `split`: the form with a thread for each part of an entry (the Dirac shader has one part, mixed batches keep the
+// plain form).
 template <uint32_t kModes, bool kInst>
-void launch_shade_modes(int shader, int grid, cudaStream_t s, const PtParams& P, int cur, uint32_t b,
+void launch_shade_modes(int shader, bool split, int grid, cudaStream_t s, const PtParams& P, int cur, uint32_t b,
                         const uint32_t* q, int2 classes) {
+    auto launch = [&](auto kernel, int block) { kernel<<<grid, block, 0, s>>>(P, cur, b, q, classes); };
     if constexpr (kModes != 3u) {
-        if (shader == 1) {
-            k_shade<kModes, kInst, 1><<<grid, kShadeBlock<kModes, 1>, 0, s>>>(P, cur, b, q, classes);
-            return;
-        }
-        if (shader == 2) {
-            k_shade<kModes, kInst, 2><<<grid, kShadeBlock<kModes, 2>, 0, s>>>(P, cur, b, q, classes);
-            return;
-        }
+        if (shader == 2) return launch(k_shade<kModes, kInst, 2, false>, kShadeBlock<kModes, 2>);
+        if (shader == 1 && split) return launch(k_shade<kModes, kInst, 1, true>, kShadeBlock<kModes, 1>);
+        if (shader == 1) return launch(k_shade<kModes, kInst, 1, false>, kShadeBlock<kModes, 1>);
+        if (split) return launch(k_shade<kModes, kInst, -1, true>, kShadeBlock<kModes, -1>);
     }
-    k_shade<kModes, kInst, -1><<<grid, kShadeBlock<kModes, -1>, 0, s>>>(P, cur, b, q, classes);
+    launch(k_shade<kModes, kInst, -1, false>, kShadeBlock<kModes, -1>);
 }
 
-void launch_shade(uint32_t modes, bool inst, int shader, int grid, cudaStream_t s, const PtParams& P, int cur,
-                  uint32_t b, const uint32_t* q, int2 classes) {
+void launch_shade(uint32_t modes, bool inst, int shader, bool split, int grid, cudaStream_t s, const PtParams& P,
+                  int cur, uint32_t b, const uint32_t* q, int2 classes) {
     if (inst) {
-        if (modes == 2u) launch_shade_modes<2, true>(shader, grid, s, P, cur, b, q, classes);
-        else if (modes == 3u) launch_shade_modes<3, true>(shader, grid, s, P, cur, b, q, classes);
-        else launch_shade_modes<1, true>(shader, grid, s, P, cur, b, q, classes);
+        if (modes == 2u) launch_shade_modes<2, true>(shader, split, grid, s, P, cur, b, q, classes);
+        else if (modes == 3u) launch_shade_modes<3, true>(shader, split, grid, s, P, cur, b, q, classes);
+        else launch_shade_modes<1, true>(shader, split, grid, s, P, cur, b, q, classes);
     } else {
-        if (modes == 2u) launch_shade_modes<2, false>(shader, grid, s, P, cur, b, q, classes);
-        else if (modes == 3u) launch_shade_modes<3, false>(shader, grid, s, P, cur, b, q, classes);
-        else launch_shade_modes<1, false>(shader, grid, s, P, cur, b, q, classes);
+        if (modes == 2u) launch_shade_modes<2, false>(shader, split, grid, s, P, cur, b, q, classes);
+        else if (modes == 3u) launch_shade_modes<3, false>(shader, split, grid, s, P, cur, b, q, classes);
+        else launch_shade_modes<1, false>(shader, split, grid, s, P, cur, b, q, classes);
     }
 }
 
@@ -944,6 +961,7 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
     const uint32_t kinds = shader_kinds & 7u;
     const bool one_kind = kinds != 0u && (kinds & (kinds - 1u)) == 0u;
     const int single = one_kind ? __builtin_ctz(kinds) : -1;
+    const bool split = batch_paths <= uint64_t(sms) * (modes == 1u ? shade_share<1u, -1> : shade_share<2u, -1>);
     auto enqueue = [&](cudaStream_t s) {
         k_batch_begin<<<1, 32, 0, s>>>(P);
         k_generate<<<gen_grid, kBlock, 0, s>>>(P);
@@ -988,13 +1006,13 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
             else if (texture) k_texture<false, false><<<shade_grid, kBlock, 0, s>>>(P, cur, q);
             const int2 whole = make_int2(-1, -1);
             if (one_kind) {
-                launch_shade(modes, instanced, single, sms, s, P, cur, b, q, whole);
+                launch_shade(modes, instanced, single, split, sms, s, P, cur, b, q, whole);
             } else if (sort) {
-                launch_shade(modes, instanced, -1, sms, s, P, cur, b, q, make_int2(0, 4));
-                if (kinds & 2u) launch_shade(modes, instanced, 1, sms, s, P, cur, b, q, make_int2(5, 8));
-                if (kinds & 4u) launch_shade(modes, instanced, 2, sms, s, P, cur, b, q, make_int2(9, 12));
+                launch_shade(modes, instanced, -1, split, sms, s, P, cur, b, q, make_int2(0, 4));
+                if (kinds & 2u) launch_shade(modes, instanced, 1, split, sms, s, P, cur, b, q, make_int2(5, 8));
+                if (kinds & 4u) launch_shade(modes, instanced, 2, split, sms, s, P, cur, b, q, make_int2(9, 12));
             } else {
-                launch_shade(modes, instanced, -1, sms, s, P, cur, b, q, whole);
+                launch_shade(modes, instanced, -1, split, sms, s, P, cur, b, q, whole);
             }
             if (ray_sort && b + 1 < bounces) {
                 // order the next bounce's queue by (direction bin, origin cell): two 8-bit radix passes, the
@@ -1024,7 +1042,7 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
         int kind, sms;
         uint32_t bounces, sort;
         int tb;
-        uint32_t modes, instanced, texture, ray_sort, face_order, kinds, quad_ptex;
+        uint32_t modes, instanced, texture, ray_sort, face_order, kinds, quad_ptex, split;
     } key;
     std::memset(&key, 0, sizeof(key));
     std::memcpy(&key.P, &P, sizeof(P));
@@ -1040,6 +1058,7 @@ cudaError_t pt_run_batches(int bvh_kind, uint32_t bounces, bool sort, const PtSt
     key.face_order = face_order ? 1u : 0u;
     key.kinds = kinds;
     key.quad_ptex = quad_ptex ? 1u : 0u;
+    key.split = split ? 1u : 0u;
     return replay(graphs, &key, sizeof(key), stream, batches, enqueue);
 }
 

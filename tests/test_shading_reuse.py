@@ -54,10 +54,12 @@ def test_metallic_zero_equals_denormal_metallic(base, tint):
         assert np.array_equal(got[0].view(np.uint32), got[1].view(np.uint32))
 
 
-# batches around one warp, around the wave of 512- and 640-thread blocks on 152 SMs, and two steps with a remainder
+# batches around one warp, around the most that the forms with a thread for each part of an entry take (160 and 256 a
+# block on 152 SMs), around the wave of 512- and 640-thread blocks, and two steps with a remainder
 @pytest.mark.gpu
-@pytest.mark.parametrize("size,batch", [((9, 7), 1), ((9, 7), 31), ((9, 7), 33), ((400, 250), 77823), ((400, 250), 77825),
-                                        ((400, 250), 97279), ((400, 250), 97281)])
+@pytest.mark.parametrize("size,batch", [((9, 7), 1), ((9, 7), 31), ((9, 7), 33), ((400, 250), 24320), ((400, 250), 24321),
+                                        ((400, 250), 38912), ((400, 250), 38913), ((400, 250), 77823),
+                                        ((400, 250), 77825), ((400, 250), 97279), ((400, 250), 97281)])
 def test_batches_of_any_size_give_one_image(device, size, batch):
     import selas_gb300 as sel
     from selas_gb300 import scenes
