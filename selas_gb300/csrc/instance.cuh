@@ -130,18 +130,22 @@ __device__ __forceinline__ void inst_record_hit(InstState& s, float t, float u, 
 
 // The instanced traversal of one lane, as trace_stream steps it.
 struct InstWalk {
+    static constexpr bool kAims = true;
     InstState s;
+    uint32_t turn;  // kStay; kLeave, kEnter: the level changed and the ray has yet to follow (aim)
+    static constexpr uint32_t kStay = 0u, kLeave = 1u, kEnter = 2u;
     uint32_t tmask, tbase;  // leaf records of the current level still to test: bit k is record tbase + k
 
     template <typename Rays>
     __device__ __forceinline__ bool start(const QueryRay& r, const Rays& rays) {
         inst_init(s, r, rays.nodes(), rays.tris(), rays.insts());
         tmask = 0;
+        turn = kStay;
         return !ray_untraceable(r);
     }
 
     // Enters the instance of leaf record words p0: pushes what is left of the current node and leaf and a level
-    // marker, and goes on at the instanced BVH's root.  Returns false when a limit is reached.
+    // marker; the ray follows in aim.  Returns false when a limit is reached.
     __device__ __forceinline__ bool enter(const float4& p0, const WideStack& stack, uint32_t& status) {
         if (s.level >= 2) {
             status |= kErrInstanceDepth;
@@ -159,15 +163,29 @@ struct InstWalk {
         if (s.level == 0) s.chain0 = s.insts + __float_as_uint(p0.w);
         else s.chain1 = s.insts + __float_as_uint(p0.w);
         ++s.level;
+        s.w.group = make_uint2(0u, 0u);
+        tmask = 0;
+        turn = kEnter;
+        return true;
+    }
+
+    __device__ __forceinline__ bool aiming() const { return turn != kStay; }
+
+    // Takes the ray to the current level: an entered instance's BVH starts at its root (with nothing to do in one that
+    // the transformed ray cannot hit), a level returned to goes on with what was popped.  One place a step for both,
+    // not where a record is met and where a marker is popped: lanes that enter and lanes that return transform their
+    // rays together, and a ray with nothing left in the parent ends without (terrain with instances 11.42 -> 10.51 ms
+    // a frame; waiting for 4, 8, 16 such lanes 10.61, 10.90, 12.10 ms).
+    __device__ __forceinline__ void aim() {
         inst_level_pointers(s);
         inst_level_ray(s);
-        QueryRay lr;
-        lr.ox = s.w.ox; lr.oy = s.w.oy; lr.oz = s.w.oz;
-        lr.dx = s.w.dx; lr.dy = s.w.dy; lr.dz = s.w.dz;
-        // the instanced BVH's root; nothing to do in an instance the transformed ray cannot hit
-        s.w.group = ray_untraceable(lr) ? make_uint2(0u, 0u) : make_uint2(0u, (1u << (24 + s.w.oct)) | 1u);
-        tmask = 0;
-        return true;
+        if (turn == kEnter) {
+            QueryRay lr;
+            lr.ox = s.w.ox; lr.oy = s.w.oy; lr.oz = s.w.oz;
+            lr.dx = s.w.dx; lr.dy = s.w.dy; lr.dz = s.w.dz;
+            if (!ray_untraceable(lr)) s.w.group = make_uint2(0u, (1u << (24 + s.w.oct)) | 1u);
+        }
+        turn = kStay;
     }
 
     __device__ __forceinline__ bool pending() const { return tmask != 0u; }
@@ -221,8 +239,7 @@ struct InstWalk {
             const uint2 e = stack.mem[(--s.w.sp) * stack.stride];
             if (e.y == 0u) {  // level marker: back to the parent level
                 --s.level;
-                inst_level_pointers(s);
-                inst_level_ray(s);
+                turn = kLeave;
             } else if (e.x & kPendingLeaf) {
                 tbase = e.x & ~kPendingLeaf;
                 tmask = e.y;

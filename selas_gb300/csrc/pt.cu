@@ -522,8 +522,9 @@ __global__ void __launch_bounds__(kBlock) k_texture(PtParams P, int cur, const u
 // whole queue.
 // Bound by instruction fetches and latency (see even_step): one block per SM, its warps in step.  The frame, base
 // colour and material address are held from stage to stage and the rest of the surface is read again from the
-// material's record, so that little spills.  640 threads at 96 registers against 512 at 128: 1280 x 720 still 21.7 and
-// 22.4 ms, textured room 27.7 and 27.4 ms, deferred sky 5.09 and 5.22 ms; the kernels for any shader spill too much at 96.
+// material's record, so that little spills.  640 threads at 96 registers against 512 at 128: Cornell box 512 x 512 x
+// 64 spp 21.7 and 22.4 ms, textured room 27.7 and 27.4, deferred sky 5.09 and 5.22; the kernels for any shader spill
+// too much at 96.
 template <uint32_t kModes, int kShader>
 constexpr int kShadeBlock = kModes == 3u || kShader < 0 ? 512 : 640;
 template <uint32_t kModes>
@@ -533,9 +534,9 @@ constexpr uint32_t shade_share = (kShadeBlock<kModes, kShader> / kParts<kModes>)
 
 // kSplit (batches of at most one share of every block): an entry has a thread for each of its parts, the estimate of the
 // light, the deferred form's of the background, and the next segment, which so run at the same time; the blocks would
-// otherwise be a quarter full.  All set the hit up; a part skips the draws of those before it.  128 x 128 preview: 285 -> 260
-// us.
-// Larger batches keep the plain form: the split costs it registers (1280 x 720 still 21.6 -> 21.9 ms).
+// otherwise be a fifth full.  All set the hit up; a part skips the draws of those before it.  160 x 120 preview of the
+// Cornell box 285 -> 260 us.  Larger batches keep the plain form: the split costs it registers (512 x 512 x 64 spp
+// 21.6 -> 21.9 ms).
 template <uint32_t kModes, bool kInst, int kShader, bool kSplit>
 __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
     k_shade(PtParams P, int cur, uint32_t bounce, const uint32_t* in_queue, int2 classes) {

@@ -304,9 +304,9 @@ SEL_HD float3 offset_origin(float3 p, float3 n, float error, float3 dir, float s
 
 // The shading kernels are straight lines of 80 to 170 KB of code that every hit runs once: with the warps of an SM at
 // different places their rate is set by instruction fetches.  So an SM runs one block that meets at barriers between
-// the stages of a hit, and one fetch serves its warps (1280 x 720 still 22.9 -> 21.7 ms, textured room 29.0 -> 27.7 ms,
-// deferred sky 6.39 -> 5.09 ms; the large block without barriers gave a third of that, smaller code through calls
-// nothing more).
+// the stages of a hit, and one fetch serves its warps (Cornell box 512 x 512 x 64 spp 22.9 -> 21.7 ms, textured room
+// 1280 x 720 x 4 spp 29.0 -> 27.7, deferred sky 641 x 359 x 16 spp 6.39 -> 5.09; the large block without barriers gave a
+// third of that, smaller code through calls nothing more).
 //
 // Entries a block of such a grid takes per step: all blocks take as many steps with as many entries, so that a short
 // queue spreads over the SMs.

@@ -285,6 +285,8 @@ __device__ __forceinline__ bool wide_test(WideState& s, const float4* __restrict
 
 // The flat traversal of one lane, as trace_stream steps it.
 struct WideWalk {
+    static constexpr bool kAims = false;
+    __device__ __forceinline__ bool aiming() const { return false; }
     WideState s;
     uint32_t tmask, tbase;  // leaf records still to test: bit k is record tbase + k
 
@@ -373,6 +375,10 @@ __device__ __forceinline__ void trace_stream(Rays& rays, const WideStack& stack,
                 break;
             }
         }
+        if constexpr (Walk::kAims) {
+            if (busy && w.aiming()) w.aim();
+            __syncwarp();
+        }
         if (busy && !w.pending()) busy = w.visit(rays, stack, status);
         uint32_t testing = __ballot_sync(0xffffffffu, busy && w.pending());
         while (testing) {
@@ -380,7 +386,7 @@ __device__ __forceinline__ void trace_stream(Rays& rays, const WideStack& stack,
             if (__popc(testing) < kTestLanes) break;
             testing = __ballot_sync(0xffffffffu, busy && w.pending());
         }
-        if (busy) busy = w.advance(stack, status);
+        if (busy && !w.aiming()) busy = w.advance(stack, status);
     }
 }
 
