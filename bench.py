@@ -491,7 +491,7 @@ def render_metrics(sel, scenes, dev, stream, args, room=None):
     alg = q["extension_rays"] * 296 + q["shadow_rays"] * 68
     peak, peak_kind = measured_peaks()
     ach = alg / (q["ms_per_image"] * 1e-3) / 1e9
-    pt["roofline"] = {"bound": "hbm", "kernel": "whole path-tracer wavefront (k_extend + k_shade + k_shadow + "
+    pt["roofline"] = {"bound": "hbm", "kernel": "whole path-tracer wavefront (k_trace + k_shade + "
                       "queue kernels) over one image", "achieved": round(ach, 2), "peak": peak, "unit": "GB/s",
                       "frac": round(ach / peak, 5), "peak_source": peak_kind, "algorithmic_bytes_per_image": int(alg),
                       "traffic": ncu_traffic().get("pt.cornell_image")}
