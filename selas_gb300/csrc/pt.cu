@@ -534,9 +534,10 @@ constexpr uint32_t shade_share = (kShadeBlock<kModes, kShader> / kParts<kModes>)
 
 // kSplit (batches of at most one share of every block): an entry has a thread for each of its parts, the estimate of the
 // light, the deferred form's of the background, and the next segment, which so run at the same time; the blocks would
-// otherwise be a fifth full.  All set the hit up; a part skips the draws of those before it.  160 x 120 preview of the
-// Cornell box 285 -> 260 us.  Larger batches keep the plain form: the split costs it registers (512 x 512 x 64 spp
-// 21.6 -> 21.9 ms).
+// otherwise be partly full.  All set the hit up; a part skips the draws of those before it.  Split against plain, Cornell
+// box previews of 3,072, 19,200 and 38,400 paths 236, 263, 315 against 261, 286, 337 us (the limit is 38,912), deferred
+// sky of 23,040 paths 559 against 623 us (limit 24,320).  Larger batches keep the plain form: the split costs it
+// registers (512 x 512 x 64 spp 21.6 -> 21.9 ms).
 template <uint32_t kModes, bool kInst, int kShader, bool kSplit>
 __global__ void __launch_bounds__(kShadeBlock<kModes, kShader>, 1)
     k_shade(PtParams P, int cur, uint32_t bounce, const uint32_t* in_queue, int2 classes) {
