@@ -1419,6 +1419,7 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
     const bool sort = sc.sort_hint != 0 || inst;
     const bool quads = sc.ptex_quads != 0;
     const bool pretex = sort || quads;
+    const bool textured = pretex && pt_scene_textured(sc);  // else no hit reads a texture and the pass is left out
     const int merge_grid = wave(reinterpret_cast<const void*>(&k_c_merge));
     // material-class sort and Ptex of a bounce's hits; returns the queue the shading kernel reads
     auto sort_hits = [&](cudaStream_t stream, int cur) -> const uint32_t* {
@@ -1431,7 +1432,7 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
         } else {
             k_bounce_reset<<<1, 32, 0, stream>>>(st.counters, cur);
         }
-        if (!pretex || !pt_scene_textured(sc)) return q;  // no hit reads a texture
+        if (!textured) return q;
         if (inst && quads) k_vtexture<true, true><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
         else if (inst) k_vtexture<true, false><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
         else if (quads) k_vtexture<false, true><<<shade_grid, kBlock, 0, stream>>>(P, cur, q);
@@ -1484,9 +1485,10 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
         trace(stream, -1);
         k_pass_end<<<1, 32, 0, stream>>>(st.iter);
     };
+    // everything that the launches above follow besides the kernels' arguments
     struct Key {
         VcmParams P;
-        int kind, sms, radix_passes, sort, tb, quads, depth;
+        int kind, sms, radix_passes, sort, tb, quads, textured, depth;
     } key;
     std::memset(&key, 0, sizeof(key));
     std::memcpy(&key.P, &P, sizeof(P));
@@ -1496,6 +1498,7 @@ cudaError_t vcm_run_passes(const PtScene& sc, const VcmCamera& cam, const VcmSet
     key.radix_passes = radix_passes;
     key.sort = sort ? 1 : 0;
     key.quads = quads ? 1 : 0;
+    key.textured = textured ? 1 : 0;
     key.depth = depth;
     return replay(graphs, &key, sizeof(key), stream, passes, enqueue);
 }
