@@ -973,6 +973,25 @@ std::string build_wide_device(const std::vector<MeshInput>& meshes, uint32_t max
     float* vertices = nullptr;
     uint32_t* indices = nullptr;
     MeshDev* mesh_table = nullptr;
+    // What is copied to the GPU lies in memory that lives until the stream is synchronised below, on every way out;
+    // the host's allocations come before the GPU's, so that one that fails leaves nothing behind.
+    constexpr size_t kDirectBytes = 64 * 1024;
+    std::vector<MeshDev> table;
+    std::vector<uint32_t> packed;  // small meshes: vertices (as bits) and indices, in the order of their places
+    size_t small_words = 0;
+    for (const MeshInput& m : meshes)
+        for (const size_t words : {m.vertices.size(), m.indices.size()})
+            if (words * 4 < kDirectBytes) small_words += words;
+    table.reserve(meshes.size());
+    packed.reserve(small_words);
+    const uint4 root = make_uint4(0, n, 0, 0);
+    Counters ctr;
+    std::memset(&ctr, 0, sizeof(ctr));
+    ctr.small = n > kSmall ? 0u : 1u;  // the scene is one small subtree
+    for (int k = 0; k < 6; ++k) {
+        // +-infinity as ordered ints
+        ctr.box[k] = ctr.cbox[k] = k < 3 ? 0x7f800000 : int(0xff800000u ^ 0x7fffffffu);
+    }
     // one scratch block for everything but the result: sized on the first walk, carved on the second
     size_t scratch_bytes = 0;
     char* scratch = nullptr;
@@ -1014,9 +1033,6 @@ std::string build_wide_device(const std::vector<MeshInput>& meshes, uint32_t max
     if (e == cudaSuccess) e = cudaMalloc(&C.tris, sizeof(TriRecord) * size_t(n));
 
     // the meshes' arrays: large ones are copied from where they lie, small ones gathered into one copy
-    constexpr size_t kDirectBytes = 64 * 1024;
-    std::vector<MeshDev> table;
-    std::vector<uint32_t> packed;  // small meshes: vertices (as bits) and indices, in the order of their places
     size_t vat = 0, iat = 0;
     uint32_t first = 0;
     for (const MeshInput& m : meshes) {
@@ -1058,12 +1074,6 @@ std::string build_wide_device(const std::vector<MeshInput>& meshes, uint32_t max
     upload(vertices, [](const MeshInput& m) -> const std::vector<float>& { return m.vertices; });
     upload(indices, [](const MeshInput& m) -> const std::vector<uint32_t>& { return m.indices; });
     B.mesh_count = uint32_t(table.size());
-    Counters ctr;
-    std::memset(&ctr, 0, sizeof(ctr));
-    for (int k = 0; k < 6; ++k) {
-        // +-infinity as ordered ints
-        ctr.box[k] = ctr.cbox[k] = k < 3 ? 0x7f800000 : int(0xff800000u ^ 0x7fffffffu);
-    }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(mesh_table, table.data(), sizeof(MeshDev) * table.size(), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(B.ctr, &ctr, sizeof(ctr), cudaMemcpyHostToDevice, s);
@@ -1080,14 +1090,8 @@ std::string build_wide_device(const std::vector<MeshInput>& meshes, uint32_t max
             const unsigned blocks = unsigned(std::min(most, std::max<size_t>(work, 1)));
             if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(256), args, 0, s);
         };
-        if (n > kSmall) {
-            cooperative(reinterpret_cast<const void*>(&k_top), (size_t(n) + kChunk - 1) / kChunk, top_args);
-        } else {  // the scene is one small subtree
-            const uint4 root = make_uint4(0, n, 0, 0);
-            const uint32_t one = 1;
-            e = cudaMemcpyAsync(B.small, &root, sizeof(root), cudaMemcpyHostToDevice, s);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(&B.ctr->small, &one, sizeof(one), cudaMemcpyHostToDevice, s);
-        }
+        if (n > kSmall) cooperative(reinterpret_cast<const void*>(&k_top), (size_t(n) + kChunk - 1) / kChunk, top_args);
+        else e = cudaMemcpyAsync(B.small, &root, sizeof(root), cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SmallShared)));
         if (e == cudaSuccess) {
@@ -1114,7 +1118,10 @@ std::string build_wide_device(const std::vector<MeshInput>& meshes, uint32_t max
             e = cudaMemcpyAsync(nodes, C.nodes, sizeof(WideNode) * size_t(ctr.wide), cudaMemcpyDeviceToDevice, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
-    if (s) cudaStreamDestroy(s);
+    if (s) {
+        cudaStreamSynchronize(s);  // after an error copies may still be under way
+        cudaStreamDestroy(s);
+    }
     cudaFree(scratch);
     if (e != cudaSuccess || !err.empty()) {
         cudaGetLastError();
