@@ -128,7 +128,7 @@ __device__ __forceinline__ void inst_record_hit(InstState& s, float t, float u, 
     s.hit.inst[1] = uint32_t(s.cur_inst);
 }
 
-// The instanced traversal of one lane, as trace_stream steps it.
+// The instanced traversal of one lane, as trace_stream and trace_packet step it.
 struct InstWalk {
     static constexpr bool kAims = true;
     InstState s;

@@ -1,6 +1,8 @@
-// Ray-query kernels over SelRay / SelRayHit records (Embree's RTCRay / RTCRayHit layouts) and their
-// launchers.  One lane per ray; each thread keeps its traversal stack in shared memory.
+// Ray-query kernels over SelRay / SelRayHit records (Embree's RTCRay / RTCRayHit layouts) and their launchers.  A ray is
+// traced by one lane or, in small batches, by eight; each thread keeps its traversal stack in shared memory.
 #include "query.h"
+
+#include <type_traits>
 
 #include "hitref.cuh"
 #include "instance.cuh"
@@ -76,19 +78,52 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
 }
 
 // ---------------------------------------------------------------------------------------------------
-// 8-wide traversal.  Blocks are one warp and block index k stands for records [32 k, 32 k + 32).  A warp whose
+// 8-wide traversal.  Blocks are one warp; 64 registers let 32 of them run on an SM.  Which form a batch takes follows its
+// size, in rays for each warp that runs at once, and, where the size does not settle it, a look at the warp's own
+// rays (side_by_side).  Device times in us over 10 k | 0.33 M | 5.2 M triangles; "surface" rays bounce off random
+// points, "camera" rays are a frame's in pixel order.
+//   Eight lanes a ray (trace_group) up to kGroupRays, and to kSideGroupRays for rays side by side.  Against packets:
+//     24,000 surface   closest  32 | 53 | 70 against 34 | 59 | 77   any  27 | 39 | 54 against 28 | 46 | 62
+//     45,000 surface   closest  43 | 74 | 94 against 36 | 66 | 90   any  36 | 51 | 74 against 31 | 47 | 74
+//     58,368 camera    closest  22 | 38 | 62 against 26 | 52 | 77   any  19 | 29 | 48 against 23 | 36 | 64
+//     90,000 camera    closest  26 | 46 | 88 against 28 | 54 | 106  any  22 | 36 | 55 against 20 | 44 | 60
+//     116,736 camera   closest  32 | 54 | 94 against 29 | 52 | 101  any  28 | 37 | 62 against 22 | 38 | 62
+//   (the limits lie at whole rounds of the resident warps; at 8 to 9 rays a warp closest hits of 0.33 M triangles still
+//   favour the groups, 56 against 63, any hit everywhere the packets).
+//   A lane a ray, side by side to the end (trace_packet), up to kPacketRays, and at any size for rays side by side.
+//   Against streams:
+//     90,000 surface   closest  41 | 73 | 117 against 47 | 93 | 131        any  34 | 52 | 97 against 43 | 67 | 119
+//     300,000 surface  closest  88 | 138 | 253 against 96 | 145 | 257      any  74 | 117 | 213 against 82 | 126 | 210
+//     500,000 surface  closest  137 | 200 | 379 against 140 | 206 | 350    any  114 | 162 | 279 against 117 | 163 | 282
+//     4.2 M surface    closest  960 | 1404 | 2598 against 890 | 1210 | 2048   any  794 | 1103 | 1844 against 720 | 940 | 1470
+//     1 M camera       closest  52 | 113 | 273 against 73 | 145 | 272      any  40 | 86 | 164 against 58 | 105 | 192
+//   Streams of rays (trace_stream) otherwise.
+// Scenes with instances: streams, but for kInstStreamRays to 32 rays a warp, where rays that part are packets (40,000
+// random rays, closest hit over 20 | 500 | 2000 instances 46 | 92 | 174 against 45 | 99 | 181, any hit 36 | 73 | 114
+// against 41 | 84 | 125; camera rays, which meet different instances from lane to lane, stay streams: 170 against 156 us as
+// packets over 500 instances, and 4 M of them 3.0 against 2.6 ms).
+//
+// Records in host memory, traced in place (far): the link carries every look, so eight looks at a record cost more than any
+// form (45,000 camera rays, closest hit over 0.33 M triangles: a call of 161 us with them, 66 as groups, 82 as packets).
+// Groups up to kFarGroupRays (58,368 rays surface, packets against groups: closest 78 | 107 | 131 against 73 | 95 | 144, any
+// 60 | 71 | 105 against 60 | 75 | 105; camera 64 | 93 | 117 against 60 | 79 | 93, any 50 | 63 | 87 against 36 | 44 | 65), then
+// packets; closest hits are streams, without a look, from kFarPacketRays on (300,000 camera rays 303 | 321 | 329 against 315 |
+// 326 | 343 us as packets, surface 238 | 277 | 357 against 233 | 276 | 372).
+//
+// A stream's warp starts with its block's records, block index k standing for records [32 k, 32 k + 32).  A warp whose
 // lanes run out of rays takes over the block index of a block that has not started (cluster launch control) and
-// refills its finished lanes from it (trace_stream), so a batch of any size is balanced without a work counter in
+// refills its finished lanes from it, so a batch of any size is balanced without a work counter in
 // memory, on any number of streams at once and under graph capture.  The next index is requested while the
 // warp still traces the last, which hides the answer's latency.  An atomic counter in place of the block indices
 // measured 3 % faster (4 M incoherent rays over 5.2 M triangles, closest hit 1.81 against 1.87 ms) but would have to
 // be allocated and zeroed by every call.
 // 64 registers, 32 warps per SM: with 36 (56 registers) closest hit takes 1.89 against 1.81 ms and any hit 1.34
-// against 1.22, with 40 (48 registers) 2.08 and 1.46.  Whole calls on that scene, start of a call to its end: closest
-// hit 2.92 ms with one thread per ray and a 24-entry stack, 1.95 now; any hit 1.95 and 1.33; camera rays 0.50 and
-// 0.45, any hit 0.28 and 0.27.
+// against 1.22, with 40 (48 registers) 2.08 and 1.46.
 // ---------------------------------------------------------------------------------------------------
-constexpr int kWarpsPerSm = 32;
+constexpr uint32_t kWarpsPerSm = 32, kInstWarpsPerSm = 16;
+template <bool kAnyHit>
+constexpr uint32_t kGroupRays = kAnyHit ? 7 : 8;
+constexpr uint32_t kSideGroupRays = 20, kPacketRays = 64, kInstStreamRays = 2, kFarGroupRays = 12, kFarPacketRays = 32;
 constexpr uint32_t kErrClaimTimeout = 32u;  // the answer to a work request never came
 
 __device__ __forceinline__ uint32_t shared_address(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -96,13 +131,15 @@ __device__ __forceinline__ uint32_t shared_address(const void* p) { return uint3
 // The records a warp traces.  kOrdered: record `order[i]` in place of record i when ctl[0] is non-zero.
 struct RecordRanges {
     uint32_t n, status;
-    bool claim, started;     // claim: more blocks were launched than run at once
+    bool claim, started;     // claim: takes over blocks that have not started
     uint32_t phase;
     uint32_t answer, barrier;  // shared memory: 16-byte answer, its mbarrier
 
-    __device__ __forceinline__ RecordRanges(uint32_t count, bool more_blocks, const uint4* ans, const uint64_t* bar)
-        : n(count), status(0), claim(more_blocks), started(false), phase(0), answer(0), barrier(0) {
-        if (!claim) return;
+    __device__ __forceinline__ explicit RecordRanges(uint32_t count)
+        : n(count), status(0), claim(false), started(false), phase(0), answer(0), barrier(0) {}
+
+    __device__ __forceinline__ void take_over(const uint4* ans, const uint64_t* bar) {
+        claim = true;
         answer = shared_address(ans);
         barrier = shared_address(bar);
         if ((threadIdx.x & 31u) == 0) {
@@ -211,59 +248,148 @@ struct QueryArgs {
     const uint32_t* order;  // with ctl: the records' order, used when ctl[0] is non-zero
     const uint32_t* ctl;
     int stack_depth;
-    uint32_t claim;
+    uint32_t claim;         // streams take over blocks that have not started
+    float reach2;           // side_by_side: the square of the distance between neighbours' origins
     uint32_t* err;
 };
 
-template <bool kAnyHit, bool kInst, typename Walk>
-__device__ __forceinline__ void query_warp(const QueryArgs& a) {
-    extern __shared__ uint2 query_stack[];
-    __shared__ __align__(16) uint4 answer;
-    __shared__ __align__(8) uint64_t barrier;
-    RecordRays<kAnyHit, kInst> rays(a.n, a.claim != 0, &answer, &barrier);
+template <bool kAnyHit, bool kInst>
+__device__ __forceinline__ RecordRays<kAnyHit, kInst> query_records(const QueryArgs& a) {
+    RecordRays<kAnyHit, kInst> rays(a.n);
     rays.node_array = a.nodes;
     rays.tri_array = a.tris;
     rays.inst_array = a.insts;
     rays.recs = a.rays;
     rays.record_float4s = a.record_float4s;
     rays.order = a.ctl && a.ctl[0] ? a.order : nullptr;
+    return rays;
+}
+
+// Whether a warp's rays (lanes 0 .. count - 1) run side by side: three of four neighbours start within a thirty-second
+// of the scene's diagonal of one another and point within about 2.5 degrees of one another.
+__device__ __forceinline__ bool side_by_side(const QueryRay& r, uint32_t count, float reach2) {
+    float v[6] = {r.ox, r.oy, r.oz, r.dx, r.dy, r.dz}, w[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) w[k] = __shfl_down_sync(0xffffffffu, v[k], 1);
+    const float ex = w[0] - v[0], ey = w[1] - v[1], ez = w[2] - v[2];
+    const float d = v[3] * w[3] + v[4] * w[4] + v[5] * w[5];
+    const float nn = (v[3] * v[3] + v[4] * v[4] + v[5] * v[5]) * (w[3] * w[3] + w[4] * w[4] + w[5] * w[5]);
+    const bool close = (threadIdx.x & 31u) + 1 < count && ex * ex + ey * ey + ez * ez <= reach2 && nn > 0.0f &&
+                       d > 0.0f && d * d > 0.998f * nn;
+    return 4 * __popc(__ballot_sync(0xffffffffu, close)) >= 3 * int(count - 1);
+}
+
+// The rays of records [base, base + 32), a lane each; count of them exist.
+template <bool kAnyHit, bool kInst>
+struct Packet {
+    QueryRay r;
+    uint32_t base, count;
+    __device__ __forceinline__ Packet(const RecordRays<kAnyHit, kInst>& rays, uint32_t first)
+        : r{}, base(first), count(rays.n - first < 32u ? rays.n - first : 32u) {
+        if (threadIdx.x < count) rays.begin(base + threadIdx.x, r);
+    }
+    __device__ __forceinline__ void trace(const RecordRays<kAnyHit, kInst>& rays, const WideStack& stack,
+                                          uint32_t& status) const {
+        const bool live = threadIdx.x < count;
+        if constexpr (kAnyHit && !kInst) {
+            WideState s;
+            trace_packet_any(rays.nodes(), rays.tris(), live, r, s, stack, status);
+            if (live) rays.end(base + threadIdx.x, s);
+        } else {
+            std::conditional_t<kInst, InstWalk, WideWalk> w;
+            trace_packet<kAnyHit>(rays, live, r, w, stack, status);
+            if (live) rays.end(base + threadIdx.x, w.s);
+        }
+    }
+};
+
+extern __shared__ uint2 query_stack[];
+
+__device__ __forceinline__ WideStack warp_stack(const QueryArgs& a) {
+    return WideStack{query_stack + threadIdx.x, 32, a.stack_depth};
+}
+
+// kLook: a warp looks at its block's rays; flat scenes' rays that run side by side are traced as a packet, instanced
+// scenes' rays that do not.
+template <bool kAnyHit, bool kInst, bool kLook>
+__device__ __forceinline__ void query_warp(const QueryArgs& a) {
+    __shared__ __align__(16) uint4 answer;
+    __shared__ __align__(8) uint64_t barrier;
+    RecordRays<kAnyHit, kInst> rays = query_records<kAnyHit, kInst>(a);
     uint32_t status = 0;
-    trace_stream<kAnyHit, Walk>(rays, WideStack{query_stack + threadIdx.x, 32, a.stack_depth}, status);
-    status |= rays.status;
+    bool stream = true;
+    if constexpr (kLook) {
+        const Packet<kAnyHit, kInst> packet(rays, blockIdx.x * 32u);
+        stream = side_by_side(packet.r, packet.count, a.reach2) == kInst;
+        if (!stream) packet.trace(rays, warp_stack(a), status);
+    }
+    if (stream) {
+        if (a.claim) rays.take_over(&answer, &barrier);
+        trace_stream<kAnyHit, std::conditional_t<kInst, InstWalk, WideWalk>>(rays, warp_stack(a), status);
+        status |= rays.status;
+    }
     if (status) atomicOr(a.err, status);
 }
 
-template <bool kAnyHit>
+template <bool kAnyHit, bool kLook>
 __global__ void __launch_bounds__(32, kWarpsPerSm) k_query_wide(const __grid_constant__ QueryArgs a) {
-    query_warp<kAnyHit, false, WideWalk>(a);
+    query_warp<kAnyHit, false, kLook>(a);
 }
 
 // Scenes with instances or curves: 16 warps per SM (the walk's state takes up to 128 registers).
-template <bool kAnyHit>
-__global__ void __launch_bounds__(32, 16) k_query_instanced(const __grid_constant__ QueryArgs a) {
-    query_warp<kAnyHit, true, InstWalk>(a);
+template <bool kAnyHit, bool kLook>
+__global__ void __launch_bounds__(32, kInstWarpsPerSm) k_query_instanced(const __grid_constant__ QueryArgs a) {
+    query_warp<kAnyHit, true, kLook>(a);
 }
 
-// Batches of at most one ray a group of eight lanes: 4 rays a one-warp block.
 template <bool kAnyHit>
-__global__ void __launch_bounds__(32, kWarpsPerSm) k_query_groups(const __grid_constant__ QueryArgs a) {
-    extern __shared__ uint2 query_stack[];
-    RecordRays<kAnyHit, false> rays(a.n, false, nullptr, nullptr);
-    rays.node_array = a.nodes;
-    rays.tri_array = a.tris;
-    rays.recs = a.rays;
-    rays.record_float4s = a.record_float4s;
-    rays.order = nullptr;
+__global__ void __launch_bounds__(32, kWarpsPerSm) k_query_packet(const __grid_constant__ QueryArgs a) {
+    const RecordRays<kAnyHit, false> rays = query_records<kAnyHit, false>(a);
     uint32_t status = 0;
-    trace_groups<kAnyHit>(rays, a.n, WideStack{query_stack + threadIdx.x, 32, a.stack_depth}, status);
+    Packet<kAnyHit, false>(rays, blockIdx.x * 32u).trace(rays, warp_stack(a), status);
+    if (status) atomicOr(a.err, status);
+}
+
+// Four rays a one-warp block, eight lanes each.  kLook: the eight blocks of 32 records look at these records' rays (whose
+// origins and directions no query writes) and, unless they run side by side, leave them to the first of the eight.  The
+// first blocks of all records come before the others, which mostly find nothing to do when the rays part.
+template <bool kAnyHit, bool kLook>
+__global__ void __launch_bounds__(32, kWarpsPerSm) k_query_groups(const __grid_constant__ QueryArgs a) {
+    RecordRays<kAnyHit, false> rays = query_records<kAnyHit, false>(a);
+    uint32_t status = 0, first = blockIdx.x * 4u;
+    QueryRay r;
+    if constexpr (kLook) {
+        const uint32_t ranges = (a.n + 31u) / 32u;
+        const uint32_t range = blockIdx.x < ranges ? blockIdx.x : (blockIdx.x - ranges) / 7u;
+        first = range * 32u + (blockIdx.x < ranges ? 0u : 4u + (blockIdx.x - ranges) % 7u * 4u);
+        const Packet<kAnyHit, false> packet(rays, range * 32u);
+        if (!side_by_side(packet.r, packet.count, a.reach2)) {
+            if (blockIdx.x >= ranges) return;
+            packet.trace(rays, warp_stack(a), status);
+            if (status) atomicOr(a.err, status);
+            return;
+        }
+        const float* f = reinterpret_cast<const float*>(&packet.r);
+        float* mine = reinterpret_cast<float*>(&r);
+#pragma unroll
+        for (int k = 0; k < int(sizeof(QueryRay) / sizeof(float)); ++k)
+            mine[k] = __shfl_sync(0xffffffffu, f[k], int((first & 31u) + (threadIdx.x >> 3)));
+    }
+    const uint32_t i = first + (threadIdx.x >> 3);
+    if (i >= a.n) return;
+    WideState s;
+    if (!kLook) rays.begin(i, r);
+    trace_group<kAnyHit>(rays.nodes(), rays.tris(), r, s, warp_stack(a), status);
+    if ((threadIdx.x & 7u) == 0) rays.end(i, s);
     if (status) atomicOr(a.err, status);
 }
 
 template <bool kAnyHit>
 cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_float4s, uint32_t n,
-                        const uint32_t* order, const uint32_t* ctl, uint32_t* d_err, cudaStream_t s) {
+                        const uint32_t* order, const uint32_t* ctl, uint32_t* d_err, cudaStream_t s, bool far) {
     const bool inst = bvh.insts != nullptr;
     const uint32_t blocks = (n + 31u) / 32u;
+    const uint32_t resident = uint32_t(bvh.sm_count) * (inst ? kInstWarpsPerSm : kWarpsPerSm);
     QueryArgs a;
     a.nodes = static_cast<const uint4*>(bvh.nodes);
     a.tris = bvh.tris;
@@ -274,15 +400,31 @@ cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_fl
     a.order = order;
     a.ctl = ctl;
     a.stack_depth = bvh.stack_depth;
-    // a batch whose blocks all run at once leaves none to take over
-    a.claim = blocks > uint32_t(bvh.sm_count) * (inst ? 16u : uint32_t(kWarpsPerSm)) ? 1u : 0u;
+    a.claim = n > 32u * resident ? 1u : 0u;  // a batch whose blocks all run at once leaves none to take over
+    float diagonal2 = 0.0f;
+    for (int k = 0; k < 3; ++k) diagonal2 += (bvh.hi[k] - bvh.lo[k]) * (bvh.hi[k] - bvh.lo[k]);
+    a.reach2 = diagonal2 / 1024.0f;
     a.err = d_err;
     const size_t stack_bytes = size_t(bvh.stack_depth) * 32 * sizeof(uint2);
-    const uint32_t group_blocks = (n + 3u) / 4u;
-    if (inst) k_query_instanced<kAnyHit><<<blocks, 32, stack_bytes, s>>>(a);
-    else if (group_blocks <= kGroupWaves * uint32_t(bvh.sm_count) * kWarpsPerSm)
-        k_query_groups<kAnyHit><<<group_blocks, 32, stack_bytes, s>>>(a);
-    else k_query_wide<kAnyHit><<<blocks, 32, stack_bytes, s>>>(a);
+    const auto up_to = [&](uint32_t rays) { return n <= rays * resident; };
+    if (inst) {
+        if (far || a.claim || up_to(kInstStreamRays)) k_query_instanced<kAnyHit, false><<<blocks, 32, stack_bytes, s>>>(a);
+        else k_query_instanced<kAnyHit, true><<<blocks, 32, stack_bytes, s>>>(a);
+    } else if (up_to(far ? kFarGroupRays : kGroupRays<kAnyHit>)) {
+        k_query_groups<kAnyHit, false><<<(n + 3u) / 4u, 32, stack_bytes, s>>>(a);
+    } else if (!far && up_to(kSideGroupRays)) {
+        k_query_groups<kAnyHit, true><<<8 * blocks, 32, stack_bytes, s>>>(a);
+    } else if (up_to(far && !kAnyHit ? kFarPacketRays : kPacketRays)) {
+        k_query_packet<kAnyHit><<<blocks, 32, stack_bytes, s>>>(a);
+    } else {
+        if constexpr (!kAnyHit) {
+            if (far) {
+                k_query_wide<false, false><<<blocks, 32, stack_bytes, s>>>(a);
+                return cudaGetLastError();
+            }
+        }
+        k_query_wide<kAnyHit, true><<<blocks, 32, stack_bytes, s>>>(a);
+    }
     return cudaGetLastError();
 }
 
@@ -373,7 +515,7 @@ cudaError_t launch_query_ordered(const DeviceBvh& bvh, float4* d_rays, uint32_t 
                                                ntiles);
         in ^= 1;
     }
-    e = launch_wide<kAnyHit>(bvh, d_rays, record_float4s, n, vals[in], ctl, d_err, s);
+    e = launch_wide<kAnyHit>(bvh, d_rays, record_float4s, n, vals[in], ctl, d_err, s, false);
     const cudaError_t ef = cudaFreeAsync(mem, s);
     return e != cudaSuccess ? e : ef;
 }
@@ -401,10 +543,10 @@ __global__ void __launch_bounds__(kQueryBlock) k_query_binary(const float4* __re
 
 template <bool kAnyHit>
 cudaError_t launch_query(const DeviceBvh& bvh, float4* d_rays, uint32_t record_float4s, uint32_t n, uint32_t* d_err,
-                         cudaStream_t s) {
+                         cudaStream_t s, bool far = false) {
     if (n == 0) return cudaSuccess;
     if (bvh.insts || bvh.kind == SEL_BVH_WIDE8_Q8)
-        return launch_wide<kAnyHit>(bvh, d_rays, record_float4s, n, nullptr, nullptr, d_err, s);
+        return launch_wide<kAnyHit>(bvh, d_rays, record_float4s, n, nullptr, nullptr, d_err, s, far);
     const dim3 grid((n + kQueryBlock - 1) / kQueryBlock);
     k_query_binary<kAnyHit><<<grid, kQueryBlock, 0, s>>>(static_cast<const float4*>(bvh.nodes), bvh.tris, d_rays,
                                                          record_float4s, n, d_err);
@@ -429,7 +571,8 @@ cudaError_t launch_query_strided(bool any_hit, const DeviceBvh& bvh, void* recs,
                                  uint32_t* d_err, cudaStream_t s) {
     float4* r = static_cast<float4*>(recs);
     const uint32_t stride = uint32_t(record_bytes / 16);
-    return any_hit ? launch_query<true>(bvh, r, stride, n, d_err, s) : launch_query<false>(bvh, r, stride, n, d_err, s);
+    return any_hit ? launch_query<true>(bvh, r, stride, n, d_err, s, true)
+                   : launch_query<false>(bvh, r, stride, n, d_err, s, true);
 }
 
 }  // namespace sel

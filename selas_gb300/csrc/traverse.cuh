@@ -283,7 +283,7 @@ __device__ __forceinline__ bool wide_test(WideState& s, const float4* __restrict
     return true;
 }
 
-// The flat traversal of one lane, as trace_stream steps it.
+// The flat traversal of one lane, as trace_stream and trace_packet step it.
 struct WideWalk {
     static constexpr bool kAims = false;
     __device__ __forceinline__ bool aiming() const { return false; }
@@ -387,6 +387,104 @@ __device__ __forceinline__ void trace_stream(Rays& rays, const WideStack& stack,
             testing = __ballot_sync(0xffffffffu, busy && w.pending());
         }
         if (busy && !w.aiming()) busy = w.advance(stack, status);
+    }
+}
+
+// Traces one ray of each lane to its end: a node visit, then every leaf record that it exposed.  The lanes of a warp
+// whose rays run side by side stay in step that way and share their fetches, and a batch that gives each resident
+// warp only a few ranges of rays cannot refill its lanes long enough to gain from trace_stream (query.cu has the
+// figures of both).  live: the lane has a ray; its result is in w.s.
+template <bool kAnyHit, typename Walk, typename Rays>
+__device__ __forceinline__ void trace_packet(const Rays& rays, bool live, const QueryRay& r, Walk& w,
+                                             const WideStack& stack, uint32_t& status) {
+    bool busy = live && w.start(r, rays);
+    while (busy) {
+        if constexpr (Walk::kAims) {
+            if (w.aiming()) w.aim();
+        }
+        if (!w.pending()) busy = w.visit(rays, stack, status);
+        while (busy && w.pending()) busy = w.template test<kAnyHit>(rays, stack, status);
+        if (busy && !w.aiming()) busy = w.advance(stack, status);
+    }
+}
+
+// The any-hit packet of a flat scene: the warp tests the records that a step exposed together, 32 (ray, record) pairs a
+// round, each lane one pair with its owner's ray taken by shuffles.  Rays that part leave most lanes idle otherwise
+// (300,000 surface rays over 0.33 M triangles 117 against 122 us, 500,000 camera rays over 10,000 triangles 32 against
+// 42).  For closest hits the shuffles and result slots cost what the fuller warps save.  Called by the whole warp; only
+// the fact of a hit is reported (s.hit.tri is not the record's index).
+__device__ __forceinline__ void trace_packet_any(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
+                                                 bool live, const QueryRay& r, WideState& s, const WideStack& stack,
+                                                 uint32_t& status) {
+    wide_init(s, r);
+    bool busy = live && !ray_untraceable(r);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t axes = uint32_t(s.wt.kx) | (uint32_t(s.wt.ky) << 2) | (uint32_t(s.wt.kz) << 4);
+    while (__any_sync(0xffffffffu, busy)) {
+        uint32_t tmask = 0, tbase = 0;
+        if (busy && !wide_visit(s, nodes, stack, status, tmask, tbase)) {
+            busy = false;
+            tmask = 0;
+        }
+        // lane L owns pairs [first, last) of the warp's concatenation: its records in ascending order
+        uint32_t last = __popc(tmask);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, last, o);
+            if (lane >= uint32_t(o)) last += y;
+        }
+        const uint32_t first = last - __popc(tmask), total = __shfl_sync(0xffffffffu, last, 31);
+        for (uint32_t base = 0; base < total; base += 32) {
+            const uint32_t j = base + lane;
+            uint32_t owner = 0;  // the first lane whose last exceeds j
+#pragma unroll
+            for (uint32_t step = 16; step >= 1; step >>= 1) {
+                const uint32_t e = __shfl_sync(0xffffffffu, last, int(owner + step - 1));
+                if (e <= j) owner += step;
+            }
+            const int from = int(owner);
+            const uint32_t o_mask = __shfl_sync(0xffffffffu, tmask, from);
+            const uint32_t o_base = __shfl_sync(0xffffffffu, tbase, from);
+            const uint32_t o_first = __shfl_sync(0xffffffffu, first, from);
+            const uint32_t o_axes = __shfl_sync(0xffffffffu, axes, from);
+            Watertight w;
+            w.kx = int(o_axes & 3u);
+            w.ky = int((o_axes >> 2) & 3u);
+            w.kz = int((o_axes >> 4) & 3u);
+            w.sx = __shfl_sync(0xffffffffu, s.wt.sx, from);
+            w.sy = __shfl_sync(0xffffffffu, s.wt.sy, from);
+            w.sz = __shfl_sync(0xffffffffu, s.wt.sz, from);
+            const float ox = __shfl_sync(0xffffffffu, s.ox, from), oy = __shfl_sync(0xffffffffu, s.oy, from);
+            const float oz = __shfl_sync(0xffffffffu, s.oz, from);
+            const float tnear = __shfl_sync(0xffffffffu, s.tnear, from);
+            const float tfar = __shfl_sync(0xffffffffu, s.tfar, from);
+            bool got = false;
+            const uint32_t bit = j < total ? __fns(o_mask, 0u, int(j - o_first) + 1) : 0xffffffffu;
+            if (bit < 32u) {
+                const float4* tp = tris + size_t(o_base + bit) * 3;
+                const float4 p0 = __ldg(tp), p1 = __ldg(tp + 1), p2 = __ldg(tp + 2);
+                float t, u, v;
+                got = watertight_intersect(w, ox, oy, oz, p0, p1, p2, tnear, tfar, t, u, v);
+            }
+            const uint32_t hits = __ballot_sync(0xffffffffu, got);
+            const uint32_t a = first > base ? first : base, b = last < base + 32 ? last : base + 32;  // own pairs
+            if (busy && a < b && ((hits >> (a - base)) & (0xffffffffu >> (32u - (b - a))))) {
+                s.hit.tri = 0u;
+                busy = false;
+            }
+        }
+        if (busy && ++s.iters > kIterationCap) {
+            status |= kErrIterationCap;
+            busy = false;
+        }
+        if (busy && !(s.group.y & 0xff000000u)) {
+            if (s.sp == 0) {
+                busy = false;
+            } else {
+                --s.sp;
+                s.group = stack.mem[s.sp * stack.stride];
+            }
+        }
     }
 }
 
