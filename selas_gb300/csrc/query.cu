@@ -88,8 +88,9 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
 //     58,368 camera    closest  22 | 38 | 62 against 26 | 52 | 77   any  19 | 29 | 48 against 23 | 36 | 64
 //     90,000 camera    closest  26 | 46 | 88 against 28 | 54 | 106  any  22 | 36 | 55 against 20 | 44 | 60
 //     116,736 camera   closest  32 | 54 | 94 against 29 | 52 | 101  any  28 | 37 | 62 against 22 | 38 | 62
-//   (the limits lie at whole rounds of the resident warps; at 8 to 9 rays a warp closest hits of 0.33 M triangles still
-//   favour the groups, 56 against 63, any hit everywhere the packets).
+//   (from 34,500 to 45,000 surface rays the packets gain on seven scenes of up to 0.5 M triangles, 1.05 times in the
+//   middle; over 1.2 and 2.4 M triangles the groups lead up to kLargeGroupRays, 39,500 rays closest hit 82 and 74
+//   against 77 and 90, any hit 60 and 65 against 72 and 76, and over 5.2 M neither does, 92 and 72 against 91 and 69).
 //   A lane a ray, side by side to the end (trace_packet), up to kPacketRays, and at any size for rays side by side.
 //   Against streams:
 //     90,000 surface   closest  41 | 73 | 117 against 47 | 93 | 131        any  34 | 52 | 97 against 43 | 67 | 119
@@ -123,6 +124,7 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
 constexpr uint32_t kWarpsPerSm = 32, kInstWarpsPerSm = 16;
 template <bool kAnyHit>
 constexpr uint32_t kGroupRays = kAnyHit ? 7 : 8;
+constexpr uint32_t kLargeGroupRays = 9, kLargeScene = 1u << 20;  // triangles
 constexpr uint32_t kSideGroupRays = 20, kPacketRays = 64, kInstStreamRays = 2, kFarGroupRays = 12, kFarPacketRays = 32;
 constexpr uint32_t kErrClaimTimeout = 32u;  // the answer to a work request never came
 
@@ -410,7 +412,7 @@ cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_fl
     if (inst) {
         if (far || a.claim || up_to(kInstStreamRays)) k_query_instanced<kAnyHit, false><<<blocks, 32, stack_bytes, s>>>(a);
         else k_query_instanced<kAnyHit, true><<<blocks, 32, stack_bytes, s>>>(a);
-    } else if (up_to(far ? kFarGroupRays : kGroupRays<kAnyHit>)) {
+    } else if (up_to(far ? kFarGroupRays : bvh.tri_count > kLargeScene ? kLargeGroupRays : kGroupRays<kAnyHit>)) {
         k_query_groups<kAnyHit, false><<<(n + 3u) / 4u, 32, stack_bytes, s>>>(a);
     } else if (!far && up_to(kSideGroupRays)) {
         k_query_groups<kAnyHit, true><<<8 * blocks, 32, stack_bytes, s>>>(a);
