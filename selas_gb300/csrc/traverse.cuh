@@ -19,6 +19,7 @@ constexpr uint32_t kIterationCap = 1u << 22;  // node visits + triangle tests pe
 constexpr uint32_t kErrIterationCap = 1u;
 constexpr uint32_t kErrStackOverflow = 2u;
 constexpr float kBoxMargin = 1.0f / 1048576.0f;  // relative widening of the ray interval for box tests
+constexpr float kOut = 1.0f / 2097152.0f;        // relative outward widening of a node's plane offsets
 
 __device__ __forceinline__ float pick3(int k, float x, float y, float z) { return k == 0 ? x : (k == 1 ? y : z); }
 
@@ -196,10 +197,12 @@ __device__ __forceinline__ float qbyte(uint32_t word, uint32_t byte) {
 // hit leaf children as a bit mask over records tbase..tbase+31.  Returns false on stack overflow.
 //
 // A plane's distance is (2^15 + q) * (scale / d) + (origin - 2^15 * scale / d): one byte permute and one
-// multiply-add, the bias folded into the offset.  The fold costs 2^-9 of a quantum in the offset's rounding;
-// widening the offsets outward by 2^-22 of their magnitude covers that and the offset's own rounding, so no
-// distance of the ray's origin makes a box smaller.  Offsets that overflow turn into infinities and NaN that the
-// minima and maxima ignore: their axis then accepts every box.
+// multiply-add, the bias folded into the offset.  The offset is widened outward by 2^-21 of its magnitude.  That
+// covers every rounding of the distance (three in the node's own distance p, one in the offset, one in the sum) once p
+// exceeds 2^17 quanta; nearer, where p and the bias can cancel, at most 0.04 of a quantum is left uncovered, well within
+// the half quantum that both builders leave between a child's planes and its box.  So no distance of the ray's origin
+// loses what a box holds.  Offsets that overflow turn into infinities and NaN that the minima and maxima ignore: their
+// axis then accepts every box.
 __device__ __forceinline__ bool wide_visit(WideState& s, const uint4* __restrict__ nodes, const WideStack& stack,
                                            uint32_t& status, uint32_t& tmask, uint32_t& tbase) {
     const int b = __ffs(s.group.y >> 24) - 1;
@@ -219,7 +222,6 @@ __device__ __forceinline__ bool wide_visit(WideState& s, const uint4* __restrict
     const float ax = fmaf(-32768.0f, sx, __fmul_rn(__fsub_rn(__uint_as_float(n0.x), s.ox), s.ix));
     const float ay = fmaf(-32768.0f, sy, __fmul_rn(__fsub_rn(__uint_as_float(n0.y), s.oy), s.iy));
     const float az = fmaf(-32768.0f, sz, __fmul_rn(__fsub_rn(__uint_as_float(n0.z), s.oz), s.iz));
-    constexpr float kOut = 1.0f / 4194304.0f;
     // (near, far) pairs
     const uint64_t sx2 = pack2(sx, sx), sy2 = pack2(sy, sy), sz2 = pack2(sz, sz);
     const uint64_t ax2 = pack2(fmaf(-kOut, fabsf(ax), ax), fmaf(kOut, fabsf(ax), ax));
@@ -519,7 +521,6 @@ __device__ __forceinline__ void trace_group(const uint4* __restrict__ nodes, con
         const float ax = __fmul_rn(__fsub_rn(__uint_as_float(n0.x), s.ox), s.ix);
         const float ay = __fmul_rn(__fsub_rn(__uint_as_float(n0.y), s.oy), s.iy);
         const float az = __fmul_rn(__fsub_rn(__uint_as_float(n0.z), s.oz), s.iz);
-        constexpr float kOut = 1.0f / 4194304.0f;  // outward, as wide_visit widens
         auto plane = [&](uint32_t w0, uint32_t w1) { return __uint2float_rn(__byte_perm(w0, w1, child) & 0xffu); };
         const float lx = plane(n2.x, n2.y), hx = plane(n3.z, n3.w);
         const float ly = plane(n2.z, n2.w), hy = plane(n4.x, n4.y);
