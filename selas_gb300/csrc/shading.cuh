@@ -302,7 +302,7 @@ SEL_HD float3 offset_origin(float3 p, float3 n, float error, float3 dir, float s
     return p + (side * error * scale) * n;
 }
 
-// The shading kernels are straight lines of 80 to 170 KB of code that every hit runs once: with the warps of an SM at
+// The shading kernels are long straight lines of code that every hit runs once: with the warps of an SM at
 // different places their rate is set by instruction fetches.  So an SM runs one block that meets at barriers between
 // the stages of a hit, and one fetch serves its warps (Cornell box 512 x 512 x 64 spp 22.9 -> 21.7 ms, textured room
 // 1280 x 720 x 4 spp 29.0 -> 27.7, deferred sky 641 x 359 x 16 spp 6.39 -> 5.09; the large block without barriers gave a
