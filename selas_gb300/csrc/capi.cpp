@@ -121,6 +121,7 @@ int sel_device_new(int cuda_device, SelDevice* out_device) {
     e = cudaStreamCreateWithFlags(&dev->stream, cudaStreamNonBlocking);
     for (int k = 0; k < 4 && e == cudaSuccess; ++k) e = cudaStreamCreateWithFlags(&dev->qstream[k], cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&dev->sm_count, cudaDevAttrMultiProcessorCount, cuda_device);
+    if (e == cudaSuccess) e = cudaMalloc(&dev->d_small, 256);
     if (e == cudaSuccess) e = cudaHostAlloc(&dev->h_err, sizeof(uint32_t), cudaHostAllocMapped);
     if (e == cudaSuccess) {
         *dev->h_err = 0;
@@ -153,6 +154,7 @@ int sel_device_new(int cuda_device, SelDevice* out_device) {
         for (cudaStream_t q : dev->qstream)
             if (q) cudaStreamDestroy(q);
         if (dev->h_err) cudaFreeHost(dev->h_err);
+        if (dev->d_small) cudaFree(dev->d_small);
         delete dev;
         return cuda_fail(e, "device setup");
     }
@@ -170,6 +172,7 @@ int sel_device_release(SelDevice device) {
         cudaStreamDestroy(q);
     }
     cudaFreeHost(device->h_err);
+    cudaFree(device->d_small);
     if (device->order_pool) cudaMemPoolDestroy(device->order_pool);  // released once its last block is freed
     delete device;
     return SEL_OK;
