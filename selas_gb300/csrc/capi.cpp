@@ -78,6 +78,7 @@ DeviceBvh device_bvh(const SelSceneTy* sc) {
     b.stack_depth = int(scene_stack_depth(sc));
     b.sm_count = sc->dev->sm_count;
     b.insts = static_cast<const InstanceRecord*>(sc->d_insts);
+    b.curves = sc->tree_curves;
     for (int a = 0; a < 3; ++a) {
         b.lo[a] = sc->info.bounds_lo[a];
         b.hi[a] = sc->info.bounds_hi[a];
@@ -497,6 +498,8 @@ int finish_instances(SelSceneTy* scene, uint32_t levels, uint32_t below) {
         if (e != cudaSuccess) return cuda_fail(e, "instance table");
     }
     scene->inst_levels = levels;
+    scene->tree_curves = !scene->curves.empty();
+    for (const SelSceneTy::InstanceInput& ii : scene->instances) scene->tree_curves |= ii.scene->tree_curves;
     for (auto& r : scene->referenced) --r.first->instanced_by;
     scene->referenced.clear();
     for (const SelSceneTy::InstanceInput& ii : scene->instances) {

@@ -61,6 +61,7 @@ struct SelSceneTy {
     bool sort_hint_ptex = false;              // a material of this scene uses Ptex
     uint32_t inst_levels = 0;                 // instance levels below this scene at the last commit (0..2)
     uint32_t stack_need = 0;                  // worst-case instanced-traversal stack entries from here down
+    bool tree_curves = false;                 // the scene or one that it instances holds curves
     uint64_t generation = 0;                  // incremented by every commit
     std::vector<std::pair<SelSceneTy*, uint64_t>> referenced;  // instanced scenes and their generations
     int instanced_by = 0;                     // committed scenes whose instances reference this one

@@ -102,7 +102,8 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
 // Scenes with instances: streams, but for kInstStreamRays to 32 rays a warp, where rays that part are packets (40,000
 // random rays, closest hit over 20 | 500 | 2000 instances 46 | 92 | 174 against 45 | 99 | 181, any hit 36 | 73 | 114
 // against 41 | 84 | 125; camera rays, which meet different instances from lane to lane, stay streams: 170 against 156 us as
-// packets over 500 instances, and 4 M of them 3.0 against 2.6 ms).
+// packets over 500 instances, and 4 M of them 3.0 against 2.6 ms).  Scenes with curves stay streams, one segment a step
+// (40,000 random rays over 22,000 segments 2.2 ms, as packets 3.5).
 //
 // Records in host memory, traced in place (far): the link carries every look, so eight looks at a record cost more than any
 // form (45,000 camera rays, closest hit over 0.33 M triangles: a call of 161 us with them, 66 as groups, 82 as packets).
@@ -410,7 +411,7 @@ cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_fl
     const size_t stack_bytes = size_t(bvh.stack_depth) * 32 * sizeof(uint2);
     const auto up_to = [&](uint32_t rays) { return n <= rays * resident; };
     if (inst) {
-        if (far || a.claim || up_to(kInstStreamRays)) k_query_instanced<kAnyHit, false><<<blocks, 32, stack_bytes, s>>>(a);
+        if (far || bvh.curves || a.claim || up_to(kInstStreamRays)) k_query_instanced<kAnyHit, false><<<blocks, 32, stack_bytes, s>>>(a);
         else k_query_instanced<kAnyHit, true><<<blocks, 32, stack_bytes, s>>>(a);
     } else if (up_to(far ? kFarGroupRays : bvh.tri_count > kLargeScene ? kLargeGroupRays : kGroupRays<kAnyHit>)) {
         k_query_groups<kAnyHit, false><<<(n + 3u) / 4u, 32, stack_bytes, s>>>(a);

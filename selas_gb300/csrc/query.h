@@ -15,6 +15,7 @@ struct DeviceBvh {
     uint32_t tri_count = 0;
     int stack_depth = kWideStack;  // traversal stack entries a ray may need (8-wide layout)
     int sm_count = 1;
+    bool curves = false;  // the scene or one that it instances holds curves
     const InstanceRecord* insts = nullptr;  // instance table of a scene with instances (8-wide layout only)
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // scene bounds (ray ordering keys)
     bool order_rays = false;  // SEL_OPTION_RAY_SORT: large incoherent batches in HBM are traced in key order
