@@ -98,7 +98,9 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
 //     500,000 surface  closest  137 | 200 | 379 against 140 | 206 | 350    any  114 | 162 | 279 against 117 | 163 | 282
 //     4.2 M surface    closest  960 | 1404 | 2598 against 890 | 1210 | 2048   any  794 | 1103 | 1844 against 720 | 940 | 1470
 //     1 M camera       closest  52 | 113 | 273 against 73 | 145 | 272      any  40 | 86 | 164 against 58 | 105 | 192
-//   Streams of rays (trace_stream) otherwise.
+//   Streams of rays (trace_stream) otherwise, and, over more than a million triangles, for closest hits of more than
+//   kLargeLookRays whatever the rays: there both forms trace camera rays alike (2 M 372 against 370 us, 4.2 M
+//   from four places 511 | 533 | 560 | 595 against 515 | 553 | 555 | 580) and parting rays are spared the look.
 // Scenes with instances: streams, but for kInstStreamRays to 32 rays a warp, where rays that part are packets (40,000
 // random rays, closest hit over 20 | 500 | 2000 instances 46 | 92 | 174 against 45 | 99 | 181, any hit 36 | 73 | 114
 // against 41 | 84 | 125; camera rays, which meet different instances from lane to lane, stay streams: 170 against 156 us as
@@ -125,7 +127,7 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
 constexpr uint32_t kWarpsPerSm = 32, kInstWarpsPerSm = 16;
 template <bool kAnyHit>
 constexpr uint32_t kGroupRays = kAnyHit ? 7 : 8;
-constexpr uint32_t kLargeGroupRays = 9, kLargeScene = 1u << 20;  // triangles
+constexpr uint32_t kLargeGroupRays = 9, kLargeLookRays = 256, kLargeScene = 1u << 20;  // triangles
 constexpr uint32_t kSideGroupRays = 20, kPacketRays = 64, kInstStreamRays = 2, kFarGroupRays = 12, kFarPacketRays = 32;
 constexpr uint32_t kErrClaimTimeout = 32u;  // the answer to a work request never came
 
@@ -421,7 +423,7 @@ cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_fl
         k_query_packet<kAnyHit><<<blocks, 32, stack_bytes, s>>>(a);
     } else {
         if constexpr (!kAnyHit) {
-            if (far) {
+            if (far || (bvh.tri_count > kLargeScene && !up_to(kLargeLookRays))) {
                 k_query_wide<false, false><<<blocks, 32, stack_bytes, s>>>(a);
                 return cudaGetLastError();
             }

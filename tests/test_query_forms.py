@@ -82,11 +82,13 @@ def test_flat_scenes_around_each_limit(device, kind, where, per_warp):
     sc.release()
 
 
+@pytest.mark.parametrize("per_warp", [9, 256])
 @pytest.mark.parametrize("kind", ["camera", "surface"])
-def test_large_scenes_around_their_limit(device, kind):
-    """Scenes of more than 2^20 triangles stay with eight lanes a ray a little longer; against batches a tenth the size."""
+def test_large_scenes_around_their_limits(device, kind, per_warp):
+    """Scenes of more than 2^20 triangles stay with eight lanes a ray a little longer, and their largest closest-hit batches
+    are streams whatever the rays; against smaller batches."""
     data = scenes.displaced_icospheres(count=13, level=6, seed=43)
-    limit = 9 * _warps(32)
+    limit = per_warp * _warps(32)
     org, d = _rays(data, limit + 37, kind, 9)
     sc = sel.Scene(device)
     data.attach_to(sc)
@@ -94,7 +96,7 @@ def test_large_scenes_around_their_limit(device, kind):
     assert sc.info().triangle_count > 1 << 20
     for make in (sel.make_rayhits, sel.make_rays):
         recs = make(org, d)
-        want = np.concatenate([_trace(sc, part.copy(), "device") for part in np.array_split(recs, 10)])
+        want = np.concatenate([_trace(sc, part.copy(), "device") for part in np.array_split(recs, 10 * (per_warp // 8))])
         for n in (limit - 1, limit, limit + 1, limit + 37):
             assert_hits_equal(_trace(sc, recs[:n].copy(), "device"), want[:n],
                               fields=("tfar",) if make is sel.make_rays else HIT_FIELDS)
