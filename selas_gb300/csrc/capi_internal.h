@@ -18,9 +18,10 @@ struct SelDeviceTy {
     int sm_count = 1;
     uint32_t* h_err = nullptr;      // kernel error word (iteration cap / stack overflow bits), page-locked host memory
     uint32_t* d_err = nullptr;      // its device address
-    // A few bytes held for as long as the device: while none of a process's small allocations is left, the driver gives the
-    // 2 MB block that they share back, and the next scene's first and last one pay for making and freeing it (a scene of
-    // 22 triangles attached, committed on the host and released: 0.24 against 0.07 ms, on the GPU 0.30 against 0.16).
+    // A few bytes held for as long as the device: while none of a process's small allocations is left, the driver gives
+    // the 2 MB block that they share back, and the next scene's first and last one pay for making and freeing it (a
+    // scene of 22 triangles attached, committed on the host and released: 0.24 against 0.07 ms, on the GPU 0.30 against
+    // 0.16).
     void* d_small = nullptr;
     bool pageable_access = false;   // the GPU reads and writes any host memory through the host's page tables
     cudaMemPool_t order_pool = nullptr;  // stream-ordered scratch of ordered queries (keeps freed memory)

@@ -1,5 +1,5 @@
-// Ray-query kernels over SelRay / SelRayHit records (Embree's RTCRay / RTCRayHit layouts) and their launchers.  A ray is
-// traced by one lane or, in small batches, by eight; each thread keeps its traversal stack in shared memory.
+// Ray-query kernels over SelRay / SelRayHit records (Embree's RTCRay / RTCRayHit layouts) and their launchers.  A ray
+// is traced by one lane or, in small batches, by eight; each thread keeps its traversal stack in shared memory.
 #include "query.h"
 
 #include <type_traits>
@@ -78,8 +78,8 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
 }
 
 // ---------------------------------------------------------------------------------------------------
-// 8-wide traversal.  Blocks are one warp; 64 registers let 32 of them run on an SM.  Which form a batch takes follows its
-// size, in rays for each warp that runs at once, and, where the size does not settle it, a look at the warp's own
+// 8-wide traversal.  Blocks are one warp; 64 registers let 32 of them run on an SM.  Which form a batch takes follows
+// its size, in rays for each warp that runs at once, and, where the size does not settle it, a look at the warp's own
 // rays (side_by_side).  Device times in us over 10 k | 0.33 M | 5.2 M triangles; "surface" rays bounce off random
 // points, "camera" rays are a frame's in pixel order.
 //   Eight lanes a ray (trace_group) up to kGroupRays, and to kSideGroupRays for rays side by side.  Against packets:
@@ -96,23 +96,24 @@ __device__ __forceinline__ void store_hit_instanced(SelRayHit* rh, const InstHit
 //     90,000 surface   closest  41 | 73 | 117 against 47 | 93 | 131        any  34 | 52 | 97 against 43 | 67 | 119
 //     300,000 surface  closest  88 | 138 | 253 against 96 | 145 | 257      any  74 | 117 | 213 against 82 | 126 | 210
 //     500,000 surface  closest  137 | 200 | 379 against 140 | 206 | 350    any  114 | 162 | 279 against 117 | 163 | 282
-//     4.2 M surface    closest  960 | 1404 | 2598 against 890 | 1210 | 2048   any  794 | 1103 | 1844 against 720 | 940 | 1470
+//     4.2 M surface    closest  960 | 1404 | 2598 against 890 | 1210 | 2048
+//                      any  794 | 1103 | 1844 against 720 | 940 | 1470
 //     1 M camera       closest  52 | 113 | 273 against 73 | 145 | 272      any  40 | 86 | 164 against 58 | 105 | 192
 //   Streams of rays (trace_stream) otherwise, and, over more than a million triangles, for closest hits of more than
 //   kLargeLookRays whatever the rays: there both forms trace camera rays alike (2 M 372 against 370 us, 4.2 M
 //   from four places 511 | 533 | 560 | 595 against 515 | 553 | 555 | 580) and parting rays are spared the look.
 // Scenes with instances: streams, but for kInstStreamRays to 32 rays a warp, where rays that part are packets (40,000
 // random rays, closest hit over 20 | 500 | 2000 instances 46 | 92 | 174 against 45 | 99 | 181, any hit 36 | 73 | 114
-// against 41 | 84 | 125; camera rays, which meet different instances from lane to lane, stay streams: 170 against 156 us as
-// packets over 500 instances, and 4 M of them 3.0 against 2.6 ms).  Scenes with curves stay streams, one segment a step
-// (40,000 random rays over 22,000 segments 2.2 ms, as packets 3.5).
+// against 41 | 84 | 125; camera rays, which meet different instances from lane to lane, stay streams: 170 against 156
+// us as packets over 500 instances, and 4 M of them 3.0 against 2.6 ms).  Scenes with curves stay streams, one segment
+// a step (40,000 random rays over 22,000 segments 2.2 ms, as packets 3.5).
 //
-// Records in host memory, traced in place (far): the link carries every look, so eight looks at a record cost more than any
-// form (45,000 camera rays, closest hit over 0.33 M triangles: a call of 161 us with them, 66 as groups, 82 as packets).
-// Groups up to kFarGroupRays (58,368 rays surface, packets against groups: closest 78 | 107 | 131 against 73 | 95 | 144, any
-// 60 | 71 | 105 against 60 | 75 | 105; camera 64 | 93 | 117 against 60 | 79 | 93, any 50 | 63 | 87 against 36 | 44 | 65), then
-// packets; closest hits are streams, without a look, from kFarPacketRays on (300,000 camera rays 303 | 321 | 329 against 315 |
-// 326 | 343 us as packets, surface 238 | 277 | 357 against 233 | 276 | 372).
+// Records in host memory, traced in place (far): the link carries every look, so eight looks at a record cost more than
+// any form (45,000 camera rays, closest hit over 0.33 M triangles: a call of 161 us with them, 66 as groups, 82 as
+// packets). Groups up to kFarGroupRays (58,368 rays surface, packets against groups: closest 78 | 107 | 131 against 73
+// | 95 | 144, any 60 | 71 | 105 against 60 | 75 | 105; camera 64 | 93 | 117 against 60 | 79 | 93, any 50 | 63 | 87
+// against 36 | 44 | 65), then packets; closest hits are streams, without a look, from kFarPacketRays on (300,000 camera
+// rays 303 | 321 | 329 against 315 | 326 | 343 us as packets, surface 238 | 277 | 357 against 233 | 276 | 372).
 //
 // A stream's warp starts with its block's records, block index k standing for records [32 k, 32 k + 32).  A warp whose
 // lanes run out of rays takes over the block index of a block that has not started (cluster launch control) and
@@ -133,7 +134,7 @@ constexpr uint32_t kErrClaimTimeout = 32u;  // the answer to a work request neve
 
 __device__ __forceinline__ uint32_t shared_address(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
-// The records a warp traces.  kOrdered: record `order[i]` in place of record i when ctl[0] is non-zero.
+// The ranges of records a warp traces.
 struct RecordRanges {
     uint32_t n, status;
     bool claim, started;     // claim: takes over blocks that have not started
@@ -355,9 +356,9 @@ __global__ void __launch_bounds__(32, kWarpsPerSm) k_query_packet(const __grid_c
     if (status) atomicOr(a.err, status);
 }
 
-// Four rays a one-warp block, eight lanes each.  kLook: the eight blocks of 32 records look at these records' rays (whose
-// origins and directions no query writes) and, unless they run side by side, leave them to the first of the eight.  The
-// first blocks of all records come before the others, which mostly find nothing to do when the rays part.
+// Four rays a one-warp block, eight lanes each.  kLook: the eight blocks of 32 records look at these records' rays
+// (whose origins and directions no query writes) and, unless they run side by side, leave them to the first of the
+// eight.  The first blocks of all records come before the others, which mostly find nothing to do when the rays part.
 template <bool kAnyHit, bool kLook>
 __global__ void __launch_bounds__(32, kWarpsPerSm) k_query_groups(const __grid_constant__ QueryArgs a) {
     RecordRays<kAnyHit, false> rays = query_records<kAnyHit, false>(a);
@@ -413,7 +414,8 @@ cudaError_t launch_wide(const DeviceBvh& bvh, float4* d_rays, uint32_t record_fl
     const size_t stack_bytes = size_t(bvh.stack_depth) * 32 * sizeof(uint2);
     const auto up_to = [&](uint32_t rays) { return n <= rays * resident; };
     if (inst) {
-        if (far || bvh.curves || a.claim || up_to(kInstStreamRays)) k_query_instanced<kAnyHit, false><<<blocks, 32, stack_bytes, s>>>(a);
+        const bool streams = far || bvh.curves || a.claim || up_to(kInstStreamRays);
+        if (streams) k_query_instanced<kAnyHit, false><<<blocks, 32, stack_bytes, s>>>(a);
         else k_query_instanced<kAnyHit, true><<<blocks, 32, stack_bytes, s>>>(a);
     } else if (up_to(far ? kFarGroupRays : bvh.tri_count > kLargeScene ? kLargeGroupRays : kGroupRays<kAnyHit>)) {
         k_query_groups<kAnyHit, false><<<(n + 3u) / 4u, 32, stack_bytes, s>>>(a);

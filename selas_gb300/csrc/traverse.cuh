@@ -199,10 +199,10 @@ __device__ __forceinline__ float qbyte(uint32_t word, uint32_t byte) {
 // A plane's distance is (2^15 + q) * (scale / d) + (origin - 2^15 * scale / d): one byte permute and one
 // multiply-add, the bias folded into the offset.  The offset is widened outward by 2^-21 of its magnitude.  That
 // covers every rounding of the distance (three in the node's own distance p, one in the offset, one in the sum) once p
-// exceeds 2^17 quanta; nearer, where p and the bias can cancel, at most 0.04 of a quantum is left uncovered, well within
-// the half quantum that both builders leave between a child's planes and its box.  So no distance of the ray's origin
-// loses what a box holds.  Offsets that overflow turn into infinities and NaN that the minima and maxima ignore: their
-// axis then accepts every box.
+// exceeds 2^17 quanta; nearer, where p and the bias can cancel, at most 0.04 of a quantum is left uncovered, well
+// within the half quantum that both builders leave between a child's planes and its box.  So no distance of the ray's
+// origin loses what a box holds.  Offsets that overflow turn into infinities and NaN that the minima and maxima ignore:
+// their axis then accepts every box.
 __device__ __forceinline__ bool wide_visit(WideState& s, const uint4* __restrict__ nodes, const WideStack& stack,
                                            uint32_t& status, uint32_t& tmask, uint32_t& tbase) {
     const int b = __ffs(s.group.y >> 24) - 1;
